@@ -22,6 +22,7 @@
 // frequency) beyond 1e-5 relative.
 #include <cmath>
 #include "integrals.cuh"
+#include "packed_table.cuh"
 
 namespace bem {
 namespace {
@@ -877,6 +878,257 @@ __global__ void __launch_bounds__(kSymT, 5) wave_symmetric_kernel(bem_assembly_a
   if (nan_seen && a.nan_flag_dev) atomicOr(a.nan_flag_dev, 1);
 }
 
+// ---- wave term from the packed table ----------------------------------------
+// Nodes of the stencil by the packed table's estimates, decided by the float64
+// expressions next to a rounding boundary.
+__device__ __forceinline__ void packed_integrals(double r, double z, const PackedTab& P, bool high, double out[4]) {
+  if (fabs(z) < P.zmax && r < P.rmax) {
+    const int i = packed_r_node(r, P, [&](double x) { return nearest_r_index(x, P.nr, P.rmax, P.grid); });
+    const int j = packed_z_node(z, P, [&](double x) { return nearest_z_index(x, P.nz, -P.zmax, P.grid, P.dz); });
+    packed_interpolate(r, z, i, j, P, out);
+    return;
+  }
+  double I[5];
+  asymptotic<double>(r, z, I);
+  out[0] = high ? I[1] : I[0];
+  out[1] = I[2];
+  out[2] = I[3];
+  out[3] = I[4];
+}
+
+// The wave term of one pair of points for a unit weight, before the factor
+// k w: g (its value), and the derivatives along the horizontal unit vector
+// between the points (h) and along z (v), each divided by k for a better use
+// of the multiply-adds: gradient = k (h * unit vector, v).  inv_h and inv_R are
+// the reciprocals of the horizontal distance and of the distance to the other
+// point's image, both independent of the wavenumber.
+struct WavePair {
+  double g_re, g_im, h_re, h_im, v_re, v_im;
+};
+template <bool HIGH>
+__device__ __forceinline__ WavePair wave_pair(double r, double z, double k, double inv_k, double inv_R,
+                                              const PackedTab& P) {
+  double I[4];
+  packed_integrals(r, z, P, HIGH, I);
+  const double inv_r1 = inv_R * inv_k;  // 1 / |(r, z)|
+  WavePair w;
+  w.g_re = I[0];
+  w.g_im = I[1];
+  w.h_im = I[3];
+  w.v_im = I[1];
+  if (HIGH) {
+    const double s = 2 * inv_r1 * inv_r1 * inv_r1;
+    w.h_re = I[2] - r * s;
+    w.v_re = I[0] - z * s;
+  } else {
+    w.h_re = I[2];
+    w.v_re = I[0] + 2 * inv_r1;
+  }
+  return w;
+}
+
+// Running maximum of the magnitudes' high words: a NaN leaves at least
+// 0x7ff80000 (arithmetic NaNs are quiet), at two integer operations per value.
+__device__ __forceinline__ unsigned nan_track(unsigned m, double x) {
+  return max(m, (unsigned)__double2hiint(x) & 0x7fffffffu);
+}
+
+constexpr int kPairRows = 128;    // rows per CTA: four warps of 32
+constexpr int kPairChunk = 8;     // columns per mirrored write-back of a warp
+constexpr int kMirLd = 32 + 8 / kPairChunk;        // shared-memory row of 32 mirrored entries (no bank conflicts)
+
+struct PairFace {
+  double x[3];  // collocation point = quadrature point = centre
+  double dn[3];
+  double area, w, zc;
+};
+
+// S and K of one or several wavenumbers from the Rankine part and the packed
+// table (what wave_symmetric_kernel does from the plain table): a warp owns 32
+// rows and cw columns of a 128 x 128 tile, one row per lane.  Off the diagonal
+// tiles the wave term is evaluated once per unordered pair and the mirrored
+// entries go through the warp's own shared memory, 8 columns at a time, so
+// that both stores are coalesced and no warp waits for another.
+// Bound: the load pipe of L1 (68% busy, float64 pipe 18%): the nine quads of a
+// lookup are 288 bytes per lane from its own place in the table.  The 15
+// wavenumbers of the 6084-panel barge take 8.9 ms (0.60 ms each, 42 float64
+// operations fewer per pair and 11 loads in place of 57), from 15.4 ms with the
+// plain table.  Three CTAs per SM (168 registers), not four (0.64 ms): a fourth
+// takes 43 KB from the L1 that holds the table's rows; two leave too few warps
+// (0.79 ms).  128-bit loads: 0.69 ms.  Mirrored chunks of 4 or 2 columns
+// (more L1): 0.60 ms.
+// The grid is one-dimensional with the wavenumber fastest: the CTAs of one tile
+// run together and read its Rankine part from L2.  cw (8 to 128) shrinks when
+// the tiles do not fill the GPU (pair_chunk).
+template <bool GENERAL, bool INPLACE, bool HIGH>
+__global__ void __launch_bounds__(kPairRows, 3)
+    wave_pairs_kernel(bem_assembly_args a, PackedTab P, SymBatch kb, const double2* rank, int64_t rank_ld, int cw,
+                      int nbi, int nk) {
+  __shared__ PairFace faces[kSymT];
+  __shared__ double2 mir[4][2][kPairChunk * kMirLd];  // per warp: wave parts of S and K of entries (J, I)
+  int t = blockIdx.x;
+  const int kidx = t % nk;
+  t /= nk;
+  const int per_tile = kSymT / cw;
+  const int ch = t % per_tile;
+  t /= per_tile;
+  int bi, bj;
+  if (GENERAL) {
+    bi = t % nbi;
+    bj = t / nbi;
+  } else {  // tile t of the upper triangle, column bj holding bj + 1 tiles
+    bj = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+    while ((bj + 1) * (bj + 2) / 2 <= t) ++bj;
+    while (bj * (bj + 1) / 2 > t) --bj;
+    bi = t - bj * (bj + 1) / 2;
+  }
+  const int N = a.n, NJ = GENERAL ? a.nb_faces : a.n;
+  const int J0 = bj * kSymT + ch * cw;
+  const int nJ = min(cw, NJ - J0);
+  if (nJ <= 0) return;
+  const double k = kb.k[kidx];
+  const double inv_k = 1.0 / k;
+  const bool adjoint = a.adjoint_double_layer != 0;
+  P.load(HIGH);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < nJ) {
+    const int J = J0 + tid;
+    PairFace& f = faces[tid];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      f.x[d] = a.quad_points_dev[3 * J + d];
+      f.dn[d] = (!GENERAL || !adjoint) ? a.dot_normals_dev[3 * J + d] : 0.0;
+    }
+    f.area = a.areas_dev[J];
+    f.w = a.quad_weights_dev[J];
+    f.zc = a.centers_dev[3 * J + 2];
+  }
+  __syncthreads();
+  const int I0 = bi * kSymT + warp * 32;
+  if (I0 >= N) return;  // no barrier of the whole CTA below
+  const int I = I0 + lane;
+  const bool row_ok = I < N;
+  const int Ic = min(I, N - 1);  // lanes past the last row repeat it and store nothing
+  const bool mirrored = !GENERAL && bi != bj;
+  double M[3], nI[3] = {0, 0, 0}, cI = 0, areaI = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    M[d] = a.points_dev[3 * Ic + d];
+    if (!GENERAL || adjoint) nI[d] = a.dot_normals_dev[3 * Ic + d];
+  }
+  if (!GENERAL) {
+    cI = kMinusOneOverFourPi * k * a.quad_weights_dev[Ic];
+    areaI = a.areas_dev[Ic];
+  }
+  double2* S = reinterpret_cast<double2*>(a.S_dev) + kidx * kb.s_stride;
+  double2* K = reinterpret_cast<double2*>(a.K_dev) + kidx * kb.k_stride;
+  if (INPLACE) rank = K;
+  float* W = kb.w ? kb.w + kidx * kb.w_stride : nullptr;
+  double2* mS = mir[warp][0];
+  double2* mK = mir[warp][1];
+  unsigned nan_max = 0;
+  for (int jc = 0; jc < nJ; jc += kPairChunk) {
+#pragma unroll 1
+    for (int u = 0; u < kPairChunk; ++u) {
+      const int jj = jc + u;
+      if (jj >= nJ) break;
+      const PairFace& f = faces[jj];
+      const int J = J0 + jj;
+      const size_t ridx = (size_t)Ic + (size_t)rank_ld * J;
+      const double2 rk = INPLACE ? rank[ridx] : __ldg(rank + ridx);
+      const double dx = M[0] - f.x[0], dy = M[1] - f.x[1], zs = M[2] + f.x[2];
+      const double h2 = dx * dx + dy * dy;
+      const double inv_R = rsqrt(h2 + zs * zs);
+      const double ih = h2 > 0.0 ? rsqrt(h2) : 0.0;
+      const double h = h2 * ih;
+      const double rr = k * h, zz = k * zs;
+      // no horizontal derivative at r = 0 (Green_wave.f90:186)
+      const double unit = rr > 16 * kEpsilon ? ih : 0.0;
+      // along the unit vector and z: K's direction of this entry (A) and of the mirrored one (B)
+      const double hI = (nI[0] * dx + nI[1] * dy) * unit, hJ = -(f.dn[0] * dx + f.dn[1] * dy) * unit;
+      const double hA = adjoint ? hI : hJ, vA = adjoint ? nI[2] : f.dn[2];
+      const double hB = adjoint ? hJ : hI, vB = adjoint ? f.dn[2] : nI[2];
+      double cJ = kMinusOneOverFourPi * k * f.w, cB = cI;
+      WavePair w;
+      if (rr < kLit1em10 && fabs(zz) < kLit1em10) {
+        // Green_wave.f90:128-158, panel on the free surface with itself; its
+        // value takes the panel's area in place of the quadrature weight and
+        // its derivative along z has a term in 4 sqrt(pi area)
+        const double c = kMinusOneOverFourPi * k;
+        cJ = c * f.area;
+        cB = c * areaI;
+        w.g_re = (1 - log(k * k * f.area / kPI)) + 2 * (kEulerGamma - kLog2);
+        w.g_im = -2 * kPI;
+        w.h_re = w.h_im = 0.0;
+        w.v_re = w.g_re + 4 * sqrt(kPI * f.area) / (k * f.area);
+        w.v_im = w.g_im;
+      } else {
+        w = wave_pair<HIGH>(rr, zz, k, inv_k, inv_R, P);
+      }
+      const double sre = fma(cJ, w.g_re, kMinusOneOverFourPi * rk.x), sim = cJ * w.g_im;
+      const double ckJ = cJ * k;
+      double kre = fma(ckJ, hA * w.h_re + vA * w.v_re, kMinusOneOverFourPi * rk.y);
+      const double kim = ckJ * (hA * w.h_im + vA * w.v_im);
+      if (mirrored) {
+        const double ckI = cB * k;
+        mS[u * kMirLd + lane] = make_double2(cB * w.g_re, cB * w.g_im);
+        mK[u * kMirLd + lane] =
+            make_double2(ckI * (hB * w.h_re + vB * w.v_re), ckI * (hB * w.h_im + vB * w.v_im));
+      }
+      // matrices.f90:348: the centre of face I (= J) of mesh2
+      if (a.diagonal_term && I == J) kre += (fabs(f.zc - a.free_surface) < kLit1em8) ? 1.0 : 0.5;
+      if (row_ok) {
+        S[(size_t)I + (size_t)a.lds * J] = make_double2(sre, sim);
+        K[(size_t)I + (size_t)a.ldk * J] = make_double2(kre, kim);
+        if (W) {
+          const size_t wi = (size_t)I + (size_t)kb.w_ld * J;
+          W[wi] = (float)kre;
+          W[kb.w_im + wi] = (float)kim;
+        }
+        nan_max = nan_track(nan_track(nan_track(nan_track(nan_max, sre), sim), kre), kim);
+      }
+    }
+    if (mirrored) {
+      __syncwarp();
+      // mirrored entries: rows J0 + jc + u, columns I0 + c; 8 lanes per column
+      const int u = lane & (kPairChunk - 1);
+      const int J = J0 + jc + u;
+      if (jc + u < nJ) {
+#pragma unroll 2
+        for (int c = lane / kPairChunk; c < 32; c += 32 / kPairChunk) {
+          const int col = I0 + c;
+          if (col >= N) break;
+          const size_t ridx = (size_t)J + (size_t)rank_ld * col;
+          const double2 rk = INPLACE ? rank[ridx] : __ldg(rank + ridx);
+          const double2 ms = mS[u * kMirLd + c], mk = mK[u * kMirLd + c];
+          const double sre = fma(kMinusOneOverFourPi, rk.x, ms.x), kre = fma(kMinusOneOverFourPi, rk.y, mk.x);
+          S[(size_t)J + (size_t)a.lds * col] = make_double2(sre, ms.y);
+          K[(size_t)J + (size_t)a.ldk * col] = make_double2(kre, mk.y);
+          if (W) {
+            const size_t wi = (size_t)J + (size_t)kb.w_ld * col;
+            W[wi] = (float)kre;
+            W[kb.w_im + wi] = (float)mk.y;
+          }
+          nan_max = nan_track(nan_track(nan_track(nan_track(nan_max, sre), ms.y), kre), mk.y);
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (nan_max >= 0x7ff80000u && a.nan_flag_dev) atomicOr(a.nan_flag_dev, 1);
+}
+
+// Columns per warp of wave_pairs_kernel: the whole 128-column tile when the
+// tiles fill the GPU several times over (a wider share reads its rows' points
+// and the header once for more columns), else as few as 8, so that there are
+// about eight CTAs per SM: a mesh of 100 panels at one wavenumber is one tile,
+// 245 us with its columns in sequence and 8 us in 13 shares of 8.
+int pair_chunk(long long tiles_times_wavenumbers) {
+  int cw = kSymT;
+  while (cw > kPairChunk && tiles_times_wavenumbers * (kSymT / cw) < 148 * 8) cw /= 2;
+  return cw;
+}
+
 // ---- finite depth (Delhommeau's method) -------------------------------------
 // Green_Rankine.f90:202-338: Rankine term at the image (x, y, c0 z + c1) of M,
 // exact or one point by the distance to the face (one point when forced).
@@ -1218,6 +1470,15 @@ extern "C" int bem_assemble_rankine_part(const bem_assembly_args* args, void* ou
 
 namespace bem {
 namespace {
+PackedTab packed_tab(const bem_assembly_args& a) {
+  PackedTab P{};
+  P.base = a.nr > 2 && a.nz > 2 ? a.packed_table_dev : nullptr;
+  P.nr = a.nr;
+  P.nz = a.nz;
+  P.grid = a.tabulation_grid_shape;
+  return P;
+}
+
 // Shared by the single- and multi-wavenumber entry points: checks, then one
 // launch per group of up to kSymBatch wavenumbers (grid z = wavenumber).
 // planes (optional): float32 copy of K into planes[0 .. nk) (real plane, the
@@ -1273,6 +1534,10 @@ int wave_symmetric_launch(const bem_assembly_args* args, const void* rankine_dev
     std::snprintf(msg, sizeof(msg), "%s: tabulation pointers missing", who);
     return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
   }
+  if (tabulated && (uintptr_t)a.packed_table_dev % 32) {
+    std::snprintf(msg, sizeof(msg), "%s: packed_table_dev must be 32-byte aligned", who);
+    return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
+  }
   if (!tabulated && a.tabulation_nb_integration_points <= 0) {
     std::snprintf(msg, sizeof(msg), "%s: nb_integration_points <= 0", who);
     return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
@@ -1287,6 +1552,10 @@ int wave_symmetric_launch(const bem_assembly_args* args, const void* rankine_dev
                   a.z_range_dev, a.table_dev, a.table32_dev, 0.0, 0.0, a.r_inv_den_dev, a.z_inv_den_dev, 0.0};
   const int nbi = ceil_div(a.n, kSymT), nbj = ceil_div(general ? a.nb_faces : a.n, kSymT);
   cudaStream_t s = (cudaStream_t)stream;
+  // the packed table where there is one; the plain-table kernel serves hosts
+  // that pass none, the float32 wave term and the direct integration
+  const PackedTab P = packed_tab(a);
+  const bool packed = P.base && !f32 && tabulated;
   int launches = 0;
   for (int k0 = 0; k0 < nk; k0 += kSymBatch) {
     const int cnt = std::min(kSymBatch, nk - k0);
@@ -1303,7 +1572,18 @@ int wave_symmetric_launch(const bem_assembly_args* args, const void* rankine_dev
     ak.K_dev = reinterpret_cast<double2*>(a.K_dev) + (size_t)k0 * k_stride;
     {
       TimedLaunch tl(kKAssemble, s);
-      if (f32 && !general && !inplace)
+      const double2* rank = (const double2*)rankine_dev;
+      if (packed) {
+        const long long tiles = general ? (long long)nbi * nbj : (long long)nbi * (nbi + 1) / 2;
+        const int cw = pair_chunk(tiles * cnt);
+        const dim3 grid((unsigned)(tiles * cnt * (kSymT / cw)));
+        const bool high = a.gf_singularities == kHighFreq;
+        auto* kernel = general   ? (high ? wave_pairs_kernel<true, false, true> : wave_pairs_kernel<true, false, false>)
+                       : inplace ? (high ? wave_pairs_kernel<false, true, true> : wave_pairs_kernel<false, true, false>)
+                                 : (high ? wave_pairs_kernel<false, false, true>
+                                         : wave_pairs_kernel<false, false, false>);
+        kernel<<<grid, kPairRows, 0, s>>>(ak, P, kb, rank, ld, cw, nbi, cnt);
+      } else if (f32 && !general && !inplace)
         wave_symmetric_kernel<false, false, true><<<dim3(nbi, nbj, cnt), kSymT, 0, s>>>(
             ak, T, kb, a.gf_singularities, (const double2*)rankine_dev, ld);
       else if (f32 && !general)
@@ -1444,6 +1724,71 @@ extern "C" int bem_assemble_finite_depth(const bem_assembly_args* args, double d
       assemble_finite_depth_kernel<float2><<<grid, kRows, 0, s>>>(a, T, depth, method == 0 ? 1 : 0, prony_dev, nexp,
                                                                   gf_sing);
   }
+  count_launches(1);
+  BEM_CUDA_CHECK(cudaGetLastError());
+  return BEM_OK;
+}
+
+namespace bem {
+namespace {
+// One thread per node of the table, r grid and z grid first (packed_table.cuh).
+__global__ void pack_table_kernel(const double* __restrict__ r_range, int nr, const double* __restrict__ z_range,
+                                  int nz, const double* __restrict__ table, double* __restrict__ out) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx == 0) {
+    TabView T{};
+    T.nr = nr;
+    T.nz = nz;
+    T.r_range = r_range;
+    T.z_range = z_range;
+    tab_prologue(T);
+    out[0] = T.rmax;
+    out[1] = fabs(T.zlast);
+    out[2] = T.dz;
+    out[3] = T.r_slope;
+    out[4] = T.index_of_1;
+    for (int i = 5; i < kPackHeader; ++i) out[i] = 0.0;
+  }
+  if (idx < nr + nz) {
+    const bool is_r = idx < nr;
+    const double* u = is_r ? r_range : z_range;
+    const int n = is_r ? nr : nz, c = (int)(is_r ? idx : idx - nr);
+    double* rec = out + kPackHeader + 4 * idx;
+    rec[0] = rec[1] = rec[2] = rec[3] = 0.0;
+    if (c >= 1 && c + 1 < n) {
+      const double lower = u[c] - u[c - 1], upper = u[c + 1] - u[c], rho = lower / upper;
+      rec[0] = u[c];
+      rec[1] = 1.0 / upper;
+      rec[2] = rho;
+      rec[3] = 1.0 / (rho * (1.0 + rho));
+    }
+  }
+  if (idx < (long long)nr * nz) {
+    const double* t = table + kNbTab * idx;
+    double* low = out + kPackHeader + 4 * (nr + nz) + 4 * idx;
+    double* high = low + 4 * (long long)nr * nz;
+    low[0] = t[0];
+    high[0] = t[1];
+    for (int i = 1; i < 4; ++i) low[i] = high[i] = t[i + 1];
+  }
+}
+}  // namespace
+}  // namespace bem
+
+extern "C" int64_t bem_packed_table_bytes(int nr, int nz) {
+  return nr > 2 && nz > 2 ? 8 * bem::packed_table_doubles(nr, nz) : 0;
+}
+
+extern "C" int bem_pack_table(const double* r_range_dev, int nr, const double* z_range_dev, int nz,
+                              const double* table_dev, void* packed_dev, void* stream) {
+  using namespace bem;
+  if (nr <= 2 || nz <= 2 || !r_range_dev || !z_range_dev || !table_dev || !packed_dev)
+    return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_pack_table: null pointer or a grid of less than 3 values");
+  if ((uintptr_t)packed_dev % 32)
+    return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_pack_table: packed_dev must be 32-byte aligned");
+  const long long items = std::max((long long)nr * nz, (long long)nr + nz);
+  pack_table_kernel<<<ceil_div(items, 256), 256, 0, (cudaStream_t)stream>>>(r_range_dev, nr, z_range_dev, nz,
+                                                                            table_dev, (double*)packed_dev);
   count_launches(1);
   BEM_CUDA_CHECK(cudaGetLastError());
   return BEM_OK;

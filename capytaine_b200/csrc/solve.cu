@@ -92,6 +92,7 @@ struct bem_context {
   double* r_dev;
   double* z_dev;
   double* table_dev;
+  double* packed_dev;  // table_dev packed for the assembly (NULL: grids too small for it)
 };
 
 struct bem_lu {
@@ -157,6 +158,7 @@ bem_assembly_args base_args(const bem_context* ctx, int n, const double* centers
   a.z_range_dev = ctx->z_dev;
   a.table_dev = ctx->table_dev;
   a.table32_dev = nullptr;
+  a.packed_table_dev = ctx->table_dev ? ctx->packed_dev : nullptr;
   a.wavenumber = 1.0;
   a.free_surface = 0.0;
   a.gf_singularities = variant;
@@ -412,7 +414,7 @@ extern "C" int bem_context_create(int device, const bem_green_function_params* p
   ctx->params = *params;
   ctx->nr = params->tabulation_nr;
   ctx->nz = params->tabulation_nz;
-  ctx->r_dev = ctx->z_dev = ctx->table_dev = nullptr;
+  ctx->r_dev = ctx->z_dev = ctx->table_dev = ctx->packed_dev = nullptr;
   if (ctx->nr > 1 && ctx->nz > 1) {
     std::vector<double> r(ctx->nr), z(ctx->nz);
     if ((st = bem_default_r_spacing(ctx->nr, params->tabulation_rmax, params->tabulation_grid_shape, r.data())))
@@ -422,16 +424,21 @@ extern "C" int bem_context_create(int device, const bem_green_function_params* p
     BEM_CUDA_CHECK(cudaMalloc(&ctx->r_dev, r.size() * sizeof(double)));
     cudaError_t e = cudaMalloc(&ctx->z_dev, z.size() * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->table_dev, (size_t)ctx->nr * ctx->nz * 5 * sizeof(double));
+    const int64_t packed_bytes = bem_packed_table_bytes(ctx->nr, ctx->nz);
+    if (e == cudaSuccess && packed_bytes) e = cudaMalloc(&ctx->packed_dev, (size_t)packed_bytes);
     if (e == cudaSuccess) e = cudaMemcpy(ctx->r_dev, r.data(), r.size() * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(ctx->z_dev, z.data(), z.size() * sizeof(double), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
       cudaFree(ctx->r_dev);
       cudaFree(ctx->z_dev);
       cudaFree(ctx->table_dev);
+      cudaFree(ctx->packed_dev);
       return set_cuda_error(e, "bem_context_create: tabulation buffers");
     }
     st = bem_construct_tabulation(ctx->r_dev, ctx->nr, ctx->z_dev, ctx->nz, params->tabulation_nb_integration_points,
                                   ctx->table_dev, nullptr);
+    if (st == BEM_OK && ctx->packed_dev)
+      st = bem_pack_table(ctx->r_dev, ctx->nr, ctx->z_dev, ctx->nz, ctx->table_dev, ctx->packed_dev, nullptr);
     if (st == BEM_OK) {
       e = cudaDeviceSynchronize();
       if (e != cudaSuccess) st = set_cuda_error(e, "bem_context_create: tabulation");
@@ -440,6 +447,7 @@ extern "C" int bem_context_create(int device, const bem_green_function_params* p
       cudaFree(ctx->r_dev);
       cudaFree(ctx->z_dev);
       cudaFree(ctx->table_dev);
+      cudaFree(ctx->packed_dev);
       return st;
     }
   }
@@ -470,6 +478,12 @@ extern "C" int bem_context_set_tabulation(bem_context* ctx, const double* table_
   if (dg.status != cudaSuccess) return set_cuda_error(dg.status, "cudaSetDevice");
   BEM_CUDA_CHECK(cudaMemcpy(ctx->table_dev, table_host, (size_t)ctx->nr * ctx->nz * 5 * sizeof(double),
                             cudaMemcpyHostToDevice));
+  if (ctx->packed_dev) {
+    const int st =
+        bem_pack_table(ctx->r_dev, ctx->nr, ctx->z_dev, ctx->nz, ctx->table_dev, ctx->packed_dev, nullptr);
+    if (st) return st;
+    BEM_CUDA_CHECK(cudaDeviceSynchronize());
+  }
   return BEM_OK;
 }
 
@@ -611,6 +625,7 @@ extern "C" int bem_release(void* handle) {
     cudaFree(ctx->r_dev);
     cudaFree(ctx->z_dev);
     cudaFree(ctx->table_dev);
+    cudaFree(ctx->packed_dev);
     ctx->magic = 0;
     delete ctx;
     return BEM_OK;

@@ -122,6 +122,7 @@ class Delhommeau:
         self._tab_host = None
         self._dev_tab = None
         self._dev_tab_inv = (0, 0)
+        self._dev_tab_packed = 0
         self._mesh_cache: "OrderedDict[str, DeviceMesh]" = OrderedDict()
         # The caches are shared by the threads (and CUDA streams) of a request
         # server: dictionary updates under this lock, device readiness through
@@ -270,6 +271,8 @@ class Delhommeau:
         # reciprocal denominators of the Lagrange weights of both grids: the
         # lookup multiplies instead of dividing (bem_tabulation_inverse_denominators)
         self._dev_tab_inv = (0, 0)
+        self._dev_tab_packed = 0
+        extra = ()
         if nr > 2 and nz > 2:
             inv = []
             for rng in (np.ascontiguousarray(self.tabulated_r_range, dtype=np.float64),
@@ -281,7 +284,13 @@ class Delhommeau:
                 inv.append(torch.as_tensor(out, device=dev))
             self._dev_tab_inv_tensors = tuple(inv)
             self._dev_tab_inv = tuple(t.data_ptr() for t in inv)
-        self._dev_tab_shared = _lib.StreamShared(*self._dev_tab)
+            packed = torch.empty(int(_lib.load().bem_packed_table_bytes(nr, nz)), dtype=torch.uint8, device=dev)
+            _lib.call("bem_pack_table", _lib.ptr(r), nr, _lib.ptr(z), nz, _lib.ptr(table), _lib.ptr(packed),
+                      _lib.stream_ptr())
+            self._dev_tab_packed_tensor = packed
+            self._dev_tab_packed = packed.data_ptr()
+            extra = (*inv, packed)
+        self._dev_tab_shared = _lib.StreamShared(*self._dev_tab, *extra)
 
     @property
     def tabulated_integrals(self) -> np.ndarray:
@@ -409,6 +418,7 @@ class Delhommeau:
             table32_dev=table32.data_ptr() if table32 is not None else 0,
             r_inv_den_dev=self._dev_tab_inv[0] if table is not None else 0,
             z_inv_den_dev=self._dev_tab_inv[1] if table is not None else 0,
+            packed_table_dev=self._dev_tab_packed if table is not None else 0,
             wavenumber=wavenumber, free_surface=float(free_surface), gf_singularities=_SING[sing],
             adjoint_double_layer=int(bool(adjoint_double_layer)), early_dot_product=int(bool(early_dot_product)),
             diagonal_term=int(bool(diagonal_term_in_double_layer)),
@@ -566,6 +576,7 @@ class Delhommeau:
             table32_dev=table32.data_ptr() if table32 is not None else 0,
             r_inv_den_dev=self._dev_tab_inv[0] if table is not None else 0,
             z_inv_den_dev=self._dev_tab_inv[1] if table is not None else 0,
+            packed_table_dev=self._dev_tab_packed if table is not None else 0,
             wavenumber=k, free_surface=float(free_surface), gf_singularities=_SING[sing],
             adjoint_double_layer=int(bool(adjoint_double_layer)), early_dot_product=int(bool(early_dot_product)),
             diagonal_term=int(bool(diagonal_term_in_double_layer)), precision=_lib.BEM_PREC_FP64,

@@ -89,6 +89,16 @@ int bem_construct_tabulation(const double* r_range_dev, int nr, const double* z_
  * weights change by an ulp at most.  No counterpart in the reference. */
 int bem_tabulation_inverse_denominators(const double* range_host, int n, double* out_host);
 
+/* The table packed for the assembly (bem_assembly_args packed_table_dev): the
+ * stencils of both grids with their reciprocal denominators, and the four
+ * integrals that a variant of the Green function reads in one 32-byte quad per
+ * node, for low_freq and for high_freq.  bem_packed_table_bytes gives the size
+ * (0 when a grid has less than 3 values); packed_dev must be 32-byte aligned.
+ * No counterpart in the reference. */
+int64_t bem_packed_table_bytes(int nr, int nz);
+int bem_pack_table(const double* r_range_dev, int nr, const double* z_range_dev, int nz, const double* table_dev,
+                   void* packed_dev, void* stream);
+
 /* ---- assembly of the influence matrices ----------------------------------- */
 typedef struct {
   /* collocation side (mesh1 or a raw list of points) */
@@ -136,6 +146,9 @@ typedef struct {
    * (3 per node, bem_tabulation_inverse_denominators); NULL: divided each time */
   const double* r_inv_den_dev;     /* (nr, 3)                                                  */
   const double* z_inv_den_dev;     /* (nz, 3)                                                  */
+  /* optional: the table packed by bem_pack_table from the same grids and table
+   * (32-byte aligned); NULL: the wave term reads the plain table              */
+  const double* packed_table_dev;
 } bem_assembly_args;
 
 /* S and K (or D, or the full gradient) for one wavenumber, infinite depth.
