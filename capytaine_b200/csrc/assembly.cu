@@ -395,16 +395,13 @@ struct OutT<float2> {
   __device__ static float2 make(double re, double im) { return make_float2((float)re, (float)im); }
 };
 
-// RANKINE_PART: write only the wavenumber-independent Rankine part of each
-// entry, unscaled, to rank_out(I, J) = (sum of the direct and reflected Rankine
-// G, dot normal . their gradient) with the same arithmetic as the full entry.
-template <class Out, bool MIXED, bool RANKINE_PART = false>
+// The float32 wave term (BEM_PREC_MIXED) of any points against a mesh, every
+// entry on its own; the Rankine terms stay float64.
 // Four CTAs per SM (128 registers, a small spill): measured 12% faster than the
 // three that 168 registers allow on this FP64-latency-bound kernel.
+template <class Out>
 __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_args a, TabView T, double k_wave,
-                                                         int gf_sing, bool finite_k, double sign_refl,
-                                                         double2* __restrict__ rank_out = nullptr,
-                                                         int64_t rank_ld = 0) {
+                                                         int gf_sing, bool finite_k, double sign_refl) {
   __shared__ FaceRec faces[kTileJ];
   if (T.nr > 1 && T.nz > 1) {
     // Grid bounds of the tabulation (last r and z values).
@@ -454,7 +451,7 @@ __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_a
   Out* S = reinterpret_cast<Out*>(a.S_dev);
   Out* K = reinterpret_cast<Out*>(a.K_dev);
   bool nan_seen = false;
-  using R = typename std::conditional<MIXED, float, double>::type;
+  using R = float;
 
   for (int jj = 0; jj < nJ; ++jj) {
     const FaceRec& f = faces[jj];
@@ -503,7 +500,7 @@ __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_a
       dGre[2] += sign_refl * dGf[2];
       if (gf_sing == kLowFreqWithRankinePart) dGre[2] += 2 * k_wave * Gf;
       // ---- wave term --------------------------------------------------------
-      if (finite_k && !RANKINE_PART) {
+      if (finite_k) {
         const double dxh = M[0] - f.c[0], dyh = M[1] - f.c[1];
         const double rr = k_wave * norm2_2(dxh, dyh);
         const double zz = k_wave * (M[2] + f.c[2]);
@@ -546,13 +543,6 @@ __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_a
       dGim[0] = -dGim[0];
       dGim[1] = -dGim[1];
       dGre[2] = dGre[2] - 2 * dGr[2];
-    }
-    if constexpr (RANKINE_PART) {
-      const double* dn = adjoint ? nI : (a.dot_normals_dev + 3 * J);
-      const double kdot = dn[0] * dGre[0] + dn[1] * dGre[1] + dn[2] * dGre[2];
-      rank_out[(size_t)I + (size_t)rank_ld * J] = make_double2(Gre, kdot);
-      nan_seen |= isnan(Gre) || isnan(kdot);
-      continue;
     }
     const double sre = kMinusOneOverFourPi * Gre, sim = kMinusOneOverFourPi * Gim;
     const size_t sidx = (size_t)I + (size_t)a.lds * J;
@@ -881,19 +871,24 @@ __global__ void __launch_bounds__(kSymT, 5) wave_symmetric_kernel(bem_assembly_a
 // ---- wave term from the packed table ----------------------------------------
 // Nodes of the stencil by the packed table's estimates, decided by the float64
 // expressions next to a rounding boundary.
-__device__ __forceinline__ void packed_integrals(double r, double z, const PackedTab& P, bool high, double out[4]) {
-  if (fabs(z) < P.zmax && r < P.rmax) {
-    const int i = packed_r_node(r, P, [&](double x) { return nearest_r_index(x, P.nr, P.rmax, P.grid); });
-    const int j = packed_z_node(z, P, [&](double x) { return nearest_z_index(x, P.nz, -P.zmax, P.grid, P.dz); });
-    packed_interpolate(r, z, i, j, P, out);
-    return;
-  }
+__device__ __forceinline__ void packed_beyond(double r, double z, bool high, double out[4]) {
   double I[5];
   asymptotic<double>(r, z, I);
   out[0] = high ? I[1] : I[0];
   out[1] = I[2];
   out[2] = I[3];
   out[3] = I[4];
+}
+__device__ __forceinline__ void packed_integrals(double r, double z, const PackedTab& P, bool high, double out[4]) {
+  if (fabs(z) < P.zmax && r < P.rmax) {
+    const int i = packed_r_node(r, P, [&](double x) { return nearest_r_index(x, P.nr, P.rmax, P.grid); });
+    const int j = packed_z_node(z, P, [&](double x) { return nearest_z_index(x, P.nz, -P.zmax, P.grid, P.dz); });
+    double wr[3];
+    packed_weights(P.r_rec + 4 * (i - 1), r, wr);
+    packed_interpolate(wr, z, i, j, P, out);
+    return;
+  }
+  packed_beyond(r, z, high, out);
 }
 
 // The wave term of one pair of points for a unit weight, before the factor
@@ -1129,241 +1124,461 @@ int pair_chunk(long long tiles_times_wavenumbers) {
   return cw;
 }
 
-// ---- finite depth (Delhommeau's method) -------------------------------------
-// Green_Rankine.f90:202-338: Rankine term at the image (x, y, c0 z + c1) of M,
-// exact or one point by the distance to the face (one point when forced).
-__device__ __forceinline__ void reflected_rankine(const double M[3], const FaceRec& f, bool deriv_first, double c0,
-                                                  double c1, bool one_point, double& G, double dG[3]) {
-  const double Mr[3] = {M[0], M[1], c0 * M[2] + c1};
-  const double r1 = hypot(norm2_2(M[0] - f.c[0], M[1] - f.c[1]), Mr[2] - f.c[2]);
-  if (one_point || r1 > 7 * f.radius) {
-    one_point_rankine<double>(f.c[0] - Mr[0], f.c[1] - Mr[1], f.c[2] - Mr[2], f.area, G, dG);
-  } else {
-    exact_rankine(Mr, f, true, G, dG);
-  }
-  dG[2] = c0 * dG[2];
-  if (!deriv_first) {
-    dG[0] = -dG[0];
-    dG[1] = -dG[1];
-    if (c0 > 0) dG[2] = -dG[2];
-  }
-}
-
-// Green_wave.f90:50-124 for the point x and the face of centre c (quadrature
-// points of face J, each mirrored through the sea bottom when mirror_face).
-__device__ void wave_term(const double x[3], const double c[3], const bem_assembly_args& a, const FaceRec& f, int J,
-                          bool mirror_face, double depth, double k, const TabView& T, int sing, bool deriv_first,
-                          double& gre, double& gim, double dr[3], double di[3]) {
-  gre = gim = 0;
-  dr[0] = dr[1] = dr[2] = di[0] = di[1] = di[2] = 0;
-  const double rr = k * norm2_2(x[0] - c[0], x[1] - c[1]);
-  const double zz = k * (x[2] + c[2]);
-  if (fabs(rr) < kLit1em10 && fabs(zz) < kLit1em10) {
-    // Green_wave.f90:128-158, panel on the free surface with itself
-    const double re = (1 - log(k * k * f.area / kPI)) + 2 * (kEulerGamma - kLog2);
-    gre = k * f.area * re;
-    gim = k * f.area * (-2 * kPI);
-    dr[2] = k * (gre + 4 * sqrt(kPI * f.area));
-    di[2] = k * gim;
-  } else {
-    for (int q = 0; q < a.nb_quad_points; ++q) {
-      const double* qp = a.quad_points_dev + ((size_t)a.nb_quad_points * J + q) * 3;
-      const double xq[3] = {qp[0], qp[1], mirror_face ? -qp[2] - 2 * depth : qp[2]};
-      wave_part<double>(x, xq, k, T, sing, a.quad_weights_dev[(size_t)a.nb_quad_points * J + q], gre, gim, dr, di);
-    }
-  }
-  if (!deriv_first) {
-    dr[0] = -dr[0];
-    dr[1] = -dr[1];
-    di[0] = -di[0];
-    di[1] = -di[1];
-  }
-}
-
-// matrices.f90:28-325 in finite depth, Delhommeau's method: the
-// infinite-depth Rankine terms, the Rankine images through the sea bottom
-// (matrices.f90:212-268), the four wave terms of Green_wave.f90:311-425 and the
-// Prony terms of Green_wave.f90:427-508.  One thread per collocation point,
-// the panels of a tile in shared memory; every term in float64, outputs Out
-// (complex128 or complex64), K with the dot product taken or the three
-// gradient planes, as the general kernel.  prony: rates then amplitudes
-// (2 x nexp).
-template <class Out>
-__global__ void __launch_bounds__(kRows) assemble_finite_depth_kernel(const bem_assembly_args a, TabView T,
-                                                                      double depth, int legacy,
-                                                                      const double* __restrict__ prony, int nexp,
-                                                                      int gf_sing) {
-  __shared__ FaceRec faces[kTileJ];
-  if (T.nr > 1 && T.nz > 1) {
-    tab_prologue(T);
-  }
-  const int J0 = blockIdx.y * kTileJ;
-  const int nJ = min(kTileJ, a.nb_faces - J0);
-  if ((int)threadIdx.x < nJ) {
-    const int J = J0 + threadIdx.x;
-    FaceRec& f = faces[threadIdx.x];
+// ---- one entry at a time: any points, any depth --------------------------------
+// The tile's panels with what the exact integrals need of each edge, computed
+// once per panel instead of once per pair: its length (DK) and the vector
+// n x edge / DK (GYX of Green_Rankine.f90:104-109).
+struct EntryFace {
+  double v[12], c[3], n[3], q0[3];
+  double gyx[12], dk[4];
+  double area, radius, w0;
+  double far2;  // (7 radius)^2
+};
+__device__ __forceinline__ void load_entry_face(const bem_assembly_args& a, int J, EntryFace& f) {
 #pragma unroll
-    for (int L = 0; L < 4; ++L) {
-      const int v = a.faces_dev[4 * J + L];
-      f.v[3 * L] = a.vertices_dev[3 * v];
-      f.v[3 * L + 1] = a.vertices_dev[3 * v + 1];
-      f.v[3 * L + 2] = a.vertices_dev[3 * v + 2];
+  for (int L = 0; L < 4; ++L) {
+    const int v = a.faces_dev[4 * J + L];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f.v[3 * L + d] = a.vertices_dev[3 * v + d];
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    f.c[d] = a.centers_dev[3 * J + d];
+    f.n[d] = a.normals_dev[3 * J + d];
+    f.q0[d] = a.quad_points_dev[(size_t)3 * a.nb_quad_points * J + d];
+  }
+  f.area = a.areas_dev[J];
+  f.radius = a.radii_dev[J];
+  f.w0 = a.quad_weights_dev[(size_t)a.nb_quad_points * J];
+  f.far2 = (7 * f.radius) * (7 * f.radius);
+#pragma unroll
+  for (int L = 0; L < 4; ++L) {
+    const int Ln = (L + 1) & 3;
+    const double e0 = f.v[3 * Ln] - f.v[3 * L], e1 = f.v[3 * Ln + 1] - f.v[3 * L + 1],
+                 e2 = f.v[3 * Ln + 2] - f.v[3 * L + 2];
+    const double DK = dnorm3(e0, e1, e2);
+    const double PJ0 = e0 / DK, PJ1 = e1 / DK, PJ2 = e2 / DK;
+    f.dk[L] = DK;
+    f.gyx[3 * L] = f.n[1] * PJ2 - f.n[2] * PJ1;
+    f.gyx[3 * L + 1] = f.n[2] * PJ0 - f.n[0] * PJ2;
+    f.gyx[3 * L + 2] = f.n[0] * PJ1 - f.n[1] * PJ0;
+  }
+}
+
+// Green_Rankine.f90:68-157, derivative with respect to M.  The edges in a
+// loop: one copy of the logarithm and the arctangent in the kernel.
+__device__ __forceinline__ void exact_rankine_edges(const double M[3], const EntryFace& f, double& G, double dG[3]) {
+  const double n0 = f.n[0], n1 = f.n[1], n2 = f.n[2];
+  const double GZ = (M[0] - f.c[0]) * n0 + (M[1] - f.c[1]) * n1 + (M[2] - f.c[2]) * n2;
+  G = 0.0;
+  dG[0] = dG[1] = dG[2] = 0.0;
+  const double sgn = copysign(1.0, GZ), aGZ = fabs(GZ);
+  const bool use_atan = aGZ >= kLit1em4 * f.radius;
+  double x0 = M[0] - f.v[0], x1 = M[1] - f.v[1], x2 = M[2] - f.v[2];
+  double RR = dnorm3(x0, x1, x2), inv = 1.0 / RR;
+#pragma unroll 1
+  for (int L = 0; L < 4; ++L) {
+    const int Ln = (L + 1) & 3;
+    const double y0 = M[0] - f.v[3 * Ln], y1 = M[1] - f.v[3 * Ln + 1], y2 = M[2] - f.v[3 * Ln + 2];
+    const double RN = dnorm3(y0, y1, y2), invN = 1.0 / RN;
+    const double DK = f.dk[L];
+    if (DK >= kLit1em3 * f.radius) {
+      const double GYX0 = f.gyx[3 * L], GYX1 = f.gyx[3 * L + 1], GYX2 = f.gyx[3 * L + 2];
+      const double GY = x0 * GYX0 + x1 * GYX1 + x2 * GYX2;
+      const double S = RN + RR;
+      const double ANT = 2 * GY * DK;
+      const double DNT = S * S - DK * DK + 2 * aGZ * S;
+      const double ANL = S + DK;
+      const double DNL = S - DK;
+      const double ALDEN = log(ANL / DNL);
+      const double AT = use_atan ? atan(ANT / DNT) : 0.0;
+      const double ANLX0 = y0 * invN + x0 * inv, ANLX1 = y1 * invN + x1 * inv, ANLX2 = y2 * invN + x2 * inv;
+      const double two_dk = 2 * DK;
+      const double a1 = 2 * (S + aGZ), a2 = 2 * sgn * S;
+      const double DNTX0 = a1 * ANLX0 + a2 * n0;
+      const double DNTX1 = a1 * ANLX1 + a2 * n1;
+      const double DNTX2 = a1 * ANLX2 + a2 * n2;
+      G = G - 2 * AT * aGZ;
+      if (!(fabs(GY) < kLit1em5)) G = G + GY * ALDEN;
+      const double c1 = GY * (DNL - ANL) / (ANL * DNL);
+      const double cA = 2 * sgn * AT;
+      const double cB = 2 * aGZ / (ANT * ANT + DNT * DNT);
+      dG[0] += ALDEN * GYX0 - cA * n0 + c1 * ANLX0 - cB * (two_dk * GYX0 * DNT - DNTX0 * ANT);
+      dG[1] += ALDEN * GYX1 - cA * n1 + c1 * ANLX1 - cB * (two_dk * GYX1 * DNT - DNTX1 * ANT);
+      dG[2] += ALDEN * GYX2 - cA * n2 + c1 * ANLX2 - cB * (two_dk * GYX2 * DNT - DNTX2 * ANT);
     }
+    x0 = y0;
+    x1 = y1;
+    x2 = y2;
+    RR = RN;
+    inv = invN;
+  }
+}
+
+// Rankine images of a point: the point itself (c0 = 1, c1 = 0), then its images
+// (x, y, c0 z + c1) in the free surface, the sea bottom and both, and those of
+// the Prony terms, each with its weight (Green_Rankine.f90:202-338,
+// matrices.f90:212-268, Green_wave.f90:427-508).
+struct RankineImage {
+  double c0, c1, weight;
+  double exact;  // 1: the exact integral near the panel, 0: one point always
+};
+constexpr int kMaxProny = 64;
+constexpr int kMaxImages = 6 + 4 * kMaxProny;
+
+enum WaveTable { kNoWave = 0, kPackedTable = 1, kPlainTable = 2 };
+
+struct EntryParams {
+  double depth;        // +inf: infinite depth
+  int images;          // 1: the images of finite depth, 0: the free surface's alone
+  int legacy;          // finite depth, legacy method: free-surface image by one point
+  const double* prony; // rates then amplitudes (2 x nexp)
+  int nexp;
+  int gf_sing;
+  double sign_refl;
+  int cw;              // columns per CTA
+  double2* rank_out;   // the Rankine part alone
+  int64_t rank_ld;
+};
+
+constexpr int kEntryCols = 32;   // most columns per CTA
+constexpr int kEntryQueue = 64;  // near pairs of a warp waiting
+
+// S and K (dot product taken or the three gradient planes) entry by entry:
+// matrices.f90:28-325 in infinite or finite depth (Delhommeau's method).  RANK:
+// only the wavenumber-independent Rankine part, unscaled, (G, dot normal .
+// gradient) to rank_out.
+// A warp owns 32 rows, one per lane, and walks the CTA's columns.  All the
+// images of a pair have the same horizontal distance, so that a far image costs
+// one square root and about ten multiply-adds, and the four wave terms of
+// finite depth share their radial stencil.  A pair with an image near the panel
+// (r <= 7 radii: about 1% of a mesh's pairs, but a tenth of the warp's columns
+// have one) waits in the warp's queue, until 32 of them are evaluated by a full
+// warp: the exact integrals (logarithms, arctangents, divisions) otherwise run
+// with most lanes idle and dominate the kernel.  Either way one lane computes
+// and stores the whole entry, in an order that does not depend on timing.
+// The distance threshold meets exact ties on regular meshes: within 1e-12 of it
+// the reference's own expressions decide.
+template <class Out, int WAVE, bool RANK>
+__global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_assembly_args a, TabView T,
+                                                                    PackedTab P, EntryParams e) {
+  __shared__ EntryFace faces[kEntryCols];
+  __shared__ double rows[kRows][6];  // point, dot normal
+  __shared__ RankineImage img[kMaxImages];
+  __shared__ unsigned short queue[4][kEntryQueue];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int J0 = blockIdx.y * e.cw;
+  const int nJ = min(e.cw, a.nb_faces - J0);
+  const bool adjoint = a.adjoint_double_layer != 0;
+  const bool rankine_only = isinf(a.free_surface);
+  const bool finite_depth = e.images != 0;
+  const double k = a.wavenumber;
+  const int nimg = rankine_only ? 1 : finite_depth ? 6 + 4 * e.nexp : 2;
+  for (int t = tid; t < nimg; t += kRows) {
+    RankineImage m{1.0, 0.0, 1.0, 1.0};
+    const double h = e.depth;
+    if (t == 1) m = RankineImage{-1.0, 0.0, e.sign_refl, e.legacy ? 0.0 : 1.0};
+    if (t == 2) m = RankineImage{-1.0, -2 * h, 1.0, 1.0};
+    if (t == 3) m = RankineImage{1.0, -2 * h, e.sign_refl, 0.0};
+    if (t == 4) m = RankineImage{1.0, 2 * h, e.sign_refl, 0.0};
+    if (t == 5) m = RankineImage{-1.0, -4 * h, e.sign_refl, 0.0};
+    if (t >= 6) {
+      const int x = (t - 6) >> 2, w = (t - 6) & 3;
+      const double lam = e.prony[x], half = e.prony[e.nexp + x] / 2;
+      m = w == 0   ? RankineImage{1.0, h * lam - 2 * h, half, 1.0}
+          : w == 1 ? RankineImage{-1.0, -h * lam, half, 1.0}
+          : w == 2 ? RankineImage{-1.0, h * lam - 4 * h, half, 1.0}
+                   : RankineImage{1.0, -h * lam + 2 * h, half, 1.0};
+    }
+    img[t] = m;
+  }
+  if (tid < nJ) load_entry_face(a, J0 + tid, faces[tid]);
+  const int I0 = blockIdx.x * kRows + warp * 32;
+  {
+    const int Ic = min(I0 + lane, a.n - 1);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      f.c[d] = a.centers_dev[3 * J + d];
-      f.n[d] = a.normals_dev[3 * J + d];
-      f.q0[d] = a.quad_points_dev[(size_t)3 * a.nb_quad_points * J + d];
+      rows[tid][d] = a.points_dev[3 * Ic + d];
+      rows[tid][3 + d] = adjoint && a.dot_normals_dev ? a.dot_normals_dev[3 * Ic + d] : 0.0;
     }
-    f.area = a.areas_dev[J];
-    f.radius = a.radii_dev[J];
-    f.w0 = a.quad_weights_dev[(size_t)a.nb_quad_points * J];
   }
   __syncthreads();
-  const int I = blockIdx.x * kRows + threadIdx.x;
-  if (I >= a.n) return;
-  const double M[3] = {a.points_dev[3 * I], a.points_dev[3 * I + 1], a.points_dev[3 * I + 2]};
-  const double Msym[3] = {M[0], M[1], -M[2] - 2 * depth};
-  const bool adjoint = a.adjoint_double_layer != 0;
-  double nI[3] = {0, 0, 0};
-  if (adjoint) {
-    nI[0] = a.dot_normals_dev[3 * I];
-    nI[1] = a.dot_normals_dev[3 * I + 1];
-    nI[2] = a.dot_normals_dev[3 * I + 2];
-  }
-  const double k = a.wavenumber;
-  const bool finite_k = k > 0.0 && isfinite(k);
-  const double sign_refl = (gf_sing == kHighFreq) ? -1.0 : 1.0;
-  const int diag_limit = min(a.n, a.nb_faces);
-  double diag_coef = 0.5;
-  if (a.diagonal_term && I < diag_limit)
-    diag_coef = (fabs(a.centers_dev[3 * I + 2] - a.free_surface) < kLit1em8) ? 1.0 : 0.5;
-  double A = 0.0;
-  if (finite_k) {
-    const double amh = k * depth;
+  if (I0 >= a.n) return;  // no barrier of the whole CTA below
+  if (WAVE == kPackedTable) P.load(e.gf_sing == kHighFreq);
+  if (WAVE == kPlainTable && T.nr > 1 && T.nz > 1) tab_prologue(T);
+  double wave_scale = 1.0;
+  if (WAVE != kNoWave && finite_depth) {
+    const double amh = k * e.depth;
     const double akh = amh * tanh(amh);
-    A = (amh + akh) * (amh + akh) / (4 * amh * (amh * amh - akh * akh + akh));
+    wave_scale = (amh + akh) * (amh + akh) / (4 * amh * (amh * amh - akh * akh + akh));
   }
   Out* S = reinterpret_cast<Out*>(a.S_dev);
   Out* K = reinterpret_cast<Out*>(a.K_dev);
+  const int diag_limit = min(a.n, a.nb_faces);
+  const bool no_z_term = e.gf_sing == kLowFreqWithRankinePart;
   bool nan_seen = false;
-  for (int jj = 0; jj < nJ; ++jj) {
-    const FaceRec& f = faces[jj];
-    const int J = J0 + jj;
-    double Gre = 0, Gim = 0, dGre[3] = {0, 0, 0}, dGim[3] = {0, 0, 0};
-    double g, dg[3];
-    // direct Rankine term
-    {
-      const double d0 = M[0] - f.c[0], d1 = M[1] - f.c[1], d2 = M[2] - f.c[2];
-      if (norm2_3(d0, d1, d2) > 7 * f.radius) {
-        one_point_rankine<double>(-d0, -d1, -d2, f.area, g, dg);
-      } else {
-        exact_rankine(M, f, true, g, dg);
-      }
-      if (!adjoint) {
-        dg[0] = -dg[0];
-        dg[1] = -dg[1];
-        dg[2] = -dg[2];
-      }
-      Gre += g;
-      dGre[0] += dg[0];
-      dGre[1] += dg[1];
-      dGre[2] += dg[2];
+  int jj = 0, waiting = 0;
+  while (jj < nJ || waiting > 0) {
+    // one column of the warp's 32 rows, or up to 32 waiting near pairs
+    const bool near_pass = waiting >= 32 || jj >= nJ;
+    int r = lane, c = jj;
+    bool active = I0 + lane < a.n;
+    if (near_pass) {
+      const int take = min(waiting, 32);
+      active = lane < take;
+      const int item = queue[warp][waiting - take + min(lane, take - 1)];
+      r = item & 31;
+      c = item >> 5;
+      waiting -= take;
+      __syncwarp();  // the slots may be filled again
+    } else {
+      ++jj;
     }
-    // free-surface image (one point in the legacy method), with the variant's sign
-    reflected_rankine(M, f, adjoint, -1.0, 0.0, legacy != 0, g, dg);
-    Gre += sign_refl * g;
-    dGre[0] += sign_refl * dg[0];
-    dGre[1] += sign_refl * dg[1];
-    dGre[2] += sign_refl * dg[2];
-    if (gf_sing == kLowFreqWithRankinePart) dGre[2] += 2 * k * g;
-    // sea-bottom image, then the images through both boundaries
-    reflected_rankine(M, f, adjoint, -1.0, -2 * depth, false, g, dg);
-    Gre += g;
-    dGre[0] += dg[0];
-    dGre[1] += dg[1];
-    dGre[2] += dg[2];
-    const double c_one_point[3][2] = {{1.0, -2 * depth}, {1.0, 2 * depth}, {-1.0, -4 * depth}};
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      reflected_rankine(M, f, adjoint, c_one_point[t][0], c_one_point[t][1], true, g, dg);
-      Gre += sign_refl * g;
-      dGre[0] += sign_refl * dg[0];
-      dGre[1] += sign_refl * dg[1];
-      dGre[2] += sign_refl * dg[2];
+    const EntryFace& f = faces[c];
+    const double* row = rows[32 * warp + r];
+    const double Mx = row[0], My = row[1], Mz = row[2];
+    const double dx = Mx - f.c[0], dy = My - f.c[1], cz = f.c[2];
+    const double h2 = dx * dx + dy * dy;
+    const double far_hi = f.far2 * (1.0 + 1e-12);
+    if (!near_pass) {
+      // near: an image may be within 7 radii (every image is as far as h2 at least)
+      const double z0 = Mz - cz, z1 = Mz + cz;
+      const bool near = active && !(h2 > far_hi) &&
+                        (finite_depth || !(h2 + z0 * z0 > far_hi) || (nimg > 1 && !(h2 + z1 * z1 > far_hi)));
+      const unsigned m = __ballot_sync(0xffffffffu, near);
+      if (near) queue[warp][waiting + __popc(m & ((1u << lane) - 1))] = (unsigned short)(c << 5 | r);
+      __syncwarp();
+      waiting += __popc(m);
+      if (near) active = false;
+      if (!__any_sync(0xffffffffu, active)) continue;
     }
-    // four infinite-depth wave terms (point, face, each possibly mirrored through the bottom)
-    if (finite_k) {
-      const double csym[3] = {f.c[0], f.c[1], -f.c[2] - 2 * depth};
-      double wre = 0, wim = 0, wdr[3] = {0, 0, 0}, wdi[3] = {0, 0, 0};
+    // ---- Rankine images: G, horizontal derivative H (dx, dy) + (E0, E1), vertical V
+    double G = 0, H = 0, V = 0, E0 = 0, E1 = 0;
+    if (!near_pass) {
+#pragma unroll 2
+      for (int t = 0; t < nimg; ++t) {
+        const RankineImage m = img[t];
+        const double vz = cz - fma(m.c0, Mz, m.c1);
+        const double ro2 = fma(vz, vz, h2);
+        // ro > 1e-7 (Green_Rankine.f90:185)
+        const double inv = ro2 > kLit1em7 * kLit1em7 ? rsqrt(ro2) : 0.0;
+        const double g = m.weight * f.area * inv;
+        const double s = g * (inv * inv);
+        G += g;
+        H -= s;
+        V = fma(s * vz, adjoint ? m.c0 : -1.0, V);
+        if (no_z_term && t == 1) V += 2 * k * (f.area * inv);
+      }
+    } else {
 #pragma unroll 1
-      for (int t = 0; t < 4; ++t) {
-        const bool mx = (t & 1) != 0, mf = (t & 2) != 0;
-        // z of the gradient mirrored: (x_sym, face) when deriv_first, (x, face_sym)
-        // otherwise, (x_sym, face_sym) always (Green_wave.f90:375-411)
-        const bool flip_z = (mx && mf) || (mx && adjoint) || (mf && !adjoint);
-        double gr, gi, dr[3], di[3];
-        wave_term(mx ? Msym : M, mf ? csym : f.c, a, f, J, mf, depth, k, T, gf_sing, adjoint, gr, gi, dr, di);
-        if (flip_z) {
-          dr[2] = -dr[2];
-          di[2] = -di[2];
+      for (int t = 0; t < nimg; ++t) {
+        const RankineImage m = img[t];
+        const double zi = fma(m.c0, Mz, m.c1);
+        const double vz = cz - zi;
+        const double ro2 = fma(vz, vz, h2);
+        bool far = m.exact == 0.0 || ro2 > far_hi;
+        if (!far && !(ro2 < f.far2 * (1.0 - 1e-12)))
+          far = (t == 0 ? norm2_3(dx, dy, Mz - cz) : hypot(norm2_2(dx, dy), zi - cz)) > 7 * f.radius;
+        double g, gz;
+        const double flip = adjoint ? m.c0 : -1.0;
+        if (far) {
+          const double inv = ro2 > kLit1em7 * kLit1em7 ? rsqrt(ro2) : 0.0;
+          g = f.area * inv;
+          const double s = g * (inv * inv);
+          H -= m.weight * s;
+          gz = s * vz;
+        } else {
+          const double Mi[3] = {Mx, My, zi};
+          double dg[3];
+          exact_rankine_edges(Mi, f, g, dg);
+          E0 += m.weight * dg[0];
+          E1 += m.weight * dg[1];
+          gz = dg[2];
         }
-        wre += gr;
-        wim += gi;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          wdr[d] += dr[d];
-          wdi[d] += di[d];
-        }
-      }
-      Gre += A * wre;
-      Gim += A * wim;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        dGre[d] += A * wdr[d];
-        dGim[d] += A * wdi[d];
+        G += m.weight * g;
+        V += m.weight * (flip * gz);
+        if (no_z_term && t == 1) V += 2 * k * g;
       }
     }
-    // Prony exponentials: four Rankine images each, weighted a / 2
-    for (int e = 0; e < nexp; ++e) {
-      const double lam = __ldg(prony + e), amp = __ldg(prony + nexp + e);
-      const double cp[4][2] = {{1.0, depth * lam - 2 * depth},
-                               {-1.0, -depth * lam},
-                               {-1.0, depth * lam - 4 * depth},
-                               {1.0, -depth * lam + 2 * depth}};
+    double gx = fma(H, dx, E0), gy = fma(H, dy, E1), gxi = 0, gyi = 0, Gi = 0, Vi = 0;
+    // ---- wave terms: one in infinite depth, four (point and face, each
+    // possibly mirrored in the bottom) in finite depth (Green_wave.f90:50-425)
+    const int J = J0 + c;
+    if (WAVE != kNoWave) {
+      const bool high = e.gf_sing == kHighFreq;
+      const double inv_k = 1.0 / k;
 #pragma unroll 1
-      for (int t = 0; t < 4; ++t) {
-        reflected_rankine(M, f, adjoint, cp[t][0], cp[t][1], false, g, dg);
-        Gre += amp / 2 * g;
-        dGre[0] += amp / 2 * dg[0];
-        dGre[1] += amp / 2 * dg[1];
-        dGre[2] += amp / 2 * dg[2];
+      for (int q = 0; q < a.nb_quad_points; ++q) {
+        double qx = f.q0[0], qy = f.q0[1], qz = f.q0[2], wq = f.w0;
+        if (q > 0) {
+          const double* qp = a.quad_points_dev + ((size_t)a.nb_quad_points * J + q) * 3;
+          qx = qp[0];
+          qy = qp[1];
+          qz = qp[2];
+          wq = a.quad_weights_dev[(size_t)a.nb_quad_points * J + q];
+        }
+        const double wx = Mx - qx, wy = My - qy;
+        const double w2 = wx * wx + wy * wy;
+        const double ih = w2 > 0.0 ? rsqrt(w2) : 0.0;
+        const double rr = k * (w2 * ih);
+        // no horizontal derivative at r = 0 (Green_wave.f90:186)
+        const double unit = rr > 16 * kEpsilon ? ih : 0.0;
+        // the panel's own term is at its centre (Green_wave.f90:75-80)
+        const bool axis = k * norm2_2(dx, dy) < kLit1em10;
+        int ri = 2;
+        double wr[3];
+        if (WAVE == kPackedTable && rr < P.rmax) {
+          ri = packed_r_node(rr, P, [&](double x) { return nearest_r_index(x, P.nr, P.rmax, P.grid); });
+          packed_weights(P.r_rec + 4 * (ri - 1), rr, wr);
+        }
+        double g_re = 0, g_im = 0, h_re = 0, h_im = 0, v_re = 0, v_im = 0;
+#pragma unroll 1
+        for (int t = 0; t < (finite_depth ? 4 : 1); ++t) {
+          const bool mx = (t & 1) != 0, mf = (t & 2) != 0;
+          const double zp = mx ? -Mz - 2 * e.depth : Mz;
+          const double zz = k * (zp + (mf ? -qz - 2 * e.depth : qz));
+          // z of the gradient mirrored: (x_sym, face) for K, (x, face_sym) for
+          // D, (x_sym, face_sym) always (Green_wave.f90:375-411)
+          const double zs = (mx && mf) || (mx && adjoint) || (mf && !adjoint) ? -1.0 : 1.0;
+          if (axis && fabs(k * (zp + (mf ? -cz - 2 * e.depth : cz))) < kLit1em10) {
+            // Green_wave.f90:128-158, panel on the free surface with itself:
+            // once per panel, whatever its quadrature points
+            if (q == 0) {
+              const double ka = k * f.area, s = wave_scale;
+              const double re = (1 - log(k * k * f.area / kPI)) + 2 * (kEulerGamma - kLog2);
+              G += s * ka * re;
+              Gi += s * ka * (-2 * kPI);
+              V += zs * s * k * (ka * re + 4 * sqrt(kPI * f.area));
+              Vi += zs * s * k * (ka * (-2 * kPI));
+            }
+            continue;
+          }
+          double I[4];
+          if (WAVE == kPackedTable) {
+            if (rr < P.rmax && fabs(zz) < P.zmax) {
+              const int j = packed_z_node(zz, P, [&](double x) { return nearest_z_index(x, P.nz, -P.zmax, P.grid, P.dz); });
+              packed_interpolate(wr, zz, ri, j, P, I);
+            } else {
+              packed_beyond(rr, zz, high, I);
+            }
+          } else {
+            double I5[5];
+            integrals_at<double>(rr, zz, T, I5);
+            I[0] = high ? I5[1] : I5[0];
+            I[1] = I5[2];
+            I[2] = I5[3];
+            I[3] = I5[4];
+          }
+          const double inv_r1 = rsqrt(rr * rr + zz * zz);
+          double hr = I[2], vr = I[0];
+          if (high) {
+            const double s3 = 2 * inv_r1 * inv_r1 * inv_r1;
+            hr -= rr * s3;
+            vr -= zz * s3;
+          } else if (!no_z_term) {
+            vr += 2 * inv_r1;
+          }
+          g_re += I[0];
+          g_im += I[1];
+          h_re += hr;
+          h_im += I[3];
+          v_re = fma(zs, vr, v_re);
+          v_im = fma(zs, I[1], v_im);
+        }
+        const double kw = wave_scale * k * wq, kkw = kw * k;
+        G = fma(kw, g_re, G);
+        Gi = fma(kw, g_im, Gi);
+        V = fma(kkw, v_re, V);
+        Vi = fma(kkw, v_im, Vi);
+        const double sr = kkw * unit * h_re, si = kkw * unit * h_im;
+        gx = fma(sr, wx, gx);
+        gy = fma(sr, wy, gy);
+        gxi = fma(si, wx, gxi);
+        gyi = fma(si, wy, gyi);
       }
     }
-    const double sre = kMinusOneOverFourPi * Gre, sim = kMinusOneOverFourPi * Gim;
+    if (!adjoint) {  // derivative at the source point: every horizontal one changes sign
+      gx = -gx;
+      gy = -gy;
+      gxi = -gxi;
+      gyi = -gyi;
+    }
+    if (!active) continue;
+    // ---- outputs ------------------------------------------------------------
+    const int I = I0 + r;
+    double n0 = row[3], n1 = row[4], n2 = row[5];
+    if (!adjoint && (RANK || a.early_dot_product)) {
+      const double* dn = a.dot_normals_dev + 3 * (size_t)J;
+      n0 = dn[0];
+      n1 = dn[1];
+      n2 = dn[2];
+    }
+    if constexpr (RANK) {
+      const double kdot = n0 * gx + n1 * gy + n2 * V;
+      e.rank_out[(size_t)I + (size_t)e.rank_ld * J] = make_double2(G, kdot);
+      nan_seen |= isnan(G) || isnan(kdot);
+      continue;
+    }
+    const double sre = kMinusOneOverFourPi * G, sim = kMinusOneOverFourPi * Gi;
     S[(size_t)I + (size_t)a.lds * J] = OutT<Out>::make(sre, sim);
     nan_seen |= isnan(sre) || isnan(sim);
-    const bool on_diag = a.diagonal_term && I == J && I < diag_limit;
+    // matrices.f90:348: the centre of face I (= J) of mesh2
+    double diag = 0.0;
+    if (a.diagonal_term && I == J && I < diag_limit) diag = (fabs(cz - a.free_surface) < kLit1em8) ? 1.0 : 0.5;
     const size_t kidx = (size_t)I + (size_t)a.ldk * J;
     if (a.early_dot_product) {
-      const double* dn = adjoint ? nI : (a.dot_normals_dev + 3 * J);
-      double kre = kMinusOneOverFourPi * (dn[0] * dGre[0] + dn[1] * dGre[1] + dn[2] * dGre[2]);
-      const double kim = kMinusOneOverFourPi * (dn[0] * dGim[0] + dn[1] * dGim[1] + dn[2] * dGim[2]);
-      if (on_diag) kre += diag_coef;
+      const double kre = kMinusOneOverFourPi * (n0 * gx + n1 * gy + n2 * V) + diag;
+      const double kim = kMinusOneOverFourPi * (n0 * gxi + n1 * gyi + n2 * Vi);
       K[kidx] = OutT<Out>::make(kre, kim);
       nan_seen |= isnan(kre) || isnan(kim);
     } else {
+      const double re[3] = {gx, gy, V}, im[3] = {gxi, gyi, Vi};
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        double kre = kMinusOneOverFourPi * dGre[c];
-        const double kim = kMinusOneOverFourPi * dGim[c];
-        if (on_diag) kre += diag_coef * a.dot_normals_dev[3 * I + c];
-        K[kidx + (size_t)c * a.k_plane_stride] = OutT<Out>::make(kre, kim);
+      for (int d = 0; d < 3; ++d) {
+        double kre = kMinusOneOverFourPi * re[d];
+        const double kim = kMinusOneOverFourPi * im[d];
+        if (diag != 0.0) kre += diag * a.dot_normals_dev[3 * (size_t)I + d];
+        K[kidx + (size_t)d * a.k_plane_stride] = OutT<Out>::make(kre, kim);
         nan_seen |= isnan(kre) || isnan(kim);
       }
     }
   }
   if (nan_seen && a.nan_flag_dev) atomicOr(a.nan_flag_dev, 1);
+}
+
+// Launch of assemble_entries_kernel.  Columns per CTA: 32, or as few as 4 when
+// the CTAs would not fill the GPU about four times over (a near pair then
+// waits for fewer companions, but a small mesh is bound by its longest warp).
+template <class Out, bool RANK>
+int launch_entries(const bem_assembly_args& a, EntryParams e, const TabView& T, const PackedTab& P, int wave,
+                   cudaStream_t s) {
+  const long long row_blocks = ceil_div(a.n, kRows);
+  e.cw = kEntryCols;
+  while (e.cw > 4 && row_blocks * ceil_div(a.nb_faces, e.cw) < 148 * 12) e.cw /= 2;
+  const dim3 grid((unsigned)row_blocks, ceil_div(a.nb_faces, e.cw));
+  {
+    TimedLaunch tl(kKAssemble, s);
+    if constexpr (RANK) {
+      assemble_entries_kernel<Out, kNoWave, true><<<grid, kRows, 0, s>>>(a, T, P, e);
+    } else {
+      if (wave == kNoWave) assemble_entries_kernel<Out, kNoWave, false><<<grid, kRows, 0, s>>>(a, T, P, e);
+      else if (wave == kPackedTable)
+        assemble_entries_kernel<Out, kPackedTable, false><<<grid, kRows, 0, s>>>(a, T, P, e);
+      else assemble_entries_kernel<Out, kPlainTable, false><<<grid, kRows, 0, s>>>(a, T, P, e);
+    }
+  }
+  count_launches(1);
+  BEM_CUDA_CHECK(cudaGetLastError());
+  return BEM_OK;
+}
+
+PackedTab packed_tab(const bem_assembly_args& a) {
+  PackedTab P{};
+  P.base = a.nr > 2 && a.nz > 2 ? a.packed_table_dev : nullptr;
+  P.nr = a.nr;
+  P.nz = a.nz;
+  P.grid = a.tabulation_grid_shape;
+  return P;
 }
 
 }  // namespace
@@ -1402,19 +1617,28 @@ extern "C" int bem_assemble(const bem_assembly_args* args, void* stream) {
   if (a.wavenumber == 0.0) gf_sing = kLowFreq;
   else if (std::isinf(a.wavenumber)) gf_sing = kHighFreq;
   const double sign_refl = (gf_sing == kHighFreq) ? -1.0 : 1.0;
-  dim3 grid(ceil_div(a.n, kRows), ceil_div(a.nb_faces, kTileJ));
   cudaStream_t s = (cudaStream_t)stream;
-  const bool mixed = a.precision == BEM_PREC_MIXED;
-  if (a.out_dtype == BEM_DTYPE_C128) {
-    TimedLaunch tl(kKAssemble, s);
-    if (mixed) assemble_kernel<double2, true><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
-    else assemble_kernel<double2, false><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
-  } else if (a.out_dtype == BEM_DTYPE_C64) {
-    TimedLaunch tl(kKAssemble, s);
-    if (mixed) assemble_kernel<float2, true><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
-    else assemble_kernel<float2, false><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
-  } else {
+  if (a.out_dtype != BEM_DTYPE_C128 && a.out_dtype != BEM_DTYPE_C64)
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble: unknown out_dtype");
+  if (a.precision != BEM_PREC_MIXED) {
+    if ((uintptr_t)a.packed_table_dev % 32)
+      return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble: packed_table_dev must be 32-byte aligned");
+    const PackedTab P = packed_tab(a);
+    EntryParams e{};
+    e.depth = INFINITY;
+    e.gf_sing = gf_sing;
+    e.sign_refl = sign_refl;
+    const int wave = rankine_only || !finite_k ? kNoWave : P.base ? kPackedTable : kPlainTable;
+    return a.out_dtype == BEM_DTYPE_C128 ? launch_entries<double2, false>(a, e, T, P, wave, s)
+                                         : launch_entries<float2, false>(a, e, T, P, wave, s);
+  }
+  dim3 grid(ceil_div(a.n, kRows), ceil_div(a.nb_faces, kTileJ));
+  {
+    TimedLaunch tl(kKAssemble, s);
+    if (a.out_dtype == BEM_DTYPE_C128)
+      assemble_kernel<double2><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
+    else
+      assemble_kernel<float2><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, finite_k, sign_refl);
   }
   count_launches(1);
   BEM_CUDA_CHECK(cudaGetLastError());
@@ -1456,29 +1680,17 @@ extern "C" int bem_assemble_rankine_part(const bem_assembly_args* args, void* ou
   else if (std::isinf(a.wavenumber)) gf_sing = kHighFreq;
   const double sign_refl = (gf_sing == kHighFreq) ? -1.0 : 1.0;
   const TabView T{0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, 0.0, 0.0, nullptr, nullptr, 0.0};
-  dim3 grid(ceil_div(a.n, kRows), ceil_div(a.nb_faces, kTileJ));
-  cudaStream_t s = (cudaStream_t)stream;
-  {
-    TimedLaunch tl(kKAssemble, s);
-    assemble_kernel<double2, false, true><<<grid, kRows, 0, s>>>(a, T, a.wavenumber, gf_sing, false, sign_refl,
-                                                                 (double2*)out_dev, ld);
-  }
-  count_launches(1);
-  BEM_CUDA_CHECK(cudaGetLastError());
-  return BEM_OK;
+  EntryParams e{};
+  e.depth = INFINITY;
+  e.gf_sing = gf_sing;
+  e.sign_refl = sign_refl;
+  e.rank_out = (double2*)out_dev;
+  e.rank_ld = ld;
+  return launch_entries<double2, true>(a, e, T, PackedTab{}, kNoWave, (cudaStream_t)stream);
 }
 
 namespace bem {
 namespace {
-PackedTab packed_tab(const bem_assembly_args& a) {
-  PackedTab P{};
-  P.base = a.nr > 2 && a.nz > 2 ? a.packed_table_dev : nullptr;
-  P.nr = a.nr;
-  P.nz = a.nz;
-  P.grid = a.tabulation_grid_shape;
-  return P;
-}
-
 // Shared by the single- and multi-wavenumber entry points: checks, then one
 // launch per group of up to kSymBatch wavenumbers (grid z = wavenumber).
 // planes (optional): float32 copy of K into planes[0 .. nk) (real plane, the
@@ -1713,20 +1925,20 @@ extern "C" int bem_assemble_finite_depth(const bem_assembly_args* args, double d
   const int gf_sing = a.gf_singularities;
   if (gf_sing < kHighFreq || gf_sing > kLowFreqWithRankinePart)
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: unknown gf_singularities");
-  dim3 grid(ceil_div(a.n, kRows), ceil_div(a.nb_faces, kTileJ));
-  cudaStream_t s = (cudaStream_t)stream;
-  {
-    TimedLaunch tl(kKAssemble, s);
-    if (a.out_dtype == BEM_DTYPE_C128)
-      assemble_finite_depth_kernel<double2><<<grid, kRows, 0, s>>>(a, T, depth, method == 0 ? 1 : 0, prony_dev, nexp,
-                                                                   gf_sing);
-    else
-      assemble_finite_depth_kernel<float2><<<grid, kRows, 0, s>>>(a, T, depth, method == 0 ? 1 : 0, prony_dev, nexp,
-                                                                  gf_sing);
-  }
-  count_launches(1);
-  BEM_CUDA_CHECK(cudaGetLastError());
-  return BEM_OK;
+  if ((uintptr_t)a.packed_table_dev % 32)
+    return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: packed_table_dev must be 32-byte aligned");
+  const PackedTab P = packed_tab(a);
+  EntryParams e{};
+  e.depth = depth;
+  e.images = 1;
+  e.legacy = method == 0 ? 1 : 0;
+  e.prony = prony_dev;
+  e.nexp = nexp;
+  e.gf_sing = gf_sing;
+  e.sign_refl = (gf_sing == kHighFreq) ? -1.0 : 1.0;
+  const int wave = !finite_k ? kNoWave : P.base ? kPackedTable : kPlainTable;
+  return a.out_dtype == BEM_DTYPE_C128 ? launch_entries<double2, false>(a, e, T, P, wave, (cudaStream_t)stream)
+                                       : launch_entries<float2, false>(a, e, T, P, wave, (cudaStream_t)stream);
 }
 
 namespace bem {

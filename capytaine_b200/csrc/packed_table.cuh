@@ -115,11 +115,11 @@ __device__ __forceinline__ void packed_weights(const double* rec, double x, doub
   w[1] = (1.0 - w[0]) - w[2];
 }
 
-// The four integrals of the variant at (r, z) inside the table (nodes i, j, 1-based).
-__device__ __forceinline__ void packed_interpolate(double r, double z, int i, int j, const PackedTab& P,
+// The four integrals of the variant at (r, z) inside the table (nodes i, j,
+// 1-based; wr: the weights of r at node i).
+__device__ __forceinline__ void packed_interpolate(const double wr[3], double z, int i, int j, const PackedTab& P,
                                                    double out[4]) {
-  double wr[3], wz[3];
-  packed_weights(P.r_rec + 4 * (i - 1), r, wr);
+  double wz[3];
   packed_weights(P.z_rec + 4 * (j - 1), z, wz);
   const double* q = P.quads + 4 * ((size_t)(i - 2) * P.nz + (j - 2));
   out[0] = out[1] = out[2] = out[3] = 0.0;

@@ -552,7 +552,7 @@ class Delhommeau:
         else:
             sing = self._variant(dm2.centers_z, k)
         decomposition = self.find_best_exponential_decomposition(k * float(water_depth))
-        prony = torch.as_tensor(np.ascontiguousarray(decomposition, dtype=np.float64), device=self.device)
+        prony = _lib.upload(decomposition, torch.float64, self.device)
         if stream is not None:
             stream.wait_stream(torch.cuda.current_stream())
         finite_k = 0.0 < k < np.inf
