@@ -9,14 +9,15 @@
 // Factorisation (right-looking, one step per 64-column block):
 //   1. diagonal block: LU in shared memory with partial pivoting among the rows
 //      of the block (the permutation P is block diagonal, so P A = L U holds
-//      exactly);
+//      exactly), and the inverses of its triangles;
 //   2. panels: the block row is permuted (left part included, as LAPACK's
-//      zlaswp does) and solved with L11; the block column below is solved with
-//      U11;
-//   3. trailing update A22 -= A21 A12 with double-precision tensor-core MMAs
-//      (mma.sync m8n8k4 f64), four real products per complex tile.
-// Solves: diagonal blocks are inverted once; forward and backward block
-// substitutions run as one persistent kernel each, block rows handed out in
+//      zlaswp does) and multiplied by L11^-1; the block column below is
+//      multiplied by U11^-1;
+//   3. trailing update A22 -= A21 A12; the CTA of the next diagonal block also
+//      factors it.
+// All products on double-precision tensor-core MMAs (mma.sync m16n8k8 f64),
+// four real products per complex one.
+// Solves: forward and backward block substitutions run as one persistent kernel each, block rows handed out in
 // dependency order through an atomic ticket so that every wait targets a block
 // row whose CTA is already running; waits are bounded and report a timeout.
 #include <algorithm>
@@ -27,6 +28,7 @@ namespace {
 
 constexpr int kNB = 64;
 constexpr int kLd = kNB + 1;  // shared-memory leading dimension of a 64x64 tile
+constexpr int kLdD = kNB + 2;  // of the diagonal block being factored (MMA fragments)
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -41,309 +43,640 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
 __device__ __forceinline__ double cabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
 
 // ---------------------------------------------------------------------------
-// 1. Diagonal block factorisation.
-__global__ void __launch_bounds__(256) zlu_diag_kernel(double2* __restrict__ A, int64_t lda, int64_t stride, int kk,
-                                                       int* __restrict__ piv, int64_t piv_stride,
-                                                       int* __restrict__ info) {
-  extern __shared__ double2 sm[];
-  double2* T = sm;  // T[c*kLd + r]
-  __shared__ int perm[kNB];
-  __shared__ int s_piv;
-  const int b = blockIdx.x;
-  double2* Ab = A + (size_t)b * stride;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-    const int r = idx % kNB, c = idx / kNB;
-    T[c * kLd + r] = Ab[(size_t)(kk + r) + (size_t)(kk + c) * lda];
-  }
-  if (tid < kNB) perm[tid] = tid;
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int j = 0; j < kNB; ++j) {
-    // pivot search among rows j..63 of column j (first maximum of |re|+|im|, as izamax)
-    if (warp == 0) {
-      double best = -1.0;
-      int bi = j;
-      for (int r = j + lane; r < kNB; r += 32) {
-        const double v = cabs1(T[j * kLd + r]);
-        if (v > best) {
-          best = v;
-          bi = r;
-        }
-      }
-      for (int off = 16; off > 0; off >>= 1) {
-        const double ob = __shfl_down_sync(0xffffffffu, best, off);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (lane == 0) {
-        s_piv = bi;
-        if (!(best > 0.0) && info[b] == 0) info[b] = kk + j + 1;
-      }
-    }
-    __syncthreads();
-    const int p = s_piv;
-    if (p != j) {
-      if (tid < kNB) {
-        const double2 t = T[tid * kLd + j];
-        T[tid * kLd + j] = T[tid * kLd + p];
-        T[tid * kLd + p] = t;
-      }
-      if (tid == 0) {
-        const int t = perm[j];
-        perm[j] = perm[p];
-        perm[p] = t;
-      }
-    }
-    __syncthreads();
-    const double2 pivot = T[j * kLd + j];
-    const bool ok = cabs1(pivot) > 0.0;
-    if (ok) {
-      for (int r = j + 1 + tid; r < kNB; r += blockDim.x) T[j * kLd + r] = cdiv(T[j * kLd + r], pivot);
-    }
-    __syncthreads();
-    // rank-1 update: warp w takes columns j+1+w, j+1+w+8, ...
-    for (int c = j + 1 + warp; c < kNB; c += 8) {
-      const double2 tcj = T[c * kLd + j];
-      for (int r = j + 1 + lane; r < kNB; r += 32) T[c * kLd + r] = cfms(T[c * kLd + r], T[j * kLd + r], tcj);
-    }
-    __syncthreads();
-  }
-  for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-    const int r = idx % kNB, c = idx / kNB;
-    Ab[(size_t)(kk + r) + (size_t)(kk + c) * lda] = T[c * kLd + r];
-  }
-  if (tid < kNB) piv[(size_t)b * piv_stride + kk + tid] = perm[tid];
+// Double-precision tensor-core MMA, 16 x 8 x 8 (36.5 TF/s with eight warps per
+// SM, 36.0 for 8 x 8 x 4; plain float64 multiply-adds reach 27).  Lane l holds,
+// with g = l / 4 and t = l % 4: A (g, t), (g + 8, t), (g, t + 4), (g + 8, t + 4);
+// B (t, g), (t + 4, g); C (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1).
+__device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, bool valid) {
+  const int bytes = valid ? 16 : 0;  // 0: the 16 bytes are filled with zeros, nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+               "l"(gsrc), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// ---------------------------------------------------------------------------
-// 2. Panels.  blockIdx.x enumerates: [0, nleft) left tiles of the block row
-// (permute only), [nleft, nleft+nright) right tiles (permute + L11 solve), then
-// tiles below the diagonal block (U11 solve).
-__global__ void __launch_bounds__(256) zlu_panel_kernel(double2* __restrict__ A, int64_t lda, int64_t stride, int n,
-                                                        int kk, const int* __restrict__ piv, int64_t piv_stride) {
-  extern __shared__ double2 sm[];
-  double2* D = sm;              // factored diagonal block D[c*kLd + r]
-  double2* X = sm + kNB * kLd;  // working tile X[c*kLd + r]
-  __shared__ int perm[kNB];
-  const int b = blockIdx.y;
-  double2* Ab = A + (size_t)b * stride;
-  const int tid = threadIdx.x;
-  const int nleft = kk / kNB;
-  const int nright = (n - kk - kNB) / kNB;
-  const int t = blockIdx.x;
-  int kind, c0 = 0, r0 = 0;
-  if (t < nleft) {
-    kind = 0;
-    c0 = t * kNB;
-  } else if (t < nleft + nright) {
-    kind = 1;
-    c0 = kk + kNB + (t - nleft) * kNB;
-  } else {
-    kind = 2;
-    r0 = kk + kNB + (t - nleft - nright) * kNB;
-  }
-  if (tid < kNB) perm[tid] = piv[(size_t)b * piv_stride + kk + tid];
-  if (kind != 0) {
-    for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-      const int r = idx % kNB, c = idx / kNB;
-      D[c * kLd + r] = Ab[(size_t)(kk + r) + (size_t)(kk + c) * lda];
+// Complex product of a warp: 16 rows x 8 NT columns, depth K (a multiple of
+// 8), from shared memory.  A(m, k) at A[k * lda + m], B(k, n) at B[n * ldb + k]
+// (both interleaved complex: one 16-byte load gives a fragment's real and
+// imaginary parts); no bank conflicts when lda = 2 mod 8 and ldb = 4 mod 8.
+template <int NT>
+__device__ __forceinline__ void warp_zmma(const double2* __restrict__ A, int lda, const double2* __restrict__ B,
+                                          int ldb, int K, double (&re)[NT][4], double (&im)[NT][4], int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  A += t * lda + g;
+  B += g * ldb + t;
+#pragma unroll 2
+  for (int k = 0; k < K; k += 8) {
+    const double2 a0 = A[0], a1 = A[8], a2 = A[4 * lda], a3 = A[4 * lda + 8];
+    const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+    const double na[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const double2 b0 = B[8 * j * ldb], b1 = B[8 * j * ldb + 4];
+      const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
+      dmma(re[j], ar, br);
+      dmma(im[j], ar, bi);
+      dmma(re[j], na, bi);
+      dmma(im[j], ai, br);
     }
-  }
-  __syncthreads();
-  if (kind <= 1) {
-    // rows kk..kk+63, columns c0..c0+63, permuted
-    for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-      const int r = idx % kNB, c = idx / kNB;
-      X[c * kLd + r] = Ab[(size_t)(kk + perm[r]) + (size_t)(c0 + c) * lda];
-    }
-    __syncthreads();
-    if (kind == 1) {
-      // X <- L11^{-1} X, column sweep over the unit lower factor
-      const int warp = tid >> 5, lane = tid & 31;
-      for (int i = 0; i < kNB - 1; ++i) {
-        for (int c = warp; c < kNB; c += 8) {
-          const double2 xi = X[c * kLd + i];
-          for (int r = i + 1 + lane; r < kNB; r += 32) X[c * kLd + r] = cfms(X[c * kLd + r], D[i * kLd + r], xi);
-        }
-        __syncthreads();
-      }
-    }
-    for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-      const int r = idx % kNB, c = idx / kNB;
-      Ab[(size_t)(kk + r) + (size_t)(c0 + c) * lda] = X[c * kLd + r];
-    }
-  } else {
-    // rows r0..r0+63, columns kk..kk+63: X <- X U11^{-1}
-    for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-      const int r = idx % kNB, c = idx / kNB;
-      X[c * kLd + r] = Ab[(size_t)(r0 + r) + (size_t)(kk + c) * lda];
-    }
-    __syncthreads();
-    const int rr = tid & (kNB - 1), cs = tid >> 6;  // 64 rows x 4 column phases
-    for (int j = 0; j < kNB; ++j) {
-      const double2 ujj = D[j * kLd + j];
-      if (tid < kNB && cabs1(ujj) > 0.0) X[j * kLd + tid] = cdiv(X[j * kLd + tid], ujj);
-      __syncthreads();
-      const double2 xj = X[j * kLd + rr];
-      for (int c = j + 1 + cs; c < kNB; c += 4) X[c * kLd + rr] = cfms(X[c * kLd + rr], xj, D[c * kLd + j]);
-      __syncthreads();
-    }
-    for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
-      const int r = idx % kNB, c = idx / kNB;
-      Ab[(size_t)(r0 + r) + (size_t)(kk + c) * lda] = X[c * kLd + r];
-    }
+    A += 8 * lda;
+    B += 8;
   }
 }
 
 // ---------------------------------------------------------------------------
-// 3. Complex GEMM with double-precision tensor-core MMAs:
-//    C[M x N] = beta*C + alpha * A[M x K] B[K x N]   (alpha, beta real)
-// A, B, C column-major complex128.  Tile 64x64 per CTA (4 warps of 32x32),
-// K in steps of 16.  M, N, K multiples of 64 / 16 are not required: edges are
-// guarded.
-constexpr int kBM = 64, kBN = 64, kBK = 16, kPadMN = 4;
+// 1. Diagonal block: LU with partial pivoting among the block's 64 rows, and
+// the inverses of both triangles, by one CTA of 256 threads, the block in
+// shared memory (T[c * kLdD + r]).
+// Panels of 8 columns are factored by one warp in registers, two rows per lane:
+// the pivot by one warp reduction, no row moves (a row's place is settled at
+// the panel's end), no barrier inside.  Meanwhile the other warps apply the
+// previous panel to the columns beyond, as rank-8 products on the tensor
+// cores; so are the levels of the inverses.  A barrier per step of 64 columns
+// and an exchange through shared memory took 84 us per block (and the inverses
+// a pass of 180 us over the matrix); this takes 40 us with the inverses, hidden behind the other tiles where they are many.
+constexpr int kPW = 8;      // columns of a panel
+constexpr int kTmpLd = 36;  // 4 mod 8: MMA B fragments
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
+struct DiagShared {
+  int perm[kNB];     // original row at each position
+  int place[kNB];    // new position of each row after the panel
+  int moved;         // 1: the panel exchanged rows
+  double2 pivot_row[2][kPW];  // of the step (double-buffered)
+};
+
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ double2 cinv(double2 a) {  // 1 / a
+  const double d = 1.0 / (a.x * a.x + a.y * a.y);
+  return make_double2(a.x * d, -a.y * d);
+}
+// The same without a branch, for moduli well inside the exponent range: the
+// hardware's estimate of the reciprocal and two Newton steps.
+__device__ __forceinline__ double2 cinv_fast(double2 a, bool& in_range) {
+  const double d = a.x * a.x + a.y * a.y;
+  in_range = d > 1e-280 && d < 1e280;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  return make_double2(a.x * r, -a.y * r);
+}
+__device__ __forceinline__ int nth_bit(unsigned long long m, int n) {
+  for (; n > 0; --n) m &= m - 1;
+  return __ffsll((long long)m) - 1;
 }
 
-__global__ void __launch_bounds__(128) zgemm_dmma_kernel(int M, int N, int K, double alpha, const double2* __restrict__ A,
-                                                         int64_t lda, int64_t strideA, const double2* __restrict__ B,
-                                                         int64_t ldb, int64_t strideB, double beta,
-                                                         double2* __restrict__ C, int64_t ldc, int64_t strideC) {
-  __shared__ double As[2][kBK][kBM + kPadMN];  // [re/im][k][m]
-  __shared__ double Bs[2][kBK][kBN + kPadMN];  // [re/im][k][n]
-  const int bz = blockIdx.z;
-  A += (size_t)bz * strideA;
-  B += (size_t)bz * strideB;
-  C += (size_t)bz * strideC;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
+// Columns j0 .. j0 + 7 by one warp; kcol: the block's first column in the matrix.
+__device__ __forceinline__ void factor_panel(double2* T, int j0, int lane, DiagShared& sh, int* info, int kcol) {
+  double2 x[2][kPW];
+  int pos[2] = {-1, -1};  // position of a row chosen as pivot
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int s = 0; s < kPW; ++s) x[h][s] = T[(j0 + s) * kLdD + lane + 32 * h];
+  // The largest |re| + |im| of a column among the rows left: the high word of
+  // the value with its last six bits replaced by the row, so that one reduction
+  // finds both (values within 2^-14 of the largest count as equal and the first
+  // row wins: multipliers up to 1 + 2^-14); a NaN is never chosen.
+  auto pivot_key = [&](int s) {
+    unsigned key = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = lane + 32 * h;
+      const double c = cabs1(x[h][s]);
+      if (r >= j0 && pos[h] < 0 && c == c)
+        key = max(key, (((unsigned)__double2hiint(c) + 64u) & ~63u) | (unsigned)(63 - r));
+    }
+    return key;
+  };
+  unsigned key = __reduce_max_sync(0xffffffffu, pivot_key(0));
+#pragma unroll
+  for (int s = 0; s < kPW; ++s) {
+    unsigned row = 63u - (key & 63u);
+    if (key == 0) {  // only NaN left: the first row left
+      const unsigned mine = (lane >= j0 && pos[0] < 0) ? lane : (lane + 32 >= j0 && pos[1] < 0) ? lane + 32 : 64u;
+      row = __reduce_min_sync(0xffffffffu, mine);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (lane + 32 * h == (int)row) {
+        pos[h] = j0 + s;
+#pragma unroll
+        for (int c = s; c < kPW; ++c) sh.pivot_row[s & 1][c] = x[h][c];
+      }
+    __syncwarp();
+    double2 p[kPW];
+#pragma unroll
+    for (int c = s; c < kPW; ++c) p[c] = sh.pivot_row[s & 1][c];
+    bool in_range;
+    double2 inv = cinv_fast(p[s], in_range);
+    if (!in_range) {
+      const bool ok = cabs1(p[s]) > 0.0;
+      if (!ok && lane == 0 && *info == 0) *info = kcol + j0 + s + 1;
+      inv = ok ? cinv(p[s]) : make_double2(1.0, 0.0);
+    }
+    double2 l[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (lane + 32 * h >= j0 && pos[h] < 0) {
+        x[h][s] = cmul(x[h][s], inv);
+        l[h] = x[h][s];
+      } else {
+        l[h] = make_double2(0.0, 0.0);  // rows done keep their values
+      }
+    }
+    // the next pivot's column first: its reduction runs beside the others' updates
+    if (s + 1 < kPW) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) x[h][s + 1] = cfms(x[h][s + 1], l[h], p[s + 1]);
+      key = __reduce_max_sync(0xffffffffu, pivot_key(s + 1));
+#pragma unroll
+      for (int c = s + 2; c < kPW; ++c)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) x[h][c] = cfms(x[h][c], l[h], p[c]);
+    }
+  }
+  // positions: pivots in order; a row that gave its place up takes the place
+  // of a pivot that came from further down
+  const unsigned long long sel = (unsigned long long)__ballot_sync(0xffffffffu, pos[0] >= 0) |
+                                 (unsigned long long)__ballot_sync(0xffffffffu, pos[1] >= 0) << 32;
+  const unsigned long long in_panel = ((1ull << kPW) - 1) << j0;
+  const unsigned long long vacated = sel & ~in_panel, displaced = in_panel & ~sel;
+  int old[2], to[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = lane + 32 * h;
+    old[h] = sh.perm[r];
+    to[h] = r;
+    if (pos[h] >= 0) to[h] = pos[h];
+    else if (displaced >> r & 1) to[h] = nth_bit(vacated, __popcll(displaced & ((1ull << r) - 1)));
+    sh.place[r] = to[h];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    sh.perm[to[h]] = old[h];
+#pragma unroll
+    for (int s = 0; s < kPW; ++s) T[(j0 + s) * kLdD + to[h]] = x[h][s];
+  }
+  const bool moved = __any_sync(0xffffffffu, to[0] != lane || to[1] != lane + 32);
+  if (lane == 0) sh.moved = moved;
+}
+
+// 16 x 16 inverse of one triangle of the block at (base, base), by one warp,
+// in place.  Lane c < 16 holds column c.
+__device__ __forceinline__ void invert_lower16(double2* T, int base, int lane) {
+  const int c = lane & 15;
+  double2 x[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) x[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+#pragma unroll
+  for (int i = 0; i < 15; ++i)
+#pragma unroll
+    for (int r = i + 1; r < 16; ++r) x[r] = cfms(x[r], T[(base + i) * kLdD + base + r], x[i]);
+  __syncwarp();
+  if (lane < 16) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (r > c) T[(base + c) * kLdD + base + r] = x[r];
+  }
+}
+__device__ __forceinline__ void invert_upper16(double2* T, int base, int lane) {
+  const int c = lane & 15;
+  const double2 d = T[(base + c) * kLdD + base + c];
+  const double2 mine = cabs1(d) > 0.0 ? cinv(d) : make_double2(0.0, 0.0);
+  double2 x[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) x[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+#pragma unroll
+  for (int i = 15; i >= 0; --i) {
+    x[i] = cmul(x[i], shfl2(mine, i));
+#pragma unroll
+    for (int r = 0; r < i; ++r) x[r] = cfms(x[r], T[(base + i) * kLdD + base + r], x[i]);
+  }
+  __syncwarp();
+  if (lane < 16) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (r <= c) T[(base + c) * kLdD + base + r] = x[r];
+  }
+}
+
+// T(16 rows from m0, 8 columns from n0) -= panel (8 columns from j0) times the
+// rows j0 .. j0 + 7 of those columns, rows from first_row on only (a multiple of 8).
+__device__ __forceinline__ void panel_update_tile(double2* T, int j0, int m0, int n0, int first_row, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  double re[4], im[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const double2 c = T[(n0 + 2 * t + (e & 1)) * kLdD + m0 + g + 8 * (e >> 1)];
+    re[e] = c.x;
+    im[e] = c.y;
+  }
+  double ai[4], nr[4], ni[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const double2 v = T[(j0 + t + 4 * (e >> 1)) * kLdD + m0 + g + 8 * (e & 1)];
+    ai[e] = v.y;
+    nr[e] = -v.x;
+    ni[e] = -v.y;
+  }
+  const double2 b0 = T[(n0 + g) * kLdD + j0 + t], b1 = T[(n0 + g) * kLdD + j0 + t + 4];
+  const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
+  dmma(re, nr, br);
+  dmma(im, nr, bi);
+  dmma(re, ai, bi);
+  dmma(im, ni, br);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int r = m0 + g + 8 * (e >> 1);
+    if (r >= first_row) T[(n0 + 2 * t + (e & 1)) * kLdD + r] = make_double2(re[e], im[e]);
+  }
+}
+
+// The off-diagonal H x H blocks of the triangles' inverses from those of the
+// diagonal ones (H = 16, then 32): with [A 0; C B] below the diagonal,
+// -B^-1 (C A^-1); with [A C; 0 B] above it, -A^-1 (C B^-1).  In place in T, the
+// inner product through tmp; 16 x 8 tiles of the products over the 8 warps,
+// the zero blocks of the triangles skipped.
+template <int H>
+__device__ __forceinline__ void invert_level(double2* T, double2* tmp, int warp, int lane) {
+  constexpr int kCombos = 64 / H;                     // (triangle, pair of blocks)
+  constexpr int kTilesM = H / 16, kTilesN = H / 8;
+  constexpr int kTiles = kCombos * kTilesM * kTilesN;
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int stage = 0; stage < 2; ++stage) {
+#pragma unroll 1
+    for (int tile = warp; tile < kTiles; tile += 8) {
+      const int combo = tile / (kTilesM * kTilesN), in = tile % (kTilesM * kTilesN);
+      const bool lower = combo & 1;
+      const int base = (combo >> 1) * 2 * H, m0 = 16 * (in % kTilesM), n0 = 8 * (in / kTilesM);
+      double2* W = tmp + combo * H * kTmpLd;
+      const int rowC = lower ? base + H : base, colC = lower ? base : base + H;
+      double re[4] = {}, im[4] = {};
+#pragma unroll 1
+      for (int k0 = 0; k0 < H; k0 += 8) {
+        // stage 0: W = C (inverse at C's columns): its rows k against columns n0 ..
+        // stage 1: (inverse at C's rows) W: its columns k against rows m0 ..
+        if (stage == 0 ? (lower ? k0 < n0 : k0 > n0) : (lower ? k0 > m0 + 8 : k0 < m0)) continue;
+        double ar[4], ai[4], na[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int k = k0 + t + 4 * (e >> 1), m = m0 + g + 8 * (e & 1);
+          double2 v;
+          if (stage == 0) {
+            v = T[(colC + k) * kLdD + rowC + m];
+          } else {
+            v = T[(rowC + k) * kLdD + rowC + m];
+            if (lower ? k > m : k < m) v = make_double2(0.0, 0.0);
+            if (lower && k == m) v = make_double2(1.0, 0.0);
+            v.x = -v.x;
+            v.y = -v.y;
+          }
+          ar[e] = v.x;
+          ai[e] = v.y;
+          na[e] = -v.y;
+        }
+        double br[2], bi[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int k = k0 + t + 4 * e, n = n0 + g;
+          double2 v;
+          if (stage == 0) {
+            v = T[(colC + n) * kLdD + colC + k];
+            if (lower ? k < n : k > n) v = make_double2(0.0, 0.0);
+            if (lower && k == n) v = make_double2(1.0, 0.0);
+          } else {
+            v = W[n * kTmpLd + k];
+          }
+          br[e] = v.x;
+          bi[e] = v.y;
+        }
+        dmma(re, ar, br);
+        dmma(im, ar, bi);
+        dmma(re, na, bi);
+        dmma(im, ai, br);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = m0 + g + 8 * (e >> 1), n = n0 + 2 * t + (e & 1);
+        const double2 v = make_double2(re[e], im[e]);
+        if (stage == 0) W[n * kTmpLd + m] = v;
+        else T[(colC + n) * kLdD + rowC + m] = v;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The whole diagonal block at row and column kk of a matrix, already in T:
+// factors to the matrix, inverses to inv (L then U, 64 x 64 column-major).
+__device__ void factor_diagonal(double2* T, double2* tmp, DiagShared& sh, double2* __restrict__ Ab, int64_t lda,
+                                int kk, int* __restrict__ piv, int* __restrict__ info, double2* __restrict__ inv) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  double acc_re[4][4][2], acc_im[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      acc_re[i][j][0] = acc_re[i][j][1] = 0.0;
-      acc_im[i][j][0] = acc_im[i][j][1] = 0.0;
-    }
-  const int qr = lane >> 2, qc = lane & 3;
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-    // A tile: 64 (m) x 16 (k); thread loads m = tid % 64, k = tid / 64 + 2 i
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int m = tid & 63, k = (tid >> 6) + 2 * i;
-      double2 v = make_double2(0.0, 0.0);
-      if (m0 + m < M && k0 + k < K) v = A[(size_t)(m0 + m) + (size_t)(k0 + k) * lda];
-      As[0][k][m] = v.x;
-      As[1][k][m] = v.y;
-    }
-    // B tile: 16 (k) x 64 (n); thread loads k = tid % 16, n = tid / 16 + 8 i
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int k = tid & 15, nn = (tid >> 4) + 8 * i;
-      double2 v = make_double2(0.0, 0.0);
-      if (n0 + nn < N && k0 + k < K) v = B[(size_t)(k0 + k) + (size_t)(n0 + nn) * ldb];
-      Bs[0][k][nn] = v.x;
-      Bs[1][k][nn] = v.y;
+  if (tid < kNB) sh.perm[tid] = tid;
+  __syncthreads();
+#pragma unroll 1
+  for (int j0 = 0; j0 < kNB; j0 += kPW) {
+    const int j1 = j0 + kPW;
+    if (warp == 0) {
+      factor_panel(T, j0, lane, sh, info, kk);
+    } else if (j0 > 0) {
+      // columns beyond this panel: the previous panel's update
+      const int tiles_m = (kNB - (j0 & ~15)) / 16, tiles = tiles_m * ((kNB - j1) / 8);
+      for (int i = warp - 1; i < tiles; i += 7)
+        panel_update_tile(T, j0 - kPW, (j0 & ~15) + 16 * (i % tiles_m), j1 + 8 * (i / tiles_m), j0, lane);
     }
     __syncthreads();
+    if (sh.moved) {
+      for (int c = warp; c < kNB; c += 8) {
+        if (c >= j0 && c < j1) continue;
+        const double2 v0 = T[c * kLdD + lane], v1 = T[c * kLdD + lane + 32];
+        __syncwarp();
+        T[c * kLdD + sh.place[lane]] = v0;
+        T[c * kLdD + sh.place[lane + 32]] = v1;
+      }
+      __syncthreads();
+    }
+    if (tid < kNB && tid >= j1) {  // rows of U: L11^-1 applied to column tid
+      double2 x[kPW];
 #pragma unroll
-    for (int kq = 0; kq < kBK; kq += 4) {
-      double ar[4], ai[4], nai[4], br[4], bi[4];
+      for (int i = 0; i < kPW; ++i) x[i] = T[tid * kLdD + j0 + i];
+#pragma unroll
+      for (int i = 0; i < kPW - 1; ++i)
+#pragma unroll
+        for (int r = i + 1; r < kPW; ++r) x[r] = cfms(x[r], T[(j0 + i) * kLdD + j0 + r], x[i]);
+#pragma unroll
+      for (int i = 1; i < kPW; ++i) T[tid * kLdD + j0 + i] = x[i];
+    }
+    __syncthreads();
+    // the next panel's columns
+    if (j1 < kNB) {
+      const int m0 = (j1 & ~15) + 16 * warp;
+      if (m0 < kNB) panel_update_tile(T, j0, m0, j1, j1, lane);
+    }
+    __syncthreads();
+  }
+  for (int idx = tid; idx < kNB * kNB; idx += 256) {
+    const int r = idx % kNB, c = idx / kNB;
+    Ab[(size_t)(kk + r) + (size_t)(kk + c) * lda] = T[c * kLdD + r];
+  }
+  if (tid < kNB) piv[kk + tid] = sh.perm[tid];
+  __syncthreads();
+  if (warp < 4) invert_lower16(T, 16 * warp, lane);
+  else invert_upper16(T, 16 * (warp - 4), lane);
+  __syncthreads();
+  invert_level<16>(T, tmp, warp, lane);
+  invert_level<32>(T, tmp, warp, lane);
+  for (int idx = tid; idx < kNB * kNB; idx += 256) {
+    const int r = idx % kNB, c = idx / kNB;
+    const double2 v = T[c * kLdD + r], zero = make_double2(0.0, 0.0);
+    inv[idx] = r > c ? v : make_double2(r == c ? 1.0 : 0.0, 0.0);
+    inv[kNB * kNB + idx] = r <= c ? v : zero;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 2. Panels as products with the triangles' inverses.  blockIdx.x enumerates:
+// [0, nleft) the block row's 64-column tiles left of the diagonal (permuted
+// only, as LAPACK's zlaswp), then 32-column tiles right of it (permuted, times
+// L11^-1 from the left), then 32-row tiles below it (times U11^-1 from the
+// right).  In place: a CTA reads all that it overwrites first.
+constexpr int kPanelTile = 32;
+constexpr int kPanelLdB = kNB + 4;
+constexpr int kPanelSmem = kNB * (kPanelTile + 2 + kPanelLdB) * (int)sizeof(double2);  // the tiles below need more
+static_assert(kPanelSmem >= (kNB * (kNB + 2) + kPanelTile * kPanelLdB) * (int)sizeof(double2), "tiles to the right");
+static_assert(kPanelSmem >= kNB * kLd * (int)sizeof(double2), "tiles to the left");
+
+template <bool RIGHT>
+__device__ __forceinline__ void panel_tile(double2* sm, double2* __restrict__ Ab, int64_t lda, int kk, int at,
+                                           const double2* __restrict__ inv, const int* perm) {
+  // RIGHT: (64 x 32) = L11^-1 (64 x 64) X (64 x 32); else (32 x 64) = X (32 x 64) U11^-1 (64 x 64)
+  constexpr int kM = RIGHT ? kNB : kPanelTile, kN = RIGHT ? kPanelTile : kNB;
+  constexpr int kLdA = kM + 2;
+  double2* As = sm;
+  double2* Bs = sm + kNB * kLdA;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double2* X = RIGHT ? Ab + kk + (size_t)at * lda : Ab + at + (size_t)kk * lda;
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {  // depth 16 per copy group
+    for (int idx = tid; idx < 16 * kM; idx += 256) {
+      const int m = idx % kM, k = 16 * q + idx / kM;
+      cp_async16(As + k * kLdA + m, RIGHT ? inv + (size_t)k * kNB + m : X + (size_t)m + (size_t)k * lda, true);
+    }
+    for (int idx = tid; idx < 16 * kN; idx += 256) {
+      const int k = 16 * q + (idx & 15), n = idx >> 4;
+      cp_async16(Bs + n * kPanelLdB + k,
+                 RIGHT ? X + (size_t)perm[k] + (size_t)n * lda : inv + (size_t)n * kNB + k, true);
+    }
+    cp_async_commit();
+  }
+  // eight warps of 16 x 16
+  const int wm = RIGHT ? 16 * (warp & 3) : 16 * (warp & 1), wn = RIGHT ? 16 * (warp >> 2) : 16 * (warp >> 1);
+  double re[2][4] = {}, im[2][4] = {};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q == 0) cp_async_wait<3>();
+    if (q == 1) cp_async_wait<2>();
+    if (q == 2) cp_async_wait<1>();
+    if (q == 3) cp_async_wait<0>();
+    __syncthreads();
+    warp_zmma<2>(As + 16 * q * kLdA + wm, kLdA, Bs + wn * kPanelLdB + 16 * q, kPanelLdB, 16, re, im, lane);
+  }
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      X[(size_t)(wm + g + 8 * (e >> 1)) + (size_t)(wn + 8 * j + 2 * t + (e & 1)) * lda] =
+          make_double2(re[j][e], im[j][e]);
+}
+
+__global__ void __launch_bounds__(256, 2) zlu_panel_kernel(double2* __restrict__ A, int64_t lda, int64_t stride,
+                                                           int n, int kk, const int* __restrict__ piv,
+                                                           int64_t piv_stride, const double2* __restrict__ inv,
+                                                           int nblk) {
+  extern __shared__ double2 sm[];
+  __shared__ int perm[kNB];
+  const int b = blockIdx.y, tid = threadIdx.x;
+  double2* Ab = A + (size_t)b * stride;
+  const int nleft = kk / kNB, nrest = (n - kk - kNB) / kPanelTile;
+  const int t = blockIdx.x;
+  const double2* ib = inv + ((size_t)b * nblk + kk / kNB) * 2 * kNB * kNB;
+  int own = 0;
+  if (tid < kNB) {
+    own = piv[(size_t)b * piv_stride + kk + tid];
+    perm[tid] = own;
+  }
+  if (t < nleft) {
+    if (!__syncthreads_or(tid < kNB && own != tid)) return;  // no row moves
+    const int c0 = t * kNB;
+    for (int idx = tid; idx < kNB * kNB; idx += 256) {
+      const int r = idx % kNB, c = idx / kNB;
+      sm[c * kLd + r] = Ab[(size_t)(kk + perm[r]) + (size_t)(c0 + c) * lda];
+    }
+    __syncthreads();
+    for (int idx = tid; idx < kNB * kNB; idx += 256) {
+      const int r = idx % kNB, c = idx / kNB;
+      Ab[(size_t)(kk + r) + (size_t)(c0 + c) * lda] = sm[c * kLd + r];
+    }
+    return;
+  }
+  __syncthreads();
+  const int u = t - nleft;
+  if (u < nrest) panel_tile<true>(sm, Ab, lda, kk, kk + kNB + u * kPanelTile, ib, perm);
+  else panel_tile<false>(sm, Ab, lda, kk, kk + kNB + (u - nrest) * kPanelTile, ib + kNB * kNB, perm);
+}
+
+// ---------------------------------------------------------------------------
+// 3. C = beta C + alpha A B (alpha, beta real), column-major complex128, 64 x 64
+// tiles by CTAs of 8 warps (16 x 32 each), depth 16 per stage of a three-stage
+// cp.async ring, two CTAs per SM.  Edges of any size are filled with zeros and
+// not stored.
+// FACTOR (trailing update of the LU): the CTA of the tile that is the next
+// diagonal block keeps its result in shared memory and factors it, beside the
+// other CTAs' tiles: the chain of diagonal blocks is hidden behind the updates
+// where these are long, and costs no launch.  Those CTAs come first in the
+// grid.
+constexpr int kTile = 64, kDepth = 16, kStages = 3;
+constexpr int kLdTA = kTile + 2, kLdTB = kDepth + 4;
+constexpr int kStageElems = kDepth * kLdTA + kTile * kLdTB;
+constexpr int kGemmSmem = kStages * kStageElems * (int)sizeof(double2);
+static_assert((kNB * kLdD + 2 * 32 * kTmpLd) * (int)sizeof(double2) <= kGemmSmem, "the diagonal block fits");
+
+template <bool FACTOR>
+__global__ void __launch_bounds__(256, 2)
+    zgemm_dmma_kernel(int M, int N, int K, double alpha, const double2* A, int64_t lda, int64_t strideA,
+                      const double2* B, int64_t ldb, int64_t strideB, double beta, double2* C, int64_t ldc,
+                      int64_t strideC, int tiles_m, int tiles, int batch, int kk, int* __restrict__ piv,
+                      int64_t piv_stride, int* __restrict__ info, double2* __restrict__ inv, int nblk) {
+  extern __shared__ double2 sm[];
+  __shared__ DiagShared sh;
+  int t, b;
+  if ((int)blockIdx.x < batch) {  // tile 0 of every matrix
+    t = 0;
+    b = blockIdx.x;
+  } else {
+    const int rest = blockIdx.x - batch;
+    t = 1 + rest % (tiles - 1);
+    b = rest / (tiles - 1);
+  }
+  A += (size_t)b * strideA;
+  B += (size_t)b * strideB;
+  C += (size_t)b * strideC;
+  const int m0 = (t % tiles_m) * kTile, n0 = (t / tiles_m) * kTile;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nk = (K + kDepth - 1) / kDepth;
+  auto issue = [&](int q) {
+    if (q < nk) {
+      double2* As = sm + (q % kStages) * kStageElems;
+      double2* Bs = As + kDepth * kLdTA;
+      const int k0 = q * kDepth;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        ar[i] = As[0][kq + qc][wm + 8 * i + qr];
-        ai[i] = As[1][kq + qc][wm + 8 * i + qr];
-        nai[i] = -ai[i];
-        br[i] = Bs[0][kq + qc][wn + 8 * i + qr];
-        bi[i] = Bs[1][kq + qc][wn + 8 * i + qr];
+        const int idx = tid + 256 * i;
+        const int m = idx & 63, k = idx >> 6;
+        const bool ok = m0 + m < M && k0 + k < K;
+        cp_async16(As + k * kLdTA + m, ok ? A + (size_t)(m0 + m) + (size_t)(k0 + k) * lda : A, ok);
+        const int kb = idx & 15, n = idx >> 4;
+        const bool okb = n0 + n < N && k0 + kb < K;
+        cp_async16(Bs + n * kLdTB + kb, okb ? B + (size_t)(k0 + kb) + (size_t)(n0 + n) * ldb : B, okb);
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dmma(acc_re[i][j][0], acc_re[i][j][1], ar[i], br[j]);
-          dmma(acc_re[i][j][0], acc_re[i][j][1], nai[i], bi[j]);
-          dmma(acc_im[i][j][0], acc_im[i][j][1], ar[i], bi[j]);
-          dmma(acc_im[i][j][0], acc_im[i][j][1], ai[i], br[j]);
-        }
     }
-    __syncthreads();
-  }
-  // epilogue: fragment (row qr, columns 2 qc, 2 qc + 1) of each 8x8 sub-tile
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
+    cp_async_commit();
+  };
+  const int wm = 16 * (warp & 3), wn = 32 * (warp >> 2);
+  const int g = lane >> 2, tt = lane & 3;
+  double re[4][4] = {}, im[4][4] = {};
+  issue(0);
+  issue(1);
+  if (FACTOR) {
+    // C - A B as -(-C + A B): the accumulators start from the tile, so that
+    // its loads overlap the operands' (read one by one in the epilogue, behind
+    // stores that might alias, they took longer than the products)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int m = m0 + wm + 8 * i + qr;
-        const int nn = n0 + wn + 8 * j + 2 * qc + h;
-        if (m < M && nn < N) {
-          double2* p = C + (size_t)m + (size_t)nn * ldc;
-          double2 c = (beta == 0.0) ? make_double2(0.0, 0.0) : *p;
-          c.x = beta * c.x + alpha * acc_re[i][j][h];
-          c.y = beta * c.y + alpha * acc_im[i][j][h];
-          *p = c;
-        }
+      for (int e = 0; e < 4; ++e) {
+        const double2 c = C[(size_t)(m0 + wm + g + 8 * (e >> 1)) + (size_t)(n0 + wn + 8 * j + 2 * tt + (e & 1)) * ldc];
+        re[j][e] = -c.x;
+        im[j][e] = -c.y;
       }
+  }
+#pragma unroll 1
+  for (int q = 0; q < nk; ++q) {
+    cp_async_wait<1>();  // chunk q has landed (this thread's part)
+    __syncthreads();     // everybody's part; and everybody is done with chunk q - 1
+    issue(q + 2);
+    const double2* As = sm + (q % kStages) * kStageElems;
+    warp_zmma<4>(As + wm, kLdTA, As + kDepth * kLdTA + wn * kLdTB, kLdTB, kDepth, re, im, lane);
+  }
+  if constexpr (FACTOR) {
+    const bool diagonal = t == 0;
+    if (diagonal) {
+      cp_async_wait<0>();
+      __syncthreads();  // the ring becomes the block
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = wm + g + 8 * (e >> 1), n = wn + 8 * j + 2 * tt + (e & 1);
+        const double2 c = make_double2(-re[j][e], -im[j][e]);
+        if (diagonal) sm[n * kLdD + m] = c;
+        else C[(size_t)(m0 + m) + (size_t)(n0 + n) * ldc] = c;
+      }
+    if (!diagonal) return;
+    __syncthreads();
+    factor_diagonal(sm, sm + kNB * kLdD, sh, C - kk - (int64_t)kk * ldc, ldc, kk, piv + (size_t)b * piv_stride,
+                    info + b, inv + ((size_t)b * nblk + kk / kNB) * 2 * kNB * kNB);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int m = m0 + wm + g + 8 * (e >> 1), n = n0 + wn + 8 * j + 2 * tt + (e & 1);
+      if (m < M && n < N) {
+        double2* p = C + (size_t)m + (size_t)n * ldc;
+        double2 c = beta == 0.0 ? make_double2(0.0, 0.0) : *p;
+        c.x = beta * c.x + alpha * re[j][e];
+        c.y = beta * c.y + alpha * im[j][e];
+        *p = c;
+      }
+    }
 }
 
-// ---------------------------------------------------------------------------
-// Inverses of the diagonal blocks: L_ii^{-1} (unit lower) and U_ii^{-1}.
-// Output layout: inv[(b * nblk + i) * 2 + {0: L, 1: U}] is a 64x64 column-major tile.
-__global__ void __launch_bounds__(128) ztri_inv_kernel(const double2* __restrict__ A, int64_t lda, int64_t stride,
-                                                       int nblk, double2* __restrict__ inv) {
+// The first diagonal block of every matrix.
+__global__ void __launch_bounds__(256, 2) zlu_first_kernel(double2* __restrict__ A, int64_t lda, int64_t stride,
+                                                           int* __restrict__ piv, int64_t piv_stride,
+                                                           int* __restrict__ info, double2* __restrict__ inv,
+                                                           int nblk) {
   extern __shared__ double2 sm[];
-  double2* D = sm;              // factored block
-  double2* W = sm + kNB * kLd;  // inverse being built, W[c*kLd + r]
-  const int i = blockIdx.x, b = blockIdx.y;
-  const double2* Ab = A + (size_t)b * stride;
-  const int kk = i * kNB;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) {
+  __shared__ DiagShared sh;
+  const int b = blockIdx.x;
+  double2* Ab = A + (size_t)b * stride;
+  for (int idx = threadIdx.x; idx < kNB * kNB; idx += 256) {
     const int r = idx % kNB, c = idx / kNB;
-    D[c * kLd + r] = Ab[(size_t)(kk + r) + (size_t)(kk + c) * lda];
+    sm[c * kLdD + r] = Ab[(size_t)r + (size_t)c * lda];
   }
   __syncthreads();
-  double2* out = inv + ((size_t)b * nblk + i) * 2 * kNB * kNB;
-  // L^{-1}: thread c solves L x = e_c (forward substitution), column c of the inverse.
-  if (tid < kNB) {
-    const int c = tid;
-    for (int r = 0; r < kNB; ++r) {
-      double2 v = make_double2(r == c ? 1.0 : 0.0, 0.0);
-      for (int m = c; m < r; ++m) v = cfms(v, D[m * kLd + r], W[c * kLd + m]);
-      W[c * kLd + r] = (r < c) ? make_double2(0.0, 0.0) : v;
-    }
-  }
-  __syncthreads();
-  for (int idx = tid; idx < kNB * kNB; idx += blockDim.x) out[idx] = W[(idx / kNB) * kLd + idx % kNB];
-  __syncthreads();
-  // U^{-1}: thread c solves U x = e_c (backward substitution).
-  if (tid < kNB) {
-    const int c = tid;
-    for (int r = kNB - 1; r >= 0; --r) {
-      double2 v = make_double2(r == c ? 1.0 : 0.0, 0.0);
-      if (r > c) {
-        W[c * kLd + r] = make_double2(0.0, 0.0);
-        continue;
-      }
-      for (int m = r + 1; m <= c; ++m) v = cfms(v, D[m * kLd + r], W[c * kLd + m]);
-      const double2 d = D[r * kLd + r];
-      W[c * kLd + r] = (cabs1(d) > 0.0) ? cdiv(v, d) : make_double2(0.0, 0.0);
-    }
-  }
-  __syncthreads();
-  for (int idx = tid; idx < kNB * kNB; idx += blockDim.x)
-    out[kNB * kNB + idx] = W[(idx / kNB) * kLd + idx % kNB];
+  factor_diagonal(sm, sm + kNB * kLdD, sh, Ab, lda, 0, piv + (size_t)b * piv_stride, info + b,
+                  inv + (size_t)b * nblk * 2 * kNB * kNB);
 }
 
 // ---------------------------------------------------------------------------
@@ -495,10 +828,12 @@ int check_lu_args(const void* A, int n, int64_t lda, int batch) {
 bool g_smem_configured = false;
 int configure_smem() {
   if (g_smem_configured) return BEM_OK;
-  const int big = 2 * kNB * kLd * (int)sizeof(double2);
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(zlu_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(zlu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(ztri_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(zlu_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  BEM_CUDA_CHECK(
+      cudaFuncSetAttribute(zgemm_dmma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  BEM_CUDA_CHECK(
+      cudaFuncSetAttribute(zgemm_dmma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(zlu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem));
   const int trsm = (2 * kNB * kLd + 2 * kNB * kLdR) * (int)sizeof(double2);
   BEM_CUDA_CHECK(cudaFuncSetAttribute(ztrsm_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, trsm));
   g_smem_configured = true;
@@ -523,10 +858,12 @@ extern "C" int bem_zgemm(int M, int N, int K, double alpha, const void* A_dev, i
   if (M < 0 || N < 0 || K < 0 || batch <= 0) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_zgemm: bad sizes");
   if (M == 0 || N == 0) return BEM_OK;
   if (!A_dev || !B_dev || !C_dev) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_zgemm: null pointer");
-  dim3 grid(ceil_div(M, kBM), ceil_div(N, kBN), batch);
-  zgemm_dmma_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(M, N, K, alpha, (const double2*)A_dev, lda, strideA,
-                                                            (const double2*)B_dev, ldb, strideB, beta,
-                                                            (double2*)C_dev, ldc, strideC);
+  int st = configure_smem();
+  if (st) return st;
+  const int tiles_m = ceil_div(M, kTile), tiles = tiles_m * ceil_div(N, kTile);
+  zgemm_dmma_kernel<false><<<tiles * batch, 256, kGemmSmem, (cudaStream_t)stream>>>(
+      M, N, K, alpha, (const double2*)A_dev, lda, strideA, (const double2*)B_dev, ldb, strideB, beta,
+      (double2*)C_dev, ldc, strideC, tiles_m, tiles, batch, 0, nullptr, 0, nullptr, nullptr, 0);
   count_launches(1);
   BEM_CUDA_CHECK(cudaGetLastError());
   return BEM_OK;
@@ -547,35 +884,32 @@ extern "C" int bem_zlu_factor(void* A_dev, int n, int64_t lda, int64_t stride, i
   if ((st = configure_smem())) return st;
   cudaStream_t s = (cudaStream_t)stream;
   double2* A = (double2*)A_dev;
-  const int smem = 2 * kNB * kLd * (int)sizeof(double2);
+  double2* inv = (double2*)work_dev;
+  const int nblk = n / kNB;
   BEM_CUDA_CHECK(cudaMemsetAsync(info_dev, 0, sizeof(int) * batch, s));
+  {
+    TimedLaunch tl(kKZluDiag, s);
+    zlu_first_kernel<<<batch, 256, kGemmSmem, s>>>(A, lda, stride, piv_dev, n, info_dev, inv, nblk);
+  }
+  count_launches(1);
   for (int kk = 0; kk < n; kk += kNB) {
-    {
-      TimedLaunch tl(kKZluDiag, s);
-      zlu_diag_kernel<<<batch, 256, kNB * kLd * sizeof(double2), s>>>(A, lda, stride, kk, piv_dev, n, info_dev);
-    }
-    count_launches(1);
-    const int nleft = kk / kNB, nrest = (n - kk - kNB) / kNB;
-    const int ntiles = nleft + 2 * nrest;
+    const int m = n - kk - kNB;
+    const int ntiles = kk / kNB + 2 * (m / kPanelTile);
     if (ntiles > 0) {
       TimedLaunch tl(kKZluPanel, s);
-      zlu_panel_kernel<<<dim3(ntiles, batch), 256, smem, s>>>(A, lda, stride, n, kk, piv_dev, n);
+      zlu_panel_kernel<<<dim3(ntiles, batch), 256, kPanelSmem, s>>>(A, lda, stride, n, kk, piv_dev, n, inv, nblk);
       count_launches(1);
     }
-    if (nrest > 0) {
-      const int m = n - kk - kNB;
-      dim3 grid(ceil_div(m, kBM), ceil_div(m, kBN), batch);
+    if (m > 0) {
+      const int tiles_m = m / kTile, tiles = tiles_m * tiles_m, next = kk + kNB;
       TimedLaunch tl(kKZgemmDmma, s);
-      zgemm_dmma_kernel<<<grid, 128, 0, s>>>(m, m, kNB, -1.0, A + (size_t)(kk + kNB) + (size_t)kk * lda, lda, stride,
-                                             A + (size_t)kk + (size_t)(kk + kNB) * lda, lda, stride, 1.0,
-                                             A + (size_t)(kk + kNB) + (size_t)(kk + kNB) * lda, lda, stride);
+      zgemm_dmma_kernel<true><<<tiles * batch, 256, kGemmSmem, s>>>(
+          m, m, kNB, -1.0, A + (size_t)next + (size_t)kk * lda, lda, stride, A + (size_t)kk + (size_t)next * lda, lda,
+          stride, 1.0, A + (size_t)next + (size_t)next * lda, lda, stride, tiles_m, tiles, batch, next, piv_dev, n,
+          info_dev, inv, nblk);
       count_launches(1);
     }
   }
-  // diagonal block inverses for the solves
-  const int nblk = n / kNB;
-  ztri_inv_kernel<<<dim3(nblk, batch), 128, smem, s>>>(A, lda, stride, nblk, (double2*)work_dev);
-  count_launches(1);
   BEM_CUDA_CHECK(cudaGetLastError());
   return BEM_OK;
 }

@@ -1238,7 +1238,7 @@ int refine_loop(Solve solve_in_place, int* done, int* mdone, const void* K_dev, 
                 int npad,
                 int batch, const void* B_dev, void* X_dev, void* R_dev, int64_t ldb, int64_t strideB, int nrhs,
                 double tol, int max_iter, void* ts_work_dev, double* norms_dev, int* iters_out, double* resid_out,
-                cudaStream_t s) {
+                cudaStream_t s, int first_group = 4) {
   const int nvec = batch * nrhs;
   double* bn = norms_dev;
   double* rn = norms_dev + nvec;
@@ -1261,11 +1261,13 @@ int refine_loop(Solve solve_in_place, int* done, int* mdone, const void* K_dev, 
   BEM_CUDA_CHECK(cudaMemsetAsync(state, 0, 2 * sizeof(double), s));
   // Iterations are enqueued in groups without host synchronisation; once the
   // device-side test has converged the rest of the group returns at once.
+  // first_group: the first group's size (float64 factors converge in one
+  // iteration, and the kernels of three more cost 30 launches for nothing).
   constexpr int kGroup = 4;
   double host_state[2] = {0.0, 0.0};
   int enqueued = 0;
   while (enqueued < max_iter) {
-    const int group = std::min(kGroup, max_iter - enqueued);
+    const int group = std::min(enqueued == 0 ? first_group : kGroup, max_iter - enqueued);
     for (int g = 0; g < group; ++g) {
       // r <- F^{-1} r in place (the padded rows of r stay zero)
       int st = solve_in_place(R_dev, (const int*)done, (const int*)mdone);
@@ -1342,5 +1344,5 @@ extern "C" int bem_zlu_refine_solve(const void* K_dev, int64_t ldk, int64_t stri
                              err_dev, s, skip, kDefaultSpinLimit, mskip);
   };
   return refine_loop(solve, done, mdone, K_dev, ldk, strideK, n, npad, batch, B_dev, X_dev, R_dev, ldb, strideB, nrhs, tol,
-                     max_iter, ts_work_dev, norms_dev, iters_out, resid_out, s);
+                     max_iter, ts_work_dev, norms_dev, iters_out, resid_out, s, 1);
 }

@@ -1,0 +1,50 @@
+"""The float64 LU at the sizes where its blocks, panels and tiles change shape:
+factors and triangle inverses against numpy, pivots inside the 64-row blocks.
+
+Bars: the factors are compared through P A = L U, whose backward error is a few
+eps times n |L| |U| / |A| (below 1e-12 for these matrices of moderate growth);
+the triangles' inverses through L11 inv(L11) = 1, a few eps times 64 times the
+blocks' condition (below 1e3 here)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from capytaine_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _vp(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("n,batch", [(64, 1), (128, 5), (192, 2), (448, 3), (832, 1)])
+def test_factors_reproduce_the_matrix(n, batch):
+    import torch
+    rng = np.random.default_rng(n)
+    lib = _lib.load()
+    mats = []
+    for b in range(batch):
+        m = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        for k in range(0, n, 64):  # the pivots of each block in a random order of its rows
+            m[k + rng.permutation(64), k + np.arange(64)] += 3 * np.sqrt(n)
+        mats.append(m)
+    A = torch.as_tensor(np.array([m.T for m in mats]), device="cuda").contiguous()
+    piv = torch.empty((batch, n), dtype=torch.int32, device="cuda")
+    info = torch.zeros(batch, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(lib.bem_zlu_workspace_bytes(n, batch)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.bem_zlu_factor(_vp(A), n, n, n * n, batch, _vp(piv), _vp(info), _vp(work), _lib.stream_ptr()))
+    F, p = A.cpu().numpy(), piv.cpu().numpy()
+    inv = work.cpu().numpy()[:batch * (n // 64) * 2 * 4096 * 16].view(np.complex128).reshape(batch, n // 64, 2, 64, 64)
+    assert info.cpu().numpy().tolist() == [0] * batch
+    for b in range(batch):
+        lu = F[b].T
+        L, U = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+        rows = np.concatenate([k + p[b, k:k + 64] for k in range(0, n, 64)])
+        assert sorted(rows) == list(range(n))
+        assert np.abs(L @ U - mats[b][rows]).max() < 1e-12 * np.abs(mats[b]).max()
+        for i in range(n // 64):
+            s = slice(64 * i, 64 * i + 64)
+            for tri, x in ((L[s, s], inv[b, i, 0].T), (U[s, s], inv[b, i, 1].T)):
+                assert np.abs(tri @ x - np.eye(64)).max() < 1e-11
