@@ -502,69 +502,45 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
                "l"(gsrc)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ int ld_acquire_i(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_i(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
 
-// Persistent block substitution with the block LU factors; B complex128 in
-// place.  Forward: y_i = b_i - sum_{j<i} L_ij y_j (unit block lower).  Backward:
-// x_i = A_ii^{-1} y_i - sum_{j>i} U'_ij x_j with U'_ij = A_ii^{-1} U_ij stored in
-// the factorisation, so each step of the dependency chain is one block product
-// in both sweeps.  Each CTA owns one 128-row block.  The off-diagonal blocks
-// of its dependencies stream through a ring of kRing shared-memory slots, a
-// quarter block (32 columns, real and imaginary planes) per slot, copied
-// asynchronously (16-byte pieces) kRing - 1 quarters ahead of the product, so
-// the next blocks load while the current one is multiplied; only the
-// right-hand side of a dependency waits for its flag.  Thread (r, h)
-// accumulates row r over the half h of each quarter's columns for all NC
-// columns (NC/2 16-byte broadcast reads of the right-hand sides); the halves
-// meet in P at the end of each block.
-// Ring sizes: 5 slots (188 KB with 8 right-hand sides, one CTA per SM) when
-// every block row of the launch is resident at once; 2 slots (88 KB, two
-// CTAs per SM) when the block rows fill more than one wave of SMs, where
-// twice the resident CTAs hide more latency than a deeper ring.
-constexpr int kRingDeep = 5, kRingShallow = 2;
-constexpr int kQCols = 32;                   // columns of a quarter block
-constexpr int kQFloats = 2 * kQCols * kB;    // one slot: [plane][column][row]
-
-// acc += Re(A) y and acci += Im(A) y over the quarter's half h of columns for
-// row r (two pair instructions per entry and right-hand side, y = (Re, Im));
-// fold_rhs turns the two into the complex product A y.
-template <int NC>
-__device__ __forceinline__ void quarter_times_rhs(const float* __restrict__ Tre, const float* __restrict__ Tim,
-                                                  const float2* __restrict__ Y, int r, int h,
-                                                  float2 (&acc)[NC], float2 (&acci)[NC]) {
-#pragma unroll 4
-  for (int mm = 16 * h; mm < 16 * h + 16; ++mm) {
-    const float ar = Tre[mm * kB + r], ai = Tim[mm * kB + r];
-    const float2 ar2 = make_float2(ar, ar), ai2 = make_float2(ai, ai);
-    const float4* y4 = reinterpret_cast<const float4*>(Y + mm * NC);
-#pragma unroll
-    for (int c2 = 0; c2 < NC / 2; ++c2) {
-      const float4 y = y4[c2];
-      const float2 y0 = make_float2(y.x, y.y), y1 = make_float2(y.z, y.w);
-      acc[2 * c2] = fma2(ar2, y0, acc[2 * c2]);
-      acci[2 * c2] = fma2(ai2, y0, acci[2 * c2]);
-      acc[2 * c2 + 1] = fma2(ar2, y1, acc[2 * c2 + 1]);
-      acci[2 * c2 + 1] = fma2(ai2, y1, acci[2 * c2 + 1]);
-    }
-  }
-}
-template <int NC>
-__device__ __forceinline__ void fold_rhs(float2 (&acc)[NC], float2 (&acci)[NC]) {
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    acc[c] = make_float2(acc[c].x - acci[c].y, acc[c].y + acci[c].x);
-    acci[c] = make_float2(0.0f, 0.0f);
-  }
-}
+// Persistent block substitution with the block LU factors.  Forward: y_i = b_i -
+// sum_{j<i} L_ij y_j (unit block lower).  Backward: x_i = A_ii^{-1} y_i -
+// sum_{j>i} U'_ij x_j with U'_ij = A_ii^{-1} U_ij stored in the factorisation, so
+// each step of the dependency chain is one block product in both sweeps.
+//
+// A CTA owns 32 rows of a 128-row block, four CTAs per block.  What bounds the
+// sweep is the chain of nblk steps, each the time from one block's publication
+// to the next one's: a poll, the 128 x NC solution from L2, the product, the
+// sum over the CTA's warps, the stores and the release.  With one CTA per
+// block the product alone (128 x 128 x NC on one SM) was most of a step of
+// 7 us with 4 right-hand sides and 23 with 16; a quarter of it on each of four SMs
+// makes it 3.2 and 9.1 (forward and backward solve of one 3741: 0.43 -> 0.19 ms,
+// of one 20493 with 16 right-hand sides 7.3 -> 2.9, of 15 x 6084 with 7 2.26 ->
+// 1.42, half of the HBM rate).
+//
+// The rows' blocks stream through a ring of shared-memory slots, 64 columns
+// (real and imaginary planes) each, copied two or three slots ahead of the products;
+// only the right-hand sides of a dependency wait for its flag.  Warp w takes
+// columns 8 w .. 8 w + 7 of a slot, a thread two rows and half of the columns of
+// B; the partial sums stay in registers until the end (folded once per block, so
+// that no float32 sum runs over more than 16 products before it is added to
+// the rest), then the eight warps meet in shared memory.
+// Solutions pass between CTAs as float32 in scratch (Yf: forward, Xb: backward,
+// [matrix][row][NC]): half the bytes of complex128, and a CTA of a block may
+// still read all of y_i while another already publishes x_i.  B gets the result
+// of the backward sweep.  flags[b][i] counts the block's CTAs that have
+// published (forward 1 .. 4, backward 5 .. 8), the ticket runs on as well: one
+// memset per solve.
+constexpr int kSubRows = 32, kSubs = kB / kSubRows;
+constexpr int kSlotCols = 64;
+constexpr int ring_slots(int nc) { return nc <= 8 ? 4 : 5; }  // the copies run this minus two slots ahead
+constexpr int kSlotFloats = 2 * kSlotCols * kSubRows;  // [plane][column][row]
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -572,183 +548,199 @@ __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-template <int NC, int kRing>
-__global__ void __launch_bounds__(256, kRing == kRingShallow ? 2 : 1) ctrsm_persistent_kernel(Planes W, int nblk, int batch,
-                                                               const float2* __restrict__ inv, double2* B,
-                                                               int64_t ldb, int64_t strideB, int nrhs, int forward,
-                                                               int* flags, int* ticket, int* err, const int* skip,
-                                                               long long spin_limit, int withheld,
-                                                               const int* mskip) {
-  static_assert(kRing >= 2, "the ring keeps one quarter in flight beside the one multiplied");
-  // quarters of the diagonal inverse staged at a time: all four, or two per
-  // pass when the ring has fewer than four slots (a divisor of 4, never more
-  // slots than the ring has)
-  constexpr int kDiagPass = kRing >= 4 ? 4 : 2;
-  static_assert(4 % kDiagPass == 0 && kDiagPass <= kRing, "diagonal staging must fit the ring");
+template <int NC, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
+    ctrsm_persistent_kernel(Planes W, int nblk, int batch, const float2* __restrict__ inv, double2* B, int64_t ldb,
+                            int64_t strideB, int nrhs, int forward, float2* Yf, float2* Xb, int* flags, int* ticket,
+                            int* err, const int* skip, long long spin_limit, int withheld, const int* mskip) {
   if (skip && *skip) return;  // refinement already converged
+  constexpr int kC = NC / 2;  // columns of a thread
+  constexpr int kSlots = ring_slots(NC), kAhead = kSlots - 2;
   extern __shared__ __align__(16) float fsmf[];
-  float* ring = fsmf;                                                  // kRing slots of kQFloats
-  float2* X = reinterpret_cast<float2*>(ring + kRing * kQFloats);      // X[r*NC + c]
-  float2* Y = X + kB * NC;                                             // Y[m*NC + c]
-  float2* P = Y + kB * NC;                                             // P[r*NC + c]
+  float* ring = fsmf;
+  float2* Y = reinterpret_cast<float2*>(ring + kSlots * kSlotFloats);  // Y[m * NC + c]
   __shared__ int s_t;
-  const int tid = threadIdx.x;
-  const int r = tid & (kB - 1), h = tid >> 7;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rp = lane & 15, ch = lane >> 4;  // rows 2 rp, 2 rp + 1; columns ch kC ..
+  const int total = kSubs * nblk * batch;
   if (tid == 0) s_t = atomicAdd(ticket, 1);
   __syncthreads();
-  const int t = s_t;
-  const int b = t % batch, step = t / batch;
+  const int t = s_t - (forward ? 0 : total);
+  const int sub = t % kSubs, b = (t / kSubs) % batch, step = t / (kSubs * batch);
   if (mskip && mskip[b]) return;  // converged matrix: every CTA of it returns, no wait targets it
   const int i = forward ? step : (nblk - 1 - step);
-  double2* Bb = B + (size_t)b * strideB;
-  const int r0 = i * kB;
-  for (int idx = tid; idx < kB * NC; idx += blockDim.x) {
-    const int rr = idx & (kB - 1), c = idx >> 7;
-    float2 v = make_float2(0.0f, 0.0f);
-    if (c < nrhs) {
-      const double2 d = __ldcg(Bb + (size_t)(r0 + rr) + (size_t)c * ldb);
-      v = make_float2((float)d.x, (float)d.y);
-    }
-    X[rr * NC + c] = v;
-  }
+  const int row0 = i * kB + sub * kSubRows;  // first row of this CTA
   const int ndep = forward ? i : (nblk - 1 - i);
+  const int target = forward ? kSubs : 2 * kSubs;
   const float* Wre = W.re + (size_t)b * W.stride;
   const float* Wim = W.im + (size_t)b * W.stride;
-  float2 acc[NC], acci[NC];
+  double2* Bb = B + (size_t)b * strideB;
+  auto copy_solution = [&](const float2* src) {  // 128 x NC of another block into Y
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    float4* d4 = reinterpret_cast<float4*>(Y);
+    float4 v[kB * NC / 512];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = acci[c] = make_float2(0.0f, 0.0f);
-  if (!forward) {
-    // x_i = A_ii^{-1} b_i - sum_j U'_ij x_j with U' = A_ii^{-1} U: the product
-    // with the diagonal inverse comes first, off the chain of dependencies,
-    // its four quarters staged kDiagPass at a time in the first slots
-    const float2* Inv = inv + ((size_t)b * nblk + i) * kB * kB;
-#pragma unroll 1
-    for (int q0 = 0; q0 < 4; q0 += kDiagPass) {
-      // columns [32 q0, 32 (q0 + kDiagPass)) of the inverse into slots 0 .. kDiagPass - 1
-      for (int idx = tid; idx < kDiagPass * kQCols * kB; idx += blockDim.x) {
-        const int col = q0 * kQCols + (idx >> 7), row = idx & (kB - 1);
-        const float2 v = __ldg(Inv + (size_t)col * kB + row);  // element (row, col)
-        float* slot = ring + (col / kQCols - q0) * kQFloats;
-        slot[(col % kQCols) * kB + row] = v.x;
-        slot[kQCols * kB + (col % kQCols) * kB + row] = v.y;
-      }
-      __syncthreads();
-#pragma unroll 1
-      for (int qq = q0; qq < q0 + kDiagPass; ++qq) {
-        const float* slot = ring + (qq - q0) * kQFloats;
-        quarter_times_rhs<NC>(slot, slot + kQCols * kB, X + qq * kQCols * NC, r, h, acc, acci);
-      }
-      __syncthreads();  // the slots are restaged by the next pass
-    }
-    fold_rhs<NC>(acc, acci);
-    if (h == 1) {
+    for (int u = 0; u < kB * NC / 512; ++u) v[u] = __ldcg(s4 + tid + 256 * u);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) P[r * NC + c] = acc[c];
-    }
-    __syncthreads();
-    if (h == 0) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float2 o = P[r * NC + c];
-        X[r * NC + c] = make_float2(acc[c].x + o.x, acc[c].y + o.y);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] = make_float2(0.0f, 0.0f);
-    __syncthreads();  // the slots are reused for the off-diagonal blocks
-  }
-  // quarter q of the dependencies (block q / 4, columns 32 (q % 4) ..) into
-  // its ring slot: 32 columns x 128 rows per plane, 8 sixteen-byte pieces per
-  // thread
-  const int nq = 4 * ndep;
+    for (int u = 0; u < kB * NC / 512; ++u) d4[tid + 256 * u] = v[u];
+  };
+  // slot q: columns 64 (q % 2) .. of dependency q / 2
+  const int nq = 2 * ndep;
   auto issue = [&](int q) {
-    const int jd = q >> 2, qq = q & 3;
-    const int j = forward ? jd : (nblk - 1 - jd);
-    float* slot = ring + (q % kRing) * kQFloats;
-    for (int idx = tid; idx < kQCols * 32; idx += blockDim.x) {
-      const int mm = idx >> 5, piece = idx & 31;
-      const size_t g = (size_t)(r0 + piece * 4) + (size_t)(j * kB + qq * kQCols + mm) * W.ld;
-      cp_async16(slot + mm * kB + piece * 4, Wre + g);
-      cp_async16(slot + kQCols * kB + mm * kB + piece * 4, Wim + g);
+    if (q < nq) {
+      const int j = forward ? (q >> 1) : (nblk - 1 - (q >> 1));
+      float* slot = ring + (q % kSlots) * kSlotFloats;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int idx = tid + 256 * u, col = idx >> 3, piece = idx & 7;
+        const size_t g = (size_t)(row0 + piece * 4) + (size_t)(j * kB + (q & 1) * kSlotCols + col) * W.ld;
+        cp_async16(slot + col * kSubRows + piece * 4, Wre + g);
+        cp_async16(slot + kSlotCols * kSubRows + col * kSubRows + piece * 4, Wim + g);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int q = 0; q < kAhead; ++q) issue(q);
+  // the outputs of this thread: idx = tid + 256 u, row idx / NC, column idx % NC
+  constexpr int kOut = kSubRows * NC / 256;
+  float2 own[kOut];
+#pragma unroll
+  for (int u = 0; u < kOut; ++u) {
+    const int idx = tid + 256 * u, row = idx / NC, c = idx % NC;
+    own[u] = make_float2(0.0f, 0.0f);
+    if (forward && c < nrhs) {
+      const double2 d = __ldcg(Bb + (size_t)(row0 + row) + (size_t)c * ldb);
+      own[u] = make_float2((float)d.x, (float)d.y);
+    }
+  }
+  float2 tot[2][kC], acc[2][kC], acci[2][kC];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < kC; ++c) tot[h][c] = acc[h][c] = acci[h][c] = make_float2(0.0f, 0.0f);
+  // acc += Re(A) y, acci += Im(A) y for one column of A; fold: tot += their complex product
+  auto column = [&](float2 ar, float2 ai, const float2* y) {
+    const float2 r0 = make_float2(ar.x, ar.x), r1 = make_float2(ar.y, ar.y);
+    const float2 i0 = make_float2(ai.x, ai.x), i1 = make_float2(ai.y, ai.y);
+    const float4* y4 = reinterpret_cast<const float4*>(y + ch * kC);
+#pragma unroll
+    for (int c2 = 0; c2 < kC / 2; ++c2) {
+      const float4 v = y4[c2];
+      const float2 v0 = make_float2(v.x, v.y), v1 = make_float2(v.z, v.w);
+      acc[0][2 * c2] = fma2(r0, v0, acc[0][2 * c2]);
+      acci[0][2 * c2] = fma2(i0, v0, acci[0][2 * c2]);
+      acc[1][2 * c2] = fma2(r1, v0, acc[1][2 * c2]);
+      acci[1][2 * c2] = fma2(i1, v0, acci[1][2 * c2]);
+      acc[0][2 * c2 + 1] = fma2(r0, v1, acc[0][2 * c2 + 1]);
+      acci[0][2 * c2 + 1] = fma2(i0, v1, acci[0][2 * c2 + 1]);
+      acc[1][2 * c2 + 1] = fma2(r1, v1, acc[1][2 * c2 + 1]);
+      acci[1][2 * c2 + 1] = fma2(i1, v1, acci[1][2 * c2 + 1]);
     }
   };
-#pragma unroll 1
-  for (int q = 0; q < kRing - 1; ++q) {
-    if (q < nq) issue(q);
-    cp_async_commit();
+  auto fold = [&](float sign) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < kC; ++c) {
+        tot[h][c].x += sign * (acc[h][c].x - acci[h][c].y);
+        tot[h][c].y += sign * (acc[h][c].y + acci[h][c].x);
+        acc[h][c] = acci[h][c] = make_float2(0.0f, 0.0f);
+      }
+  };
+  if (!forward) {
+    // - A_ii^{-1} y_i, off the chain of dependencies: the inverse straight from
+    // global memory, two rows of a column per thread
+    copy_solution(Yf + ((size_t)b * nblk + i) * kB * NC);
+    __syncthreads();
+    const float2* Inv = inv + ((size_t)b * nblk + i) * kB * kB + sub * kSubRows + 2 * rp;
+    float4 v[8];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+      for (int mm = 0; mm < 8; ++mm)
+        v[mm] = __ldg(reinterpret_cast<const float4*>(Inv + (size_t)(16 * warp + 8 * half + mm) * kB));
+#pragma unroll
+      for (int mm = 0; mm < 8; ++mm)
+        column(make_float2(v[mm].x, v[mm].z), make_float2(v[mm].y, v[mm].w), Y + (16 * warp + 8 * half + mm) * NC);
+    }
+    fold(-1.0f);
   }
 #pragma unroll 1
   for (int q = 0; q < nq; ++q) {
-    const int jd = q >> 2, qq = q & 3;
-    __syncthreads();  // every thread is done with the slot refilled below (and with Y, at a new block)
-    if (qq == 0) {
-      const int j = forward ? jd : (nblk - 1 - jd);
+    if ((q & 1) == 0) {
+      const int j = forward ? (q >> 1) : (nblk - 1 - (q >> 1));
       if (tid == 0) {
         long long it = 0;
-        while (ld_acquire_i(flags + (size_t)b * nblk + j) == 0) {
+        while (ld_acquire_i(flags + (size_t)b * nblk + j) < target) {
           if (++it > spin_limit) {
             atomicExch(err, 1);
             break;
           }
-          __nanosleep(64);
+          __nanosleep(20);
         }
       }
-      __syncthreads();
-      for (int idx = tid; idx < kB * NC; idx += blockDim.x) {
-        const int m = idx & (kB - 1), c = idx >> 7;
-        float2 v = make_float2(0.0f, 0.0f);
-        if (c < nrhs) {
-          const double2 d = __ldcg(Bb + (size_t)(j * kB + m) + (size_t)c * ldb);
-          v = make_float2((float)d.x, (float)d.y);
-        }
-        Y[m * NC + c] = v;
-      }
+      __syncthreads();  // the dependency is there, and everyone is done with Y
+      copy_solution((forward ? Yf : Xb) + ((size_t)b * nblk + j) * kB * NC);
     }
-    if (q + kRing - 1 < nq) issue(q + kRing - 1);
-    cp_async_commit();
-    cp_async_wait_group<kRing - 1>();  // this thread's copies of quarter q have landed
-    __syncthreads();                   // everyone's copies, and Y
-    const float* slot = ring + (q % kRing) * kQFloats;
-    quarter_times_rhs<NC>(slot, slot + kQCols * kB, Y + qq * kQCols * NC, r, h, acc, acci);
-    if (qq == 3) {
-      fold_rhs<NC>(acc, acci);
-      if (h == 1) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) P[r * NC + c] = acc[c];
-      }
-      __syncthreads();
-      if (h == 0) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float2 o = P[r * NC + c];
-          float2 x = X[r * NC + c];
-          x.x -= acc[c].x + o.x;
-          x.y -= acc[c].y + o.y;
-          X[r * NC + c] = x;
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] = make_float2(0.0f, 0.0f);
-    }
+    // that slot was read two products ago: a barrier lies between
+    issue(q + kAhead);
+    cp_async_wait_group<kAhead>();  // this thread's copies of slot q have landed
+    __syncthreads();                // everyone's, and Y
+    const float* re = ring + (q % kSlots) * kSlotFloats + 8 * warp * kSubRows + 2 * rp;
+    const float* im = re + kSlotCols * kSubRows;
+    const float2* y = Y + ((q & 1) * kSlotCols + 8 * warp) * NC;
+#pragma unroll 4
+    for (int mm = 0; mm < 8; ++mm)
+      column(*reinterpret_cast<const float2*>(re + mm * kSubRows), *reinterpret_cast<const float2*>(im + mm * kSubRows),
+             y + mm * NC);
+    if (q & 1) fold(1.0f);
   }
-  cp_async_wait_all();
-  // forward (unit block lower factor): y_i = X; backward: x_i = X
+  cp_async_wait_group<0>();
   __syncthreads();
-  for (int idx = tid; idx < kB * NC; idx += blockDim.x) {
-    const int rr = idx & (kB - 1), c = idx >> 7;
-    if (c < nrhs) {
-      const float2 v = X[rr * NC + c];
-      Bb[(size_t)(r0 + rr) + (size_t)c * ldb] = make_double2((double)v.x, (double)v.y);
+  // the warps' sums: red[warp][row][column] in the ring
+  float2* red = reinterpret_cast<float2*>(ring);
+  static_assert(8 * kSubRows * NC * sizeof(float2) <= kSlots * kSlotFloats * sizeof(float), "the sums fit the ring");
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < kC; c += 2)
+      *reinterpret_cast<float4*>(red + (warp * kSubRows + 2 * rp + h) * NC + ch * kC + c) =
+          make_float4(tot[h][c].x, tot[h][c].y, tot[h][c + 1].x, tot[h][c + 1].y);
+  __syncthreads();
+  float2* dst = (forward ? Yf : Xb) + ((size_t)b * nblk + i) * kB * NC + sub * kSubRows * NC;
+#pragma unroll
+  for (int u = 0; u < kOut; ++u) {
+    const int idx = tid + 256 * u;
+    float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const float2 o = red[w * kSubRows * NC + idx];
+      v.x += o.x;
+      v.y += o.y;
     }
+    own[u] = make_float2(own[u].x - v.x, own[u].y - v.y);
+    dst[idx] = own[u];
   }
-  __threadfence();
   __syncthreads();
   // withheld >= 0 only from the bounded-wait test entry point: that block row
-  // never publishes its flag, so the waits on it run out
-  if (tid == 0 && i != withheld) st_release_i(flags + (size_t)b * nblk + i, 1);
+  // never publishes, so the waits on it run out
+  if (tid == 0 && i != withheld) {
+    __threadfence();
+    atomicAdd(flags + (size_t)b * nblk + i, 1);
+  }
+  if (!forward) {
+#pragma unroll
+    for (int u = 0; u < kOut; ++u) {
+      const int idx = tid + 256 * u, row = idx / NC, c = idx % NC;
+      if (c < nrhs) Bb[(size_t)(row0 + row) + (size_t)c * ldb] = make_double2((double)own[u].x, (double)own[u].y);
+    }
+  }
 }
 
-constexpr int trsm_smem_bytes(int nc, int ring) { return ring * kQFloats * (int)sizeof(float) + 3 * kB * nc * (int)sizeof(float2); }
+constexpr int trsm_smem_bytes(int nc) {
+  return ring_slots(nc) * kSlotFloats * (int)sizeof(float) + kB * nc * (int)sizeof(float2);
+}
 
 // x += r (the correction solved in place in r), then r = b for the residual.
 __global__ void ir_update_kernel(double2* __restrict__ X, double2* __restrict__ R, const double2* __restrict__ Bv,
@@ -822,15 +814,12 @@ bool g_mixed_configured = false;
 int configure_mixed() {
   if (g_mixed_configured) return BEM_OK;
   BEM_CUDA_CHECK(cudaFuncSetAttribute(clu_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjOutBytes));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, kRingDeep>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem_bytes(8, kRingDeep)));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<16, kRingDeep>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem_bytes(16, kRingDeep)));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, kRingShallow>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem_bytes(8, kRingShallow)));
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<16, kRingShallow>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      trsm_smem_bytes(16, kRingShallow)));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      trsm_smem_bytes(8)));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      trsm_smem_bytes(8)));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      trsm_smem_bytes(16)));
   g_mixed_configured = true;
   return BEM_OK;
 }
@@ -1173,24 +1162,27 @@ int clu_solve_enqueue(void* work_dev, int npad, int batch, void* B_dev, int64_t 
   int launches = 0;
   int sms = 0;
   if ((st = sm_count(&sms))) return st;
-  // more block rows than SMs: two CTAs per SM with the shallow ring
-  const bool shallow = (long long)nblk * batch > sms;
+  // more CTAs than two per SM hold: three per SM (85 registers, a few spilled)
+  // stream the factors faster (15 x 6144: 1.42 ms a solve against 1.49; 60 x
+  // 1536: 0.36 against 0.39), where all are resident the chain alone counts
+  // (one 3741: 0.21 against 0.19)
+  const bool crowded = (long long)kSubs * nblk * batch > 2 * sms;
+  // scratch for the solutions passed between CTAs: the factorisation's packed
+  // operands are free by now (2 x npad x 16 of their 3 x npad x 256 values)
+  float2* Yf = reinterpret_cast<float2*>(w.Aop);
+  float2* Xb = Yf + (size_t)batch * npad * kRhs;
   for (int c0 = 0; c0 < nrhs; c0 += kRhs) {
     const int nc = std::min(kRhs, nrhs - c0);
     double2* Bc = (double2*)B_dev + (size_t)c0 * ldb;
+    BEM_CUDA_CHECK(cudaMemsetAsync(w.flags, 0, sizeof(int) * ((size_t)batch * nblk + 1), s));
     for (int forward = 1; forward >= 0; --forward) {
-      BEM_CUDA_CHECK(cudaMemsetAsync(w.flags, 0, sizeof(int) * ((size_t)batch * nblk + 1), s));
       TimedLaunch tl(kKCtrsm, s);
-#define BEM_CTRSM(NC, R)                                                                                \
-  ctrsm_persistent_kernel<NC, R><<<nblk * batch, 256, trsm_smem_bytes(NC, R), s>>>(                     \
-      W, nblk, batch, w.inv, Bc, ldb, strideB, nc, forward, w.flags, ticket, err_dev, skip, spin_limit, \
-      withheld, mskip)
-      if (nc <= 8) {
-        if (shallow) BEM_CTRSM(8, kRingShallow); else BEM_CTRSM(8, kRingDeep);
-      } else {
-        if (shallow) BEM_CTRSM(16, kRingShallow); else BEM_CTRSM(16, kRingDeep);
-      }
-#undef BEM_CTRSM
+      auto* kernel = nc > 8   ? ctrsm_persistent_kernel<16, 2>
+                     : crowded ? ctrsm_persistent_kernel<8, 3>
+                               : ctrsm_persistent_kernel<8, 2>;
+      kernel<<<kSubs * nblk * batch, 256, trsm_smem_bytes(nc <= 8 ? 8 : 16), s>>>(
+          W, nblk, batch, w.inv, Bc, ldb, strideB, nc, forward, Yf, Xb, w.flags, ticket, err_dev, skip, spin_limit,
+          withheld, mskip);
       ++launches;
     }
   }
