@@ -89,40 +89,40 @@ __global__ void convert_pad_kernel(const double2* __restrict__ K, int64_t ldk, i
   }
 }
 
-// Gauss-Jordan inverse of a diagonal block: 8 warps, thread (warp w, lane l)
-// owns rows l + 32 a (a < 4) and columns w + 8 m (m < 16) of the 128 x 128
-// block in registers; column j = 8 m + w is slot m of warp w.
+// Gauss-Jordan inverse of a diagonal block in panels of 8 columns, one per warp:
+// warp w has columns 8 w .. 8 w + 7 of the 128 x 128 block, which lies in shared
+// memory as two planes; lane l has the rows 2 l, 2 l + 1, 64 + 2 l and 65 + 2 l.
 // Pivoting is implicit: rows never move.  Step j picks the pivot of column j
 // among the rows not yet used as pivot rows (row p_j) and eliminates column j
 // from every other row with the unnormalised row p_j:
 //   a_r -= (a_rj / a_pj) a_p   (r != p_j),
 // the in-place inverse's column j ending as -a_rj / a_pj, with 1 in row p_j.
+// The eight steps of a panel act on a column x outside it as
+//   x <- x + sum_s (P_s - e_{p_s}) x_{p_s},
+// P_s the panel's columns after its steps and x_{p_s} the column's entries in the
+// pivot rows before them (each step is I - f e_p^T, and P_s is the product of the
+// steps applied to e_{p_s}): a rank-8 update from the panel as it lies.
 // Row p_j thus stays scaled by its pivot; at the end
 //   A^{-1}(j', p_c) = a(p_j', c) / pivot_j'
-// (row p_j' holds the j'-th pivot row, the slot of column c the inverse's
+// (row p_j' holds the j'-th pivot row, the place of column c the inverse's
 // column p_c).
-#ifndef BEM_GJ_WARPS
-#define BEM_GJ_WARPS 8
-#endif
-#ifndef BEM_GJ_DEPTH
-#define BEM_GJ_DEPTH 4
-#endif
-constexpr int kGjWarps = BEM_GJ_WARPS;
-constexpr int kGjSlots = kB / kGjWarps;  // columns per warp
-constexpr int kGjDepth = BEM_GJ_DEPTH;   // pivot columns published ahead of the slowest warp
-static_assert(kGjSlots <= 16 && kGjWarps * kGjSlots == kB, "a warp holds at most 16 columns of the block");
-constexpr int kGjLd = kB + 1;            // column stride of the staged inverse (fewer bank conflicts)
-constexpr int kGjOutBytes = kB * kGjLd * (int)sizeof(float2);  // dynamic shared memory of the inverse
+constexpr int kGjPanel = 8;               // columns per warp and panel
+constexpr int kGjWarps = kB / kGjPanel;
+constexpr int kGjDepth = 4;               // panels published ahead of the slowest warp
+constexpr int kGjLd = kB + 2;             // column stride of a plane (row pairs aligned, two-way conflicts across)
+constexpr int kGjSmem = (2 * kB * kGjLd + kGjDepth * kGjPanel * 2 * kB) * (int)sizeof(float);  // dynamic
 constexpr long long kGjWaitLimit = 1ll << 22;  // polls of a bounded wait (about a second)
 
-// acc - a b in two fused multiply-adds per component, in this order:
-//   acc.x = fmaf(a.y, b.y, fmaf(-a.x, b.x, acc.x)),
-//   acc.y = fmaf(-a.y, b.x, fmaf(-a.x, b.y, acc.y)),
-// as two pair instructions: an = (-a.x, -a.x), ay = (a.y, -a.y) (once per
-// multiplier), b and bs = (b.y, b.x) (once per pivot-row entry).
-__device__ __forceinline__ float2 cfms2(float2 acc, float2 an, float2 ay, float2 b, float2 bs) {
-  return fma2(ay, bs, fma2(an, b, acc));
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 ra, rb, rd;\n"
+      "mov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\n"
+      "mul.rn.f32x2 rd, ra, rb;\nmov.b64 {%0, %1}, rd;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
 __device__ __forceinline__ uint32_t gj_smem(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -144,17 +144,16 @@ __device__ __forceinline__ bool gj_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 struct GjShared {
-  // full[s]: the column of buffer s is published (32 arrivals, the owner's
-  // lanes); empty[s]: every warp has read it (8 arrivals, one per warp).
+  // full[s]: the panel of buffer s is published (32 arrivals, the owner's
+  // lanes); empty[s]: every other warp has read it (15 arrivals, one per warp).
   uint64_t full[kGjDepth];
   uint64_t empty[kGjDepth];
-  float2 colbuf[kGjDepth][kB];      // pivot column of step j in buffer j % kGjDepth, by row
-  alignas(16) float2 xbuf[kGjWarps][kGjSlots];  // per warp: its entries of the pivot row
+  // per warp: entries (re, re, im, im) of pivot rows in its columns
+  alignas(16) float4 rows[kGjWarps][kGjPanel][kGjPanel];
   float2 rowscale[kB];              // 1 / pivot of the step whose pivot row is this row
-  int piv_row[kB];                  // pivot row of each step
-  int jinv[kB];                     // step of each pivot row
-  unsigned used[kB / 32];           // rows already used as pivot rows
-  int s_piv[kGjDepth];              // pivot row of the column in each buffer
+  alignas(16) int piv_row[kB];      // pivot row of each step
+  alignas(16) int jinv[kB];         // step of each pivot row
+  unsigned char used[kB];           // rows already used as pivot rows
   int abort;                        // a wait ran out: every warp leaves
 };
 
@@ -181,238 +180,311 @@ __device__ __forceinline__ bool gj_wait(uint64_t* bar, uint32_t parity, GjShared
   return __all_sync(0xffffffffu, ok);
 }
 
-// Column j (register slot M of this warp) after the update of step j - 1
-// (multipliers f, pivot-row entry um; f = 0 for column 0): pivot among the
-// unused rows, the column published to buffer j % kGjDepth with its pivot
-// row; flags an exactly zero pivot in info.  Returns the pivot row (the slot
-// becomes the unit vector of that row once the warp's own update of step
-// j - 1 is done).
-template <int M>
-__device__ __forceinline__ int gj_publish(const float2 (&a)[4][kGjSlots], const float2 (&f)[4], float2 um, int j,
-                                          int kk, int b, int lane, GjShared& sh, int* __restrict__ info) {
-  constexpr int S = M < kGjSlots ? M : 0;  // M >= kGjSlots: a case the switch never takes
-  float2 t[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    t[i] = cfms2(a[i][S], make_float2(-f[i].x, -f[i].x), make_float2(f[i].y, -f[i].y), um, make_float2(um.y, um.x));
-  // this lane's candidate: the largest |t| among its unused rows (the first of
-  // equal ones, the smallest row), as an ordered key (the bits of the
-  // non-negative float plus one; 0: none, the used rows and NaN); then the
-  // largest key of the warp and, among equal keys, the smallest row
-  unsigned key = 0u;
-  int li = kB;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float av = fabs1(t[i]);
-    const unsigned kv = (((sh.used[i] >> lane) & 1u) || isnan(av)) ? 0u : __float_as_uint(av) + 1u;
-    if (kv > key) {
-      key = kv;
-      li = lane + 32 * i;
-    }
-  }
-  const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
-  int bi = (int)__reduce_min_sync(0xffffffffu, key == kmax ? (unsigned)li : (unsigned)kB);
-  const float best = kmax ? __uint_as_float(kmax - 1u) : -1.0f;
-  if (bi >= kB) {  // no comparable candidate (NaN): the first unused row
-#pragma unroll
-    for (int i = 3; i >= 0; --i)
-      if (~sh.used[i]) bi = 32 * i + __ffs(~sh.used[i]) - 1;
-  }
-  const int s = j % kGjDepth;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sh.colbuf[s][lane + 32 * i] = t[i];
-  if (lane == 0) {
-    sh.s_piv[s] = bi;
-    sh.piv_row[j] = bi;
-    sh.used[bi >> 5] |= 1u << (bi & 31);
-    if (!(best > 0.0f) && info[b] == 0) info[b] = kk + j + 1;
-  }
-  gj_arrive(&sh.full[s]);  // release: this lane's writes above
-  return bi;
+// Ordered key of a pivot candidate: the bits of |re| + |im| with the last seven
+// replaced by the row, so that one reduction finds the value and the row
+// (values within 2^-16 of the largest count as equal and the first row wins).
+// A NaN counts as zero; left: all ones, or 0 for a row already used (key 0).
+__device__ __forceinline__ unsigned gj_key(float re, float im, int row, unsigned left) {
+  const float m = fmaxf(fabsf(re) + fabsf(im), 0.0f);
+  return (((__float_as_uint(m) + 128u) & ~127u) | (unsigned)(127 - row)) & left;
 }
 
-template <int M>
-__device__ __forceinline__ void gj_unit(float2 (&a)[4][kGjSlots], int bi, int lane) {
-  constexpr int S = M < kGjSlots ? M : 0;  // M >= kGjSlots: a case the switch never takes
+// A warp's columns in registers: [pair of rows][column], planes apart.
+struct GjColumns {
+  float2 re[2][kGjPanel], im[2][kGjPanel];
+};
+
+// acc += p y, y = (re, re, im, im) of one column's pivot-row entry, p two rows.
+__device__ __forceinline__ void gj_fma(float2& re, float2& im, float2 pr, float2 pi, float2 npi, float4 y) {
+  const float2 yr = make_float2(y.x, y.y), yi = make_float2(y.z, y.w);
+  re = fma2(npi, yi, fma2(pr, yr, re));
+  im = fma2(pi, yr, fma2(pr, yi, im));
+}
+
+// The eight steps of panel q on its own columns, by its warp: a becomes P.  The
+// columns rotate through the register slots (the current one in slot 0, each
+// update landing one slot below, the finished column in the last), so that the
+// loop is 400 instructions; eight steps bring every column back to its slot.
+__device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, int lane, GjShared& sh,
+                                          int* __restrict__ info) {
+  const int r0 = 2 * lane;
+  unsigned left[4];  // rows r0, r0 + 1, r0 + 64, r0 + 65 not used yet
 #pragma unroll
-  for (int i = 0; i < 4; ++i) a[i][S] = make_float2(lane + 32 * i == bi ? 1.0f : 0.0f, 0.0f);
+  for (int i = 0; i < 4; ++i) left[i] = sh.used[r0 + (i & 1) + 64 * (i >> 1)] ? 0u : ~0u;
+  auto column_key = [&]() {
+    const unsigned k0 = max(gj_key(a.re[0][0].x, a.im[0][0].x, r0, left[0]),
+                            gj_key(a.re[0][0].y, a.im[0][0].y, r0 + 1, left[1]));
+    const unsigned k1 = max(gj_key(a.re[1][0].x, a.im[1][0].x, r0 + 64, left[2]),
+                            gj_key(a.re[1][0].y, a.im[1][0].y, r0 + 65, left[3]));
+    return __reduce_max_sync(0xffffffffu, max(k0, k1));
+  };
+  unsigned key = column_key(), zeros = 0u;
+  int my_p = 0;  // of step s in lane s: stored once at the end
+  float2 my_scale = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+  for (int s = 0; s < kGjPanel; ++s) {
+    const int p = 127 - (int)(key & 127u), src = (p & 63) >> 1;
+    // the pivot row's entries from its lane (the branch is the warp's: p is)
+    float ur[kGjPanel], ui[kGjPanel];
+#define BEM_GJ_ROW(H, C)                                            \
+  _Pragma("unroll") for (int m = 0; m < kGjPanel; ++m) {            \
+    ur[m] = __shfl_sync(0xffffffffu, a.re[H][m].C, src);            \
+    ui[m] = __shfl_sync(0xffffffffu, a.im[H][m].C, src);            \
+  }
+    if (p & 64) {
+      if (p & 1) { BEM_GJ_ROW(1, y) } else { BEM_GJ_ROW(1, x) }
+    } else {
+      if (p & 1) { BEM_GJ_ROW(0, y) } else { BEM_GJ_ROW(0, x) }
+    }
+#undef BEM_GJ_ROW
+    const float d = ur[0] * ur[0] + ui[0] * ui[0];
+    float rd;  // 1 / d: the hardware's estimate and a Newton step
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rd) : "f"(d));
+    rd = d > 0.0f ? fmaf(rd, fmaf(-d, rd, 1.0f), rd) : 0.0f;
+    const float dr = ur[0] * rd, di = -ui[0] * rd;
+    const bool own[4] = {p == r0, p == r0 + 1, p == r0 + 64, p == r0 + 65};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) left[i] = own[i] ? 0u : left[i];
+    // multipliers a_rj / pivot; 0 on the pivot row, which stays as it is
+    float2 nr[2], fi[2], ni[2], done_re[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 ar = a.re[h][0], ai = a.im[h][0];
+      float2 f = fma2(ai, make_float2(-di, -di), mul2(ar, make_float2(dr, dr)));
+      fi[h] = fma2(ai, make_float2(dr, dr), mul2(ar, make_float2(di, di)));
+      if (own[2 * h]) f.x = fi[h].x = 0.0f;
+      if (own[2 * h + 1]) f.y = fi[h].y = 0.0f;
+      nr[h] = neg2(f);
+      ni[h] = neg2(fi[h]);
+      done_re[h] = make_float2(own[2 * h] ? 1.0f : nr[h].x, own[2 * h + 1] ? 1.0f : nr[h].y);
+    }
+#pragma unroll
+    for (int m = 1; m < kGjPanel; ++m) {
+      const float4 y = make_float4(ur[m], ur[m], ui[m], ui[m]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2 re = a.re[h][m], im = a.im[h][m];
+        gj_fma(re, im, nr[h], ni[h], fi[h], y);
+        a.re[h][m - 1] = re;
+        a.im[h][m - 1] = im;
+      }
+      // the next pivot's column came first: its reduction runs beside the others' updates
+      if (m == 1) key = column_key();
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      a.re[h][kGjPanel - 1] = done_re[h];
+      a.im[h][kGjPanel - 1] = ni[h];
+    }
+    if (lane == s) {
+      my_p = p;
+      my_scale = make_float2(dr, di);
+    }
+    zeros |= (fabsf(ur[0]) + fabsf(ui[0]) > 0.0f ? 0u : 1u) << s;
+  }
+  if (lane < kGjPanel) {
+    sh.piv_row[kGjPanel * q + lane] = my_p;
+    sh.rowscale[my_p] = my_scale;
+    sh.used[my_p] = 1;
+  }
+  if (zeros && lane == 0 && info[b] == 0) info[b] = kk + kGjPanel * q + __ffs(zeros);
 }
 
 // Inverse of the diagonal block A_kk by Gauss-Jordan elimination with partial
-// pivoting among its rows (implicit, see above), the block in registers.  The
-// warps do not step together: the owner of column j + 1 updates that column
-// first, picks its pivot and publishes it (shared-memory buffers guarded by
-// mbarriers, kGjDepth columns deep) before its update of the other columns,
-// so that the pivot search of the next column overlaps the rank-one updates
-// of the other warps; every warp takes the pivot row's entries of its own
-// columns from its own lanes.  The step body is one loop over the columns
-// (register slots addressed through a switch only for the owner's column).
-// Output: inv (128 x 128, column-major) = A_kk^{-1}, and its packed copies for
-// the panel product (binv) and the block row of U' (ainv); info flags an
-// exactly zero pivot; err is set when a bounded wait runs out.
+// pivoting among its rows (implicit, in panels, see above).  The warps do not
+// step together: panel q's warp factors it as soon as it has applied panel
+// q - 1, and publishes it (shared-memory buffers guarded by mbarriers, kGjDepth
+// panels deep) while the other warps still apply the earlier ones; those that
+// share its scheduler (warps a multiple of four apart) stay a panel behind.
+// Bound: the chain of panels on one SM, 8000 cycles each: the factorisation 4400
+// (540 a column: shuffles of the pivot row, reciprocal, multipliers, the key and
+// its reduction), the next warp's rank-8 update 2050, the exchange 1300; the
+// other warps' updates (5000 a scheduler) run beside it.  80 us per block.  One
+// step per exchange took 1800 cycles a column (121 us per block with the packed
+// copies written by the same CTA): a pivot search, two trips through shared
+// memory and a barrier each.  Row pairs and duplicated pivot entries feed the
+// pair instructions without moves; interleaved complex entries in registers
+// spent as much on moves and divergent row extraction as panels saved (170 us).
+// Output: inv (128 x 128, column-major) = A_kk^{-1}; info flags an exactly zero
+// pivot; err is set when a bounded wait runs out.
 __global__ void __launch_bounds__(32 * kGjWarps, 1) clu_gj_kernel(Planes W, int kk, int* __restrict__ info,
                                                                  float2* __restrict__ inv, int nblk,
-                                                                 float* __restrict__ binv,
-                                                                 float* __restrict__ ainv, int* __restrict__ err) {
+                                                                 int* __restrict__ err) {
+  extern __shared__ __align__(16) float gj_smem_f[];
+  float* Mre = gj_smem_f;              // the block: element (r, c) at c * kGjLd + r
+  float* Mim = Mre + kB * kGjLd;
+  float* panels = Mim + kB * kGjLd;    // [buffer][column][plane][row]
   __shared__ GjShared sh;
   const int b = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, w = tid >> 5;
-  float2 a[4][kGjSlots];
+  const int r0 = 2 * lane;
+  {
+    const float* gr = W.re + (size_t)b * W.stride + (size_t)kk + r0;
+    const float* gi = W.im + (size_t)b * W.stride + (size_t)kk + r0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int m = 0; m < kGjPanel; ++m) {
+      const int c = kGjPanel * w + m;
 #pragma unroll
-    for (int m = 0; m < kGjSlots; ++m) a[i][m] = ldp(W, b, kk + lane + 32 * i, kk + w + kGjWarps * m);
-  if (tid < kB / 32) sh.used[tid] = 0u;
+      for (int h = 0; h < 2; ++h) {
+        const size_t g = (size_t)(kk + c) * W.ld + 64 * h;
+        *reinterpret_cast<float2*>(Mre + c * kGjLd + r0 + 64 * h) = *reinterpret_cast<const float2*>(gr + g);
+        *reinterpret_cast<float2*>(Mim + c * kGjLd + r0 + 64 * h) = *reinterpret_cast<const float2*>(gi + g);
+      }
+    }
+  }
   if (tid < kGjDepth) {
     gj_bar_init(&sh.full[tid], 32);
-    gj_bar_init(&sh.empty[tid], kGjWarps);
+    gj_bar_init(&sh.empty[tid], kGjWarps - 1);
   }
+  if (tid < kB) sh.used[tid] = 0;
   if (tid == 0) sh.abort = 0;
   __syncthreads();
-  float2 f[4];
-  if (w == 0) {  // column 0: slot 0 of warp 0, nothing to update yet
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = make_float2(0.0f, 0.0f);
-    const int bi = gj_publish<0>(a, f, make_float2(0.0f, 0.0f), 0, kk, b, lane, sh, info);
-    gj_unit<0>(a, bi, lane);
-  }
-  float2* xw = sh.xbuf[w];
+  float* const mr = Mre + kGjPanel * w * kGjLd + r0;  // this lane's rows of the warp's columns
+  float* const mi = Mim + kGjPanel * w * kGjLd + r0;
+  GjColumns a;
 #pragma unroll 1
-  for (int j = 0; j < kB; ++j) {
-    const int s = j % kGjDepth;
-    if (!gj_wait(&sh.full[s], (j / kGjDepth) & 1, sh, err)) break;
-    const int p = sh.s_piv[s];
-    const int lp = p & 31, sp = p >> 5;
-    if (lane == lp) {
-      switch (sp) {  // one lane: a branch per register slot instead of selects
-#define BEM_GJ_ROWOUT(S) \
-  case S:                \
-    _Pragma("unroll") for (int m = 0; m < kGjSlots; m += 2) \
-      reinterpret_cast<float4*>(xw)[m / 2] = make_float4(a[S][m].x, a[S][m].y, a[S][m + 1].x, a[S][m + 1].y); \
-    break;
-        BEM_GJ_ROWOUT(0) BEM_GJ_ROWOUT(1) BEM_GJ_ROWOUT(2) BEM_GJ_ROWOUT(3)
-#undef BEM_GJ_ROWOUT
-      }
-    }
-    const float2 piv = sh.colbuf[s][p];
-    const float d = piv.x * piv.x + piv.y * piv.y;
-    const float rd = d > 0.0f ? __frcp_rn(d) : 0.0f;  // = 1.0f / d, correctly rounded
-    const float2 dinv = make_float2(piv.x * rd, -piv.y * rd);
-    if (tid == 0) sh.rowscale[p] = dinv;
-    // multipliers a_rj / pivot; 0 on the pivot row, which stays as it is
+  for (int q = 0; q < kGjWarps; ++q) {
+    const int s = q % kGjDepth, parity = (q / kGjDepth) & 1;
+    float* pan = panels + (size_t)s * kGjPanel * 2 * kB;
+    const bool owner = q == w;
+    if (!owner) {
+      if (!gj_wait(&sh.full[s], parity, sh, err)) break;
+      // the next panel's warp has its scheduler for itself until it has published
+      const int next = q + 1;
+      if (next < kGjWarps && w != next && ((w ^ next) & 3) == 0 &&
+          !gj_wait(&sh.full[next % kGjDepth], (next / kGjDepth) & 1, sh, err))
+        break;
+      // this warp's entries of the pivot rows, which then start from zero
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 c = sh.colbuf[s][lane + 32 * i];
-      f[i] = (lane + 32 * i == p) ? make_float2(0.0f, 0.0f) : fmul(c, dinv);
+      for (int u = 0; u < 2; ++u) {
+        const int e = (lane >> 3) + 4 * u, m = lane & 7;
+        const int o = (kGjPanel * w + m) * kGjLd + sh.piv_row[kGjPanel * q + e];
+        const float re = Mre[o], im = Mim[o];
+        sh.rows[w][e][m] = make_float4(re, re, im, im);
+        Mre[o] = 0.0f;
+        Mim[o] = 0.0f;
+      }
+      __syncwarp();
     }
-    __syncwarp();  // the pivot row is in the warp's buffer; the warp's reads of column j are done
-    if (lane == 0) gj_arrive(&sh.empty[s]);
-    const int nj = j + 1;
-    const bool owner = nj < kB && w == (nj & (kGjWarps - 1));
-    int bi = 0;
+#pragma unroll
+    for (int m = 0; m < kGjPanel; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        a.re[h][m] = *reinterpret_cast<const float2*>(mr + m * kGjLd + 64 * h);
+        a.im[h][m] = *reinterpret_cast<const float2*>(mi + m * kGjLd + 64 * h);
+      }
     if (owner) {
-      // buffer nj % kGjDepth is free once every warp has read column nj - kGjDepth
-      if (nj >= kGjDepth && !gj_wait(&sh.empty[nj % kGjDepth], ((nj / kGjDepth) - 1) & 1, sh, err)) break;
-      switch (nj / kGjWarps) {
-#define BEM_GJ_PUB(M) \
-  case M:             \
-    bi = gj_publish<M>(a, f, xw[M < kGjSlots ? M : 0], nj, kk, b, lane, sh, info); \
-    break;
-        BEM_GJ_PUB(0) BEM_GJ_PUB(1) BEM_GJ_PUB(2) BEM_GJ_PUB(3) BEM_GJ_PUB(4) BEM_GJ_PUB(5) BEM_GJ_PUB(6)
-        BEM_GJ_PUB(7) BEM_GJ_PUB(8) BEM_GJ_PUB(9) BEM_GJ_PUB(10) BEM_GJ_PUB(11) BEM_GJ_PUB(12) BEM_GJ_PUB(13)
-        BEM_GJ_PUB(14) BEM_GJ_PUB(15)
-#undef BEM_GJ_PUB
+      gj_factor(a, q, kk, b, lane, sh, info);
+      // the buffer is free once every other warp has read panel q - kGjDepth
+      if (q >= kGjDepth && !gj_wait(&sh.empty[s], parity ^ 1, sh, err)) break;
+#pragma unroll
+      for (int m = 0; m < kGjPanel; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          *reinterpret_cast<float2*>(pan + (2 * m) * kB + r0 + 64 * h) = a.re[h][m];
+          *reinterpret_cast<float2*>(pan + (2 * m + 1) * kB + r0 + 64 * h) = a.im[h][m];
+        }
+      gj_arrive(&sh.full[s]);  // release: this lane's writes above
+    } else {
+#pragma unroll 2
+      for (int e = 0; e < kGjPanel; ++e) {
+        float2 pr[2], pi[2], npi[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          pr[h] = *reinterpret_cast<const float2*>(pan + (2 * e) * kB + r0 + 64 * h);
+          pi[h] = *reinterpret_cast<const float2*>(pan + (2 * e + 1) * kB + r0 + 64 * h);
+          npi[h] = neg2(pi[h]);
+        }
+#pragma unroll
+        for (int m = 0; m < kGjPanel; ++m) {
+          const float4 y = sh.rows[w][e][m];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) gj_fma(a.re[h][m], a.im[h][m], pr[h], pi[h], npi[h], y);
+        }
       }
     }
-    // rank-one update of every column of the warp: a - f u (u the pivot row,
-    // read from the warp's buffer two entries per load)
-    float4 u4[kGjSlots / 2];
 #pragma unroll
-    for (int m = 0; m < kGjSlots / 2; ++m) u4[m] = reinterpret_cast<const float4*>(xw)[m];
-    float2 fn[4], fy[4];
+    for (int m = 0; m < kGjPanel; ++m)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      fn[i] = make_float2(-f[i].x, -f[i].x);
-      fy[i] = make_float2(f[i].y, -f[i].y);
-    }
-#pragma unroll
-    for (int m = 0; m < kGjSlots; ++m) {
-      const float2 um = (m & 1) ? make_float2(u4[m / 2].z, u4[m / 2].w) : make_float2(u4[m / 2].x, u4[m / 2].y);
-      const float2 us = make_float2(um.y, um.x);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i][m] = cfms2(a[i][m], fn[i], fy[i], um, us);
-    }
-    if (owner) {
-      switch (nj / kGjWarps) {
-#define BEM_GJ_UNIT(M) \
-  case M:              \
-    gj_unit<M>(a, bi, lane); \
-    break;
-        BEM_GJ_UNIT(0) BEM_GJ_UNIT(1) BEM_GJ_UNIT(2) BEM_GJ_UNIT(3) BEM_GJ_UNIT(4) BEM_GJ_UNIT(5) BEM_GJ_UNIT(6)
-        BEM_GJ_UNIT(7) BEM_GJ_UNIT(8) BEM_GJ_UNIT(9) BEM_GJ_UNIT(10) BEM_GJ_UNIT(11) BEM_GJ_UNIT(12)
-        BEM_GJ_UNIT(13) BEM_GJ_UNIT(14) BEM_GJ_UNIT(15)
-#undef BEM_GJ_UNIT
+      for (int h = 0; h < 2; ++h) {
+        *reinterpret_cast<float2*>(mr + m * kGjLd + 64 * h) = a.re[h][m];
+        *reinterpret_cast<float2*>(mi + m * kGjLd + 64 * h) = a.im[h][m];
       }
-    }
-    __syncwarp();  // the warp's reads of its buffer are done before the next step rewrites it
+    __syncwarp();  // the warp's reads of the panel are done, its columns are stored
+    if (!owner && lane == 0) gj_arrive(&sh.empty[s]);
   }
   __syncthreads();
   if (sh.abort) return;
   if (tid < kB) sh.jinv[sh.piv_row[tid]] = tid;
-  __syncthreads();
-  // A_kk^{-1}(jinv[r], piv_row[c]) = a(r, c) / pivot: staged in shared memory
-  // at its place (column-major, column stride kGjLd), so that the three
-  // outputs below are written with coalesced stores (the permuted rows would
-  // scatter every store otherwise).
-  extern __shared__ float2 gj_out[];  // kB columns of kGjLd
+  // rows scaled by their pivots' reciprocals
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = lane + 32 * i;
-    const int row = sh.jinv[r];
-    const float2 sc = sh.rowscale[r];
+  for (int h = 0; h < 2; ++h) {
+    const float2 s0 = sh.rowscale[r0 + 64 * h], s1 = sh.rowscale[r0 + 1 + 64 * h];
 #pragma unroll
-    for (int m = 0; m < kGjSlots; ++m)
-      gj_out[(size_t)sh.piv_row[w + kGjWarps * m] * kGjLd + row] = fmul(a[i][m], sc);
+    for (int m = 0; m < kGjPanel; ++m) {
+      float2* pr = reinterpret_cast<float2*>(mr + m * kGjLd + 64 * h);
+      float2* pi = reinterpret_cast<float2*>(mi + m * kGjLd + 64 * h);
+      const float2 re = *pr, im = *pi;
+      const float2 v0 = fmul(make_float2(re.x, im.x), s0), v1 = fmul(make_float2(re.y, im.y), s1);
+      *pr = make_float2(v0.x, v1.x);
+      *pi = make_float2(v0.y, v1.y);
+    }
   }
   __syncthreads();
-  // inv: column-major 128 x 128
-  float2* out = inv + ((size_t)b * nblk + kk / kB) * kB * kB;
-  for (int idx = tid; idx < kB * kB; idx += blockDim.x) {
-    const int row = idx & (kB - 1), col = idx >> 7;
-    out[idx] = gj_out[col * kGjLd + row];
+  // A_kk^{-1}(row, col) = a(piv_row[row], jinv[col]): column-major 128 x 128, four
+  // rows per thread
+  float4* out = reinterpret_cast<float4*>(inv + ((size_t)b * nblk + kk / kB) * kB * kB);
+#pragma unroll 1
+  for (int col = w; col < kB; col += kGjWarps) {
+    const int o = sh.jinv[col] * kGjLd;
+    const int4 p = *reinterpret_cast<const int4*>(sh.piv_row + 4 * lane);
+    out[col * (kB / 2) + 2 * lane] = make_float4(Mre[o + p.x], Mim[o + p.x], Mre[o + p.y], Mim[o + p.y]);
+    out[col * (kB / 2) + 2 * lane + 1] = make_float4(Mre[o + p.z], Mim[o + p.z], Mre[o + p.w], Mim[o + p.w]);
   }
-  // the A operand of U' = A_kk^{-1} A12: row r = [Re A_kk^{-1}(r, :) | Im A_kk^{-1}(r, :)]
-  float* ao = ainv + (size_t)b * kB * 2 * kB;
-  for (int idx = tid; idx < kB * kB; idx += blockDim.x) {
-    const int col = idx & (kB - 1), row = idx >> 7;
-    const float2 v = gj_out[col * kGjLd + row];
-    ao[(size_t)row * 2 * kB + col] = tf32_rn(v.x);
-    ao[(size_t)row * 2 * kB + kB + col] = tf32_rn(v.y);
+}
+
+// The inverse of block kk as the operands of two products, 8 columns and 8 rows
+// per CTA: the inverse's own CTA took 20 us for these 0.9 MB.
+// binv: B operand of the split-TF32 product L21 = A21 A_kk^{-1} (three K-blocks
+// of 256: hi, hi, lo; see clu_pack_kernel for the A side): row t
+// [Re X(:, t) | -Im X(:, t)] per block, row 128 + t [Im X(:, t) | Re X(:, t)].
+// ainv: A operand of U' = A_kk^{-1} A12, row r [Re A_kk^{-1}(r, :) | Im A_kk^{-1}(r, :)].
+__global__ void __launch_bounds__(256) clu_inverse_pack_kernel(const float2* __restrict__ inv, int nblk, int kk,
+                                                              float* __restrict__ binv, float* __restrict__ ainv) {
+  const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, t = 8 * blockIdx.x + (tid >> 5);
+  const float2* X = inv + ((size_t)b * nblk + kk / kB) * kB * kB;
+  {
+    const float4* col = reinterpret_cast<const float4*>(X + (size_t)t * kB) + 2 * lane;
+    const float4 v0 = col[0], v1 = col[1];
+    const float4 re = make_float4(v0.x, v0.z, v1.x, v1.z), im = make_float4(v0.y, v0.w, v1.y, v1.w);
+    const float4 hr = make_float4(tf32_hi(re.x), tf32_hi(re.y), tf32_hi(re.z), tf32_hi(re.w));
+    const float4 hi = make_float4(tf32_hi(im.x), tf32_hi(im.y), tf32_hi(im.z), tf32_hi(im.w));
+    const float4 lr = make_float4(re.x - hr.x, re.y - hr.y, re.z - hr.z, re.w - hr.w);
+    const float4 li = make_float4(im.x - hi.x, im.y - hi.y, im.z - hi.z, im.w - hi.w);
+    const float4 nh = make_float4(-hi.x, -hi.y, -hi.z, -hi.w), nl = make_float4(-li.x, -li.y, -li.z, -li.w);
+    float* bo = binv + (size_t)b * (2 * kB) * kSplitK;
+    float4* rr = reinterpret_cast<float4*>(bo + (size_t)t * kSplitK) + lane;
+    float4* ri = reinterpret_cast<float4*>(bo + (size_t)(kB + t) * kSplitK) + lane;
+    constexpr int kQ = kB / 4;
+    rr[0] = hr;
+    rr[kQ] = nh;
+    rr[2 * kQ] = hr;
+    rr[3 * kQ] = nh;
+    rr[4 * kQ] = lr;
+    rr[5 * kQ] = nl;
+    ri[0] = hi;
+    ri[kQ] = hr;
+    ri[2 * kQ] = hi;
+    ri[3 * kQ] = hr;
+    ri[4 * kQ] = li;
+    ri[5 * kQ] = lr;
   }
-  // the B operand of the split-TF32 product L21 = A21 A_kk^{-1} (three
-  // K-blocks of 256: hi, hi, lo; see clu_pack_kernel for the A side):
-  // row t: [Re X(:, t) | -Im X(:, t)] per block, row 128 + t: [Im X(:, t) | Re X(:, t)]
-  float* bo = binv + (size_t)b * (2 * kB) * kSplitK;
-  for (int idx = tid; idx < kB * kB; idx += blockDim.x) {
-    const int row = idx & (kB - 1), col = idx >> 7;
-    const float2 v = gj_out[col * kGjLd + row];
-    const float2 hi = make_float2(tf32_hi(v.x), tf32_hi(v.y));
-    const float2 lo = make_float2(v.x - hi.x, v.y - hi.y);
-    float* rr = bo + (size_t)col * kSplitK + row;
-    float* ri = bo + (size_t)(kB + col) * kSplitK + row;
-    rr[0] = hi.x;
-    rr[kB] = -hi.y;
-    rr[2 * kB] = hi.x;
-    rr[3 * kB] = -hi.y;
-    rr[4 * kB] = lo.x;
-    rr[5 * kB] = -lo.y;
-    ri[0] = hi.y;
-    ri[kB] = hi.x;
-    ri[2 * kB] = hi.y;
-    ri[3 * kB] = hi.x;
-    ri[4 * kB] = lo.y;
-    ri[5 * kB] = lo.x;
-  }
+  float2 v[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) v[e] = X[(size_t)(4 * lane + e) * kB + t];
+  float4* dst = reinterpret_cast<float4*>(ainv + (size_t)b * kB * 2 * kB + (size_t)t * 2 * kB) + lane;
+  dst[0] = make_float4(tf32_rn(v[0].x), tf32_rn(v[1].x), tf32_rn(v[2].x), tf32_rn(v[3].x));
+  dst[kB / 4] = make_float4(tf32_rn(v[0].y), tf32_rn(v[1].y), tf32_rn(v[2].y), tf32_rn(v[3].y));
 }
 
 // Operand packing of block step kk of the block LU (A_kk^{-1} comes packed
@@ -813,7 +885,7 @@ __global__ void refine_check_kernel(const double* __restrict__ bn, const double*
 bool g_mixed_configured = false;
 int configure_mixed() {
   if (g_mixed_configured) return BEM_OK;
-  BEM_CUDA_CHECK(cudaFuncSetAttribute(clu_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjOutBytes));
+  BEM_CUDA_CHECK(cudaFuncSetAttribute(clu_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
   BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       trsm_smem_bytes(8)));
   BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1023,9 +1095,10 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
   // block's parity).
   auto inverse = [&](int kk, cudaStream_t on) {
     TimedLaunch tl(kKCluGj, on);
-    clu_gj_kernel<<<batch, 32 * kGjWarps, kGjOutBytes, on>>>(W, kk, info_dev, w.inv, nblk, w.binv,
-                                         w.ainv + ((kk / kB) & 1) * ainv_buf, err_dev);
-    ++launches;
+    clu_gj_kernel<<<batch, 32 * kGjWarps, kGjSmem, on>>>(W, kk, info_dev, w.inv, nblk, err_dev);
+    clu_inverse_pack_kernel<<<dim3(kB / 8, batch), 256, 0, on>>>(w.inv, nblk, kk, w.binv,
+                                                                 w.ainv + ((kk / kB) & 1) * ainv_buf);
+    launches += 2;
   };
   // L21 = A21 A_kk^{-1} (split TF32: A_hi B_hi + A_lo B_hi + A_hi B_lo,
   // float32-level multipliers) into the working matrix and, packed, into the
