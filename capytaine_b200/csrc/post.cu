@@ -14,7 +14,7 @@
 //   pressure (airy_waves.py:19-53, 98-102).
 #include <cmath>
 
-#include "common.cuh"
+#include "dmma.cuh"
 
 namespace bem {
 namespace {
@@ -80,62 +80,76 @@ __global__ void build_rhs_kernel(int n, int64_t ldb, int64_t strideB, int batch,
   }
 }
 
-constexpr int kTsRows = 256;
 constexpr int kTsMaxRhs = 16;
-constexpr int kTsUnroll = 8;
 
-// Partial products of the split-K tall GEMM: one thread per row of A, the
-// CTA's column chunk of X in shared memory (row kk holds NC right-hand sides,
-// zero beyond nrhs), kTsUnroll streamed 16-byte loads of A in flight per
-// thread before their FMAs.
-template <int NC>
-__global__ void __launch_bounds__(kTsRows) zgemm_ts_partial_kernel(int M, int K, int nrhs, int kchunk,
-                                                                  const double2* __restrict__ A, int64_t lda,
-                                                                  int64_t strideA, const double2* __restrict__ X,
-                                                                  int64_t ldx, int64_t strideX,
-                                                                  double2* __restrict__ part, const int* skip,
-                                                                  const int* mskip) {
+// Partial products of the split-K tall GEMM on the double-precision tensor cores,
+// 8 or 16 columns of X.  The reads of A are the bound (16 bytes per entry); with
+// plain multiply-adds (27 TF/s, one row per thread, X from shared memory) 8
+// columns already cost as much as the reads and 16 twice as much.  A CTA owns 128
+// rows, 16 per warp; A and X stream through a five-stage cp.async ring of depth 8.
+// 15 x 6084^2, 7 columns: 1.91 -> 1.42 ms (6.25 TB/s, 0.96 of the measured copy
+// rate); 20493^2, 16 columns: 3.31 -> 1.83 ms (1.5 of MMAs).
+constexpr int kTsRows = 128, kTsDepth = 8, kTsStages = 5;
+constexpr int kTsLdA = kTsRows + 2, kTsLdX = kTsDepth + 4;
+constexpr int kTsStage = kTsDepth * kTsLdA + kTsMaxRhs * kTsLdX;
+constexpr int kTsSmem = kTsStages * kTsStage * (int)sizeof(double2);
+
+template <int NT>
+__global__ void __launch_bounds__(256, 2) zgemm_ts_partial_kernel(int M, int K, int nrhs, int kchunk,
+                                                             const double2* __restrict__ A, int64_t lda,
+                                                             int64_t strideA, const double2* __restrict__ X,
+                                                             int64_t ldx, int64_t strideX,
+                                                             double2* __restrict__ part, const int* skip,
+                                                             const int* mskip) {
   if (skip && *skip) return;
-  extern __shared__ double2 xs[];  // xs[kk * NC + c]
+  extern __shared__ double2 ring[];
   const int b = blockIdx.z;
   if (mskip && mskip[b]) return;  // matrix b is not needed (converged)
   const int split = blockIdx.y;
-  const int k0 = split * kchunk;
-  const int kc = min(K, k0 + kchunk) - k0;
-  A += (size_t)b * strideA;
-  X += (size_t)b * strideX;
-  for (int c = 0; c < NC; ++c)
-    for (int kk = threadIdx.x; kk < kc; kk += blockDim.x)
-      xs[kk * NC + c] = (c < nrhs) ? X[(size_t)(k0 + kk) + (size_t)c * ldx] : make_double2(0.0, 0.0);
-  __syncthreads();
-  const int row = blockIdx.x * kTsRows + threadIdx.x;
-  if (row >= M) return;
-  double2 acc[NC];
+  const int k0 = split * kchunk, kc = min(K, k0 + kchunk) - k0;
+  const int m0 = blockIdx.x * kTsRows;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  A += (size_t)b * strideA + (size_t)k0 * lda;
+  X += (size_t)b * strideX + k0;
+  const int nk = (kc + kTsDepth - 1) / kTsDepth;
+  auto issue = [&](int q) {
+    if (q < nk) {
+      double2* As = ring + (q % kTsStages) * kTsStage;
+      double2* Xs = As + kTsDepth * kTsLdA;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = make_double2(0.0, 0.0);
-  const double2* a = A + row + (size_t)k0 * lda;
-  for (int kk = 0; kk < kc; kk += kTsUnroll) {
-    double2 v[kTsUnroll];
-#pragma unroll
-    for (int u = 0; u < kTsUnroll; ++u)
-      v[u] = (kk + u < kc) ? __ldcs(a + (size_t)(kk + u) * lda) : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int u = 0; u < kTsUnroll; ++u) {
-      if (kk + u < kc) {
-        const double2* xr = xs + (kk + u) * NC;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const double2 x = xr[c];
-          acc[c].x = fma(v[u].x, x.x, fma(-v[u].y, x.y, acc[c].x));
-          acc[c].y = fma(v[u].x, x.y, fma(v[u].y, x.x, acc[c].y));
-        }
+      for (int i = 0; i < 4; ++i) {
+        const int idx = tid + 256 * i, m = idx & (kTsRows - 1), k = idx >> 7, kq = q * kTsDepth + k;
+        const bool ok = m0 + m < M && kq < kc;
+        cp_async16(As + k * kTsLdA + m, ok ? A + (size_t)(m0 + m) + (size_t)kq * lda : A, ok);
+      }
+      if (tid < 8 * NT * kTsDepth) {
+        const int k = tid & (kTsDepth - 1), c = tid / kTsDepth, kq = q * kTsDepth + k;
+        const bool ok = c < nrhs && kq < kc;
+        cp_async16(Xs + c * kTsLdX + k, ok ? X + (size_t)kq + (size_t)c * ldx : X, ok);
       }
     }
+    cp_async_commit();
+  };
+  double re[NT][4] = {}, im[NT][4] = {};
+#pragma unroll
+  for (int q = 0; q < kTsStages - 1; ++q) issue(q);
+#pragma unroll 1
+  for (int q = 0; q < nk; ++q) {
+    cp_async_wait<kTsStages - 2>();  // stage q has landed (this thread's part)
+    __syncthreads();                 // everybody's; and everybody is done with stage q - 1
+    issue(q + kTsStages - 1);
+    const double2* As = ring + (q % kTsStages) * kTsStage;
+    warp_zmma<NT>(As + 16 * warp, kTsLdA, As + kTsDepth * kTsLdA, kTsLdX, kTsDepth, re, im, lane);
   }
+  const int g = lane >> 2, t = lane & 3;
   double2* p = part + ((size_t)b * gridDim.y + split) * (size_t)M * nrhs;
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
-    if (c < nrhs) p[(size_t)c * M + row] = acc[c];
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int row = m0 + 16 * warp + g + 8 * (e >> 1), c = 8 * j + 2 * t + (e & 1);
+      if (row < M && c < nrhs) p[(size_t)c * M + row] = make_double2(re[j][e], im[j][e]);
+    }
 }
 
 __global__ void zgemm_ts_reduce_kernel(int M, int nrhs, int nsplit, double2 alpha, double2 beta,
@@ -257,12 +271,25 @@ extern "C" int bem_build_rhs(int n, int batch, const double* omega_dev, const do
   return BEM_OK;
 }
 
-// Splits of the K dimension: up to 24 for parallelism, more when a chunk of
-// X would not fit in shared memory (768 rows x 16 columns x 16 bytes = 192 KiB).
-static int ts_nsplit(int K) { return std::max(std::max(1, std::min(24, K / 256)), ceil_div(K, 768)); }
+// Splits of the K dimension: two waves of the two CTAs that an SM holds, in shares
+// of at least 32 columns (a 735 x 735 product in 9 CTAs took 58 us, in 132 it
+// takes 15), and up to 32 CTAs per SM (an even last wave) while the shares keep
+// 256 columns: shorter ones spend their time filling the ring (3741 in shares of
+// 47 columns 66 us, of 187 58 us), and every split writes and reads M x nrhs
+// partial sums.
+static int ts_nsplit(int M, int K, int batch) {
+  const long long rows = (long long)ceil_div(M, kTsRows) * batch;
+  const int fill = std::min(ceil_div(4 * 148, rows), K / 32), even = std::min(ceil_div(32 * 148, rows), K / 256);
+  return std::max(1, std::max(fill, even));
+}
 
 extern "C" int64_t bem_zgemm_ts_workspace_bytes(int M, int K, int nrhs, int batch) {
-  return (int64_t)batch * ts_nsplit(K) * (int64_t)M * nrhs * (int64_t)sizeof(double2);
+  // enough for calls with fewer matrices too, which may take more splits
+  int64_t most = 0;
+  for (int b = 1; b <= std::max(1, batch); ++b) {
+    most = std::max(most, (int64_t)b * ts_nsplit(M, K, b));
+  }
+  return most * (int64_t)M * nrhs * (int64_t)sizeof(double2);
 }
 
 namespace bem {
@@ -273,30 +300,21 @@ int zgemm_ts_enqueue(int M, int K, int nrhs, double alpha_re, double alpha_im, c
   if (M <= 0 || K <= 0 || nrhs <= 0 || nrhs > kTsMaxRhs || batch <= 0 || !A_dev || !X_dev || !Y_dev || !work_dev ||
       lda < M || ldx < K || ldy < M)
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_zgemm_ts: bad arguments (nrhs must be <= 16)");
-  const int nsplit = ts_nsplit(K);
-  const int kchunk = ceil_div(K, nsplit);
-  const int nc = nrhs <= 8 ? 8 : 16;
-  const size_t smem = (size_t)kchunk * nc * sizeof(double2);
-  if (smem > 200 * 1024) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_zgemm_ts: chunk too large");
+  const int nsplit = ts_nsplit(M, K, batch), kchunk = ceil_div(K, nsplit);
   cudaStream_t s = (cudaStream_t)stream;
   static bool configured = false;
   if (!configured) {
-    BEM_CUDA_CHECK(cudaFuncSetAttribute(zgemm_ts_partial_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024));
-    BEM_CUDA_CHECK(cudaFuncSetAttribute(zgemm_ts_partial_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024));
+    BEM_CUDA_CHECK(
+        cudaFuncSetAttribute(zgemm_ts_partial_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmem));
+    BEM_CUDA_CHECK(
+        cudaFuncSetAttribute(zgemm_ts_partial_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmem));
     configured = true;
   }
   TimedLaunch tl(kKZgemmTs, s);
-  const dim3 grid(ceil_div(M, kTsRows), nsplit, batch);
-  if (nc == 8)
-    zgemm_ts_partial_kernel<8><<<grid, kTsRows, smem, s>>>(M, K, nrhs, kchunk, (const double2*)A_dev, lda, strideA,
-                                                           (const double2*)X_dev, ldx, strideX, (double2*)work_dev, skip,
-                                                           mskip);
-  else
-    zgemm_ts_partial_kernel<16><<<grid, kTsRows, smem, s>>>(M, K, nrhs, kchunk, (const double2*)A_dev, lda, strideA,
-                                                            (const double2*)X_dev, ldx, strideX, (double2*)work_dev, skip,
-                                                           mskip);
+  auto* kernel = nrhs <= 8 ? zgemm_ts_partial_kernel<1> : zgemm_ts_partial_kernel<2>;
+  kernel<<<dim3(ceil_div(M, kTsRows), nsplit, batch), 256, kTsSmem, s>>>(
+      M, K, nrhs, kchunk, (const double2*)A_dev, lda, strideA, (const double2*)X_dev, ldx, strideX,
+      (double2*)work_dev, skip, mskip);
   zgemm_ts_reduce_kernel<<<dim3(ceil_div(M, 256), nrhs, batch), 256, 0, s>>>(
       M, nrhs, nsplit, make_double2(alpha_re, alpha_im), make_double2(beta_re, beta_im), (const double2*)work_dev,
       (double2*)Y_dev, ldy, strideY, skip, mskip);
