@@ -1119,18 +1119,20 @@ def _fp64_checked_solve(K_ptr, ldk, strideK, n, lu, batch, Bh, nrhs, tol=FP64_RE
     column-major, ldk, strideK apart) by bem_zlu_refine_solve.  Bh: (batch,
     nrhs, npad) complex128 device tensor, rows >= n zero.  A residual that
     stops decreasing above tol is accepted up to `accept`.  Returns X shaped
-    like Bh."""
+    like Bh and the flat buffer it views, whose last element holds the solves'
+    error flag (see _raise_on_timeout)."""
     import torch
     Kf, piv, work, npad = lu
     lib = _lib.load()
     stream = _lib.stream_ptr()
-    X = torch.zeros_like(Bh)
+    buf = torch.empty(Bh.numel() + 1, dtype=torch.complex128, device=Bh.device)
+    X, err = buf[:-1].view(Bh.shape), buf[-1:]
+    err.zero_()
     R = torch.empty_like(Bh)
-    err = torch.zeros(1, dtype=torch.int32, device=Bh.device)
     for c0 in range(0, nrhs, RHS_CHUNK):
         nc = min(RHS_CHUNK, nrhs - c0)
         ts = torch.empty(int(lib.bem_zgemm_ts_workspace_bytes(n, n, nc, batch)), dtype=torch.uint8, device=Bh.device)
-        norms = torch.zeros(2 * batch * nc + 2, dtype=torch.float64, device=Bh.device)
+        norms = torch.empty(2 * batch * nc + 2, dtype=torch.float64, device=Bh.device)
         iters, resid = ctypes.c_int32(0), ctypes.c_double(0.0)
         off = 16 * npad * c0
         status = lib.bem_zlu_refine_solve(_vp(K_ptr), ldk, strideK, n, _vp(Kf), npad, npad, npad * npad, batch,
@@ -1142,9 +1144,21 @@ def _fp64_checked_solve(K_ptr, ldk, strideK, n, lu, batch, Bh, nrhs, tol=FP64_RE
         if status == _lib.BEM_ERR_NOT_CONVERGED:
             raise _lib.NotConvergedError(status, lib.bem_last_error().decode())
         _lib.check(status)
-    if int(err.item()) != 0:
+    return X, buf
+
+
+def _raise_on_timeout(err):
+    """err: one complex128 value whose first four bytes are the solves' error flag."""
+    if err.view(np.int32)[0] != 0:
         raise _lib.BemError(_lib.BEM_ERR_TIMEOUT, "bounded wait in the triangular solve timed out")
-    return X
+
+
+def _column_major(t):
+    """The (n, K) tensor t as a (K, n) contiguous complex128 one: its own memory
+    when it is column-major already (the engine's matrices are)."""
+    import torch
+    a = t.T
+    return a.contiguous() if a.dtype == torch.complex128 else a.to(torch.complex128).contiguous()
 
 
 class DeviceMatrix:
@@ -1175,11 +1189,8 @@ class DeviceMatrix:
         X = x.reshape(x.shape[0], -1).astype(np.complex128)
         n, K = self.t.shape
         nrhs = X.shape[1]
-        # Explicit column-major buffers: element (i, c) at i + c*ld (reported strides
-        # of size-1 dimensions are not reliable leading dimensions).
-        Acm = torch.empty((K, n), dtype=torch.complex128, device=self.t.device)  # Acm[j, i] = A[i, j]
-        Acm.copy_(self.t.T)
-        Xcm = torch.as_tensor(np.ascontiguousarray(X.T), device=Acm.device)   # Xcm[c, k] = X[k, c]
+        Acm = _column_major(self.t)   # Acm[j, i] = A[i, j]: element (i, j) at i + j*n
+        Xcm = _lib.upload(X.T, torch.complex128, Acm.device)   # Xcm[c, k] = X[k, c]
         Ycm = torch.empty((nrhs, n), dtype=torch.complex128, device=Acm.device)
         lib = _lib.load()
         for c0 in range(0, nrhs, 16):
@@ -1213,10 +1224,8 @@ class DeviceMatrix:
         if int(info.item()) != 0:
             raise _lib.SingularMatrixError(_lib.BEM_ERR_SINGULAR, f"zero pivot at column {int(info.item())}")
         # the unfactored matrix, column-major complex128, for the residual checks
-        Kcm = torch.empty((n, n), dtype=torch.complex128, device=dev)  # Kcm[j, i] = K[i, j]
-        Kcm.copy_(self.t.to(torch.complex128).T)
         self._lu = (Kf, piv, work, npad)
-        self._kcm = Kcm
+        self._kcm = _column_major(self.t)  # _kcm[j, i] = K[i, j]
         return self._lu
 
     def gmres(self, b: np.ndarray, *, atol=1e-6, rtol=1e-5, restart=20, maxiter=None) -> np.ndarray:
@@ -1230,9 +1239,7 @@ class DeviceMatrix:
         n, nrhs = Bm.shape
         dev = self.t.device
         lib = _lib.load()
-        A = self.t.to(torch.complex128)
-        Acm = torch.empty((n, n), dtype=torch.complex128, device=dev)  # Acm[j, i] = A[i, j]: column-major
-        Acm.copy_(A.T)
+        Acm = _column_major(self.t)  # Acm[j, i] = A[i, j]
         maxc = int(maxiter) if maxiter is not None else 10 * n
         out = np.empty_like(Bm)
         for c0 in range(0, nrhs, 16):
@@ -1262,11 +1269,13 @@ class DeviceMatrix:
         vec = b.ndim == 1
         Bm = b.reshape(b.shape[0], -1).astype(np.complex128)
         n, nrhs = Bm.shape
-        dev = Kf.device
-        Bd = torch.zeros((1, nrhs, npad), dtype=torch.complex128, device=dev)  # column-major npad x nrhs
-        Bd[0, :, :n] = torch.as_tensor(Bm.T.copy(), device=dev)
-        X = _fp64_checked_solve(self._kcm, n, 0, n, (Kf, piv, work, npad), 1, Bd, nrhs)
-        out = X[0, :, :n].T.cpu().numpy()
+        Bh = np.zeros((1, nrhs, npad), dtype=np.complex128)  # column-major npad x nrhs
+        Bh[0, :, :n] = Bm.T
+        Bd = _lib.upload(Bh, torch.complex128, Kf.device)
+        _, buf = _fp64_checked_solve(self._kcm, n, 0, n, (Kf, piv, work, npad), 1, Bd, nrhs)
+        host = buf.cpu().numpy()  # the solution and, behind it, the error flag: one copy
+        _raise_on_timeout(host[-1:])
+        out = host[:-1].reshape(nrhs, npad)[:, :n].T
         x = out[:, 0] if vec else out.reshape(b.shape)
         return x.astype(np.complex64) if self.t.dtype == torch.complex64 else x
 
@@ -1414,8 +1423,9 @@ class DeviceBlockCirculantMatrix:
         Xd, vec, shape = self._columns(b)
         nrhs = Xd.shape[0]
         Bh = self._to_systems(Xd, npad)
-        X = _fp64_checked_solve(self.systems, st.n_sys, st.n_sys * st.n_sys, st.n_sys, (Kf, piv, work, npad),
-                                st.nsys, Bh, nrhs)
+        X, buf = _fp64_checked_solve(self.systems, st.n_sys, st.n_sys * st.n_sys, st.n_sys, (Kf, piv, work, npad),
+                                     st.nsys, Bh, nrhs)
+        _raise_on_timeout(buf[-1:].cpu().numpy())
         return self._out(self._from_systems(X, npad), vec, shape)
 
     def gmres(self, b, **kw):
