@@ -111,15 +111,26 @@ int clu_planes(void* work_dev, int npad, float** re, int64_t* ld, int64_t* strid
 //   kPackRows: row i -> [Re C(i, 0..127) | Im C(i, 0..127)]  (n = 128)
 enum PackMode { kPackNone = 0, kPackRows = 1 };
 
+// Depth of a complex update: nseg segments of k values.  Row i of the A operand
+// (ka floats) has segment s's real parts at s a_seg and its imaginary parts a_im
+// further; the rows of the B operand (kb floats; 128 rows of real parts, then 128
+// of imaginary parts, per 128 columns) have segment s at b_seg[s].  embedded: no
+// parts, k values of an A row against all 256 rows of B.
+struct CgemmDepth {
+  int k, ka, kb, nseg, a_im, a_seg;
+  int b_seg[3];
+  bool embedded;
+};
+
 // C (m x n complex in two float32 planes) -= A' B' (store = 0) or = A' B'
 // (store = 1) on the tensor cores from packed operands; an optional second
-// operand pair adds K' depth in the same pass over C; limit_host: per-matrix
+// operand pair adds a second segment in the same pass over C; limit_host: per-matrix
 // active sizes (grouped launches); pack: a packed copy of the result; lshape:
 // only the first tile row and column of the square block, corner excluded;
 // reserve_sms: SMs that a kernel beside this one holds (left out of the
 // launch's width).
 int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float* Bop, int64_t b_rows, int b_row0,
-                      int kp, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
+                      const CgemmDepth& depth, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
                       int n, int batch, int* err, cudaStream_t stream, int store = 0, const float* Aop1 = nullptr,
                       const float* Bop1 = nullptr, int run = 0, long long wait_limit = 0,
                       const int* limit_host = nullptr, float* pack = nullptr, int pack_mode = kPackNone,

@@ -33,7 +33,12 @@ namespace {
 
 constexpr int kB = 128;        // LU block
 constexpr int kPT = 64;        // panel tile width
-constexpr int kSplitK = 6 * kB;  // K' of the split-TF32 panel product: (hi, lo, hi) x (re, im) x 128
+constexpr int kSplitK = 6 * kB;  // A row of the split-TF32 panel product: (hi, lo, hi) x (re, im) x 128
+constexpr int kSplitB = 2 * kB;  // its B row: (hi, lo) x 128
+// depths of the update (A row [Re | Im], B row of one part) and of the panel
+// product (A_hi B_hi + A_lo B_hi + A_hi B_lo)
+constexpr CgemmDepth kUpdateDepth{kB, 2 * kB, kB, 1, kB, 0, {0, 0, 0}, false};
+constexpr CgemmDepth kSplitDepth{kB, kSplitK, kSplitB, 3, kB, 2 * kB, {0, 0, kB}, false};
 constexpr int kRhs = 16;       // right-hand sides per solve launch
 constexpr int kOpBuffers = 3;  // packed operands of the current, previous and next block steps
 
@@ -444,10 +449,10 @@ __global__ void __launch_bounds__(32 * kGjWarps, 1) clu_gj_kernel(Planes W, int 
 }
 
 // The inverse of block kk as the operands of two products, 8 columns and 8 rows
-// per CTA: the inverse's own CTA took 20 us for these 0.9 MB.
-// binv: B operand of the split-TF32 product L21 = A21 A_kk^{-1} (three K-blocks
-// of 256: hi, hi, lo; see clu_pack_kernel for the A side): row t
-// [Re X(:, t) | -Im X(:, t)] per block, row 128 + t [Im X(:, t) | Re X(:, t)].
+// per CTA: the inverse's own CTA took 20 us to write them.
+// binv: B operand of the split-TF32 product L21 = A21 A_kk^{-1} (see
+// clu_pack_kernel for the A side): row t [hi Re X(:, t) | lo Re X(:, t)], row 128 + t
+// the imaginary parts.
 // ainv: A operand of U' = A_kk^{-1} A12, row r [Re A_kk^{-1}(r, :) | Im A_kk^{-1}(r, :)].
 __global__ void __launch_bounds__(256) clu_inverse_pack_kernel(const float2* __restrict__ inv, int nblk, int kk,
                                                               float* __restrict__ binv, float* __restrict__ ainv) {
@@ -459,25 +464,13 @@ __global__ void __launch_bounds__(256) clu_inverse_pack_kernel(const float2* __r
     const float4 re = make_float4(v0.x, v0.z, v1.x, v1.z), im = make_float4(v0.y, v0.w, v1.y, v1.w);
     const float4 hr = make_float4(tf32_hi(re.x), tf32_hi(re.y), tf32_hi(re.z), tf32_hi(re.w));
     const float4 hi = make_float4(tf32_hi(im.x), tf32_hi(im.y), tf32_hi(im.z), tf32_hi(im.w));
-    const float4 lr = make_float4(re.x - hr.x, re.y - hr.y, re.z - hr.z, re.w - hr.w);
-    const float4 li = make_float4(im.x - hi.x, im.y - hi.y, im.z - hi.z, im.w - hi.w);
-    const float4 nh = make_float4(-hi.x, -hi.y, -hi.z, -hi.w), nl = make_float4(-li.x, -li.y, -li.z, -li.w);
-    float* bo = binv + (size_t)b * (2 * kB) * kSplitK;
-    float4* rr = reinterpret_cast<float4*>(bo + (size_t)t * kSplitK) + lane;
-    float4* ri = reinterpret_cast<float4*>(bo + (size_t)(kB + t) * kSplitK) + lane;
-    constexpr int kQ = kB / 4;
+    float* bo = binv + (size_t)b * (2 * kB) * kSplitB;
+    float4* rr = reinterpret_cast<float4*>(bo + (size_t)t * kSplitB) + lane;
+    float4* ri = reinterpret_cast<float4*>(bo + (size_t)(kB + t) * kSplitB) + lane;
     rr[0] = hr;
-    rr[kQ] = nh;
-    rr[2 * kQ] = hr;
-    rr[3 * kQ] = nh;
-    rr[4 * kQ] = lr;
-    rr[5 * kQ] = nl;
+    rr[kB / 4] = make_float4(re.x - hr.x, re.y - hr.y, re.z - hr.z, re.w - hr.w);
     ri[0] = hi;
-    ri[kQ] = hr;
-    ri[2 * kQ] = hi;
-    ri[3 * kQ] = hr;
-    ri[4 * kQ] = li;
-    ri[5 * kQ] = lr;
+    ri[kB / 4] = make_float4(im.x - hi.x, im.y - hi.y, im.z - hi.z, im.w - hi.w);
   }
   float2 v[4];
 #pragma unroll
@@ -494,19 +487,18 @@ __global__ void __launch_bounds__(256) clu_inverse_pack_kernel(const float2* __r
 // nrows/32): 32 rows of the block column [col0, col0 + 128) from row row0 on,
 // packed K-major into A3 as the split-TF32 operand of the panel product (A21).
 // Both through shared memory, so that reads and writes are coalesced.
-// Bop: [batch][2*npad][2*kB]; A3: [batch][npad][kSplitK].
+// Bop: [batch][2*npad][kB]; A3: [batch][npad][kSplitK].
 __global__ void __launch_bounds__(256) clu_pack_kernel(Planes W, int npad, int kk, int nrest, int row0, int col0,
                                                        float* __restrict__ Bop, float* __restrict__ A3, int t0) {
   __shared__ float tre[kB][33], tim[kB][33];  // [column][row] of a 32 x 128 tile
   const int b = blockIdx.y, tid = threadIdx.x;
-  const size_t kp = 2 * kB;
   const int t = blockIdx.x + t0;  // a launch may cover a range of the blocks only
   if (t < nrest) {
     // 128 x 64 of A12: B operand rows of the complex columns c0 .. c0+63;
     // thread (q, cc): rows 4 q .. 4 q + 3 of column cc (16-byte loads and stores)
     const int c0 = kk + kB + t * kPT;
     const int j0 = c0 & ~(kB - 1);
-    float* Bb = Bop + (size_t)b * 2 * npad * kp;
+    float* Bb = Bop + (size_t)b * 2 * npad * kB;
     const float* re = W.re + (size_t)b * W.stride;
     const float* im = W.im + (size_t)b * W.stride;
     const int q = tid & 31;
@@ -517,12 +509,8 @@ __global__ void __launch_bounds__(256) clu_pack_kernel(Planes W, int npad, int k
       ur = make_float4(tf32_rn(ur.x), tf32_rn(ur.y), tf32_rn(ur.z), tf32_rn(ur.w));  // TF32 operands
       ui = make_float4(tf32_rn(ui.x), tf32_rn(ui.y), tf32_rn(ui.z), tf32_rn(ui.w));
       const int jj = c0 - j0 + c;
-      float4* rowR = reinterpret_cast<float4*>(Bb + (size_t)(2 * j0 + jj) * kp);
-      float4* rowI = reinterpret_cast<float4*>(Bb + (size_t)(2 * j0 + kB + jj) * kp);
-      rowR[q] = ur;
-      rowR[kB / 4 + q] = make_float4(-ui.x, -ui.y, -ui.z, -ui.w);
-      rowI[q] = ui;
-      rowI[kB / 4 + q] = ur;
+      reinterpret_cast<float4*>(Bb + (size_t)(2 * j0 + jj) * kB)[q] = ur;
+      reinterpret_cast<float4*>(Bb + (size_t)(2 * j0 + kB + jj) * kB)[q] = ui;
     }
     return;
   }
@@ -914,7 +902,7 @@ struct MixedWork {
   float* Aop;
   float* Bop;
   float2* inv;
-  float* binv;  // batch x 256 x kSplitK: packed A_kk^{-1} of the current block
+  float* binv;  // batch x 256 x kSplitB: packed A_kk^{-1} of the current block
   float* a3;    // batch x npad x kSplitK: split A21 of the current block
   float* ainv;  // 2 x batch x 128 x 256: A_kk^{-1} of the last two blocks as the A operand [Re | Im]
   int* flags;
@@ -927,12 +915,12 @@ MixedWork carve(void* work, int npad, int batch) {
   p += (size_t)batch * 2 * npad * npad * sizeof(float);
   w.Aop = (float*)p;  // three buffers of batch x npad x 256
   p += kOpBuffers * (size_t)batch * npad * 2 * kB * sizeof(float);
-  w.Bop = (float*)p;  // three buffers of batch x 2 npad x 256
-  p += kOpBuffers * (size_t)batch * 2 * npad * 2 * kB * sizeof(float);
+  w.Bop = (float*)p;  // three buffers of batch x 2 npad x 128
+  p += kOpBuffers * (size_t)batch * 2 * npad * kB * sizeof(float);
   w.inv = (float2*)p;
   p += (size_t)batch * nblk * kB * kB * sizeof(float2);
   w.binv = (float*)p;
-  p += (size_t)batch * (2 * kB) * kSplitK * sizeof(float);
+  p += (size_t)batch * (2 * kB) * kSplitB * sizeof(float);
   w.a3 = (float*)p;
   p += (size_t)batch * npad * kSplitK * sizeof(float);
   w.ainv = (float*)p;
@@ -995,8 +983,8 @@ extern "C" int64_t bem_clu_workspace_bytes(int npad, int batch) {
   if (npad <= 0 || npad % kB || batch <= 0) return -1;
   const int64_t nblk = npad / kB;
   return (int64_t)batch * 2 * npad * (int64_t)npad * 4 + kOpBuffers * (int64_t)batch * npad * 2 * kB * 4 +
-         kOpBuffers * (int64_t)batch * 2 * npad * 2 * kB * 4 + (int64_t)batch * nblk * kB * kB * 8 +
-         (int64_t)batch * (2 * kB) * kSplitK * 4 + (int64_t)batch * npad * kSplitK * 4 +
+         kOpBuffers * (int64_t)batch * 2 * npad * kB * 4 + (int64_t)batch * nblk * kB * kB * 8 +
+         (int64_t)batch * (2 * kB) * kSplitB * 4 + (int64_t)batch * npad * kSplitK * 4 +
          2 * (int64_t)batch * kB * 2 * kB * 4 +
          ((int64_t)batch * nblk + 2 + batch) * 4 + 1024;
 }
@@ -1080,7 +1068,7 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
                                                                              n, npad, W);
   }
   ++launches;
-  const size_t abuf = (size_t)batch * npad * 2 * kB, bbuf = (size_t)batch * 2 * npad * 2 * kB;
+  const size_t abuf = (size_t)batch * npad * 2 * kB, bbuf = (size_t)batch * 2 * npad * kB;
   // The updates and the panel product give each CTA an even share of up to
   // 32 tiles (the accumulator double buffer pays over a run; the runs end at
   // staggered times, so an SM frees up every few microseconds); U' (low
@@ -1107,7 +1095,7 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
     const int m = npad - kk - kB;
     if (m <= 0) return BEM_OK;
     TimedLaunch tl(kKCluPanel, on);
-    return cgemm_tf32_update(w.a3, npad, kk + kB, w.binv, 2 * kB, 0, kSplitK, W.re, W.im, npad, W.stride, kk + kB,
+    return cgemm_tf32_update(w.a3, npad, kk + kB, w.binv, 2 * kB, 0, kSplitDepth, W.re, W.im, npad, W.stride, kk + kB,
                              kk, m, kB, batch, err_dev, on, 1, nullptr, nullptr, kBigRun, 0, act, Aop[buf],
                              kPackRows, a_stride);
   };
@@ -1118,7 +1106,7 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
     if (m <= 0) return BEM_OK;
     TimedLaunch tl(kKCluPanel, on);
     return cgemm_tf32_update(w.ainv + ((kk / kB) & 1) * ainv_buf, kB, 0, Bop[buf], 2 * (int64_t)npad,
-                             2 * (kk + kB), 2 * kB, W.re, W.im, npad, W.stride, kk, kk + kB, kB, m, batch, err_dev,
+                             2 * (kk + kB), kUpdateDepth, W.re, W.im, npad, W.stride, kk, kk + kB, kB, m, batch, err_dev,
                              on, 1, nullptr, nullptr, kSideRun, 0, act);
   };
   // C rows r0.. (m), complex columns c0.. (nc) -= L21 U12 of the block step whose
@@ -1127,7 +1115,7 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
   auto update = [&](int buf, int r0, int c0, int m, int nc, int buf2, int run, bool lshape = false,
                     int reserve = 0) -> int {
     if (m <= 0 || nc <= 0) return BEM_OK;
-    return cgemm_tf32_update(Aop[buf], npad, r0, Bop[buf], 2 * (int64_t)npad, 2 * c0, 2 * kB, W.re, W.im, npad,
+    return cgemm_tf32_update(Aop[buf], npad, r0, Bop[buf], 2 * (int64_t)npad, 2 * c0, kUpdateDepth, W.re, W.im, npad,
                              W.stride, r0, c0, m, nc, batch, err_dev, s, 0, buf2 >= 0 ? Aop[buf2] : nullptr,
                              buf2 >= 0 ? Bop[buf2] : nullptr, run, 0, act, nullptr, kPackNone, 0, lshape, reserve);
   };

@@ -2,25 +2,30 @@
 // inputs, FP32 accumulation in tensor memory).
 //
 // The mixed-precision LU keeps its working matrix as two float32 planes (real,
-// imaginary), column-major.  A complex update C -= A B is one real GEMM in the
-// "4M" embedding
-//     [Cr | Ci] -= [Ar | Ai] * [[Br, Bi], [-Bi, Br]]
-// with K' = 2k.  The LU panel kernels write the two operands already packed,
-// K-major (K' contiguous per row / per output column):
-//   Aop[b][row][K']   row i: [Re A(i, 0..k), Im A(i, 0..k)]
-//   Bop[b][r][K']     per group of 128 complex output columns j0..j0+127, rows
-//                     2*j0 + t   (t < 128): [ Re B(:, j0+t); -Im B(:, j0+t)]
-//                     2*j0 + 128 + t     : [ Im B(:, j0+t);  Re B(:, j0+t)]
-// A CTA owns a 128 x 128 complex tile of C (accumulator 128 lanes x 256 fp32
-// columns: real parts then imaginary parts).  Warp 0 streams operand slices
-// with TMA (128-byte swizzle) through a 2-stage shared-memory ring (two CTAs
-// per SM, so that one CTA's epilogue overlaps the other's MMAs), one thread
-// of warp 1 issues tcgen05.mma (M=128, N=256, K=8 per instruction), warps 2-9
-// read the accumulator back with tcgen05.ld and apply C -= acc in place, the
-// loads of C running ahead of the accumulator reads: two warps per 32-lane
-// quarter of the accumulator, one for the real plane and one for the imaginary
-// plane, so that twice as many loads of C are in flight (the update is bound
-// by the read and write of C).
+// imaginary), column-major.  A complex update C -= A B is four real products
+//     Cr -= Ar Br - Ai Bi,   Ci -= Ar Bi + Ai Br
+// from operands packed K-major (rows of real parts, rows of imaginary parts):
+//   Aop[b][row][:]    row i: Re A(i, 0..k) at one place, Im A(i, 0..k) at another
+//   Bop[b][r][:]      per group of 128 complex output columns j0..j0+127, rows
+//                     2*j0 + t   (t < 128): Re B(:, j0+t)
+//                     2*j0 + 128 + t     : Im B(:, j0+t)
+// (the public entry point's B operand is the real embedding, whose rows begin with
+// these parts; see CgemmDepth).
+// A CTA owns 128 x 128 complex tiles of C (accumulator 128 lanes x 256 fp32
+// columns: real parts then imaginary parts).  Warp 0 streams operand slices with
+// TMA (128-byte swizzle) through a three-stage shared-memory ring, 32 values of
+// depth per stage of both parts of A (32 KB) and of B (32 KB); one thread of warp
+// 1 issues, per 8 of depth, one tcgen05.mma of N = 256 (Re A against [Re B; Im B])
+// and two of N = 128 (Im A against Im B, negated, and against Re B).  Every
+// operand byte crosses from L2 once per tile: with the real embedding [[Br, Bi],
+// [-Bi, Br]] stored as such, each part of B came twice, 786 KB per tile of depth
+// 256 against 524, and had to be packed twice.
+// Bound: shared-memory bandwidth.  Per 8 of depth the MMAs read 28 KB in what would
+// be 262 clocks and TMA writes 16 KB, 169 bytes per clock of the 128 there are
+// (with the embedding 184).  15 x 5888^2, depth 256: 469 -> 505 TF/s, 0.69 of cuBLAS
+// on plain TF32 matrices; a pair of SMs sharing B (cta_group::2) would read less.
+// Sixteen warps read the accumulator back with tcgen05.ld and apply C -= acc in
+// place, the loads of C running ahead of the accumulator reads.
 // Every mbarrier wait is bounded; on timeout the kernel records an error and
 // still drains its own copies before freeing tensor memory.
 #include <cuda.h>
@@ -34,11 +39,11 @@ namespace {
 constexpr int kTM = 128;            // tile rows
 constexpr int kTNc = 128;           // tile complex columns
 constexpr int kTN = 2 * kTNc;       // accumulator columns (MMA N)
-constexpr int kKC = 32;             // K' values per stage (128 bytes of fp32)
-constexpr int kStages = 4;
-constexpr int kABytes = kTM * kKC * 4;   // 16 KiB
-constexpr int kBBytes = kTN * kKC * 4;   // 32 KiB
-constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kKC = 32;             // values of depth per stage (128 bytes of fp32)
+constexpr int kStages = 3;
+constexpr int kABytes = kTM * kKC * 4;   // 16 KiB: one part of A
+constexpr int kBBytes = kTN * kKC * 4;   // 32 KiB: both parts of B
+constexpr int kStageBytes = 2 * kABytes + kBBytes;
 constexpr long long kWaitLimit = 1ll << 22;  // default polls of a bounded mbarrier wait (~ a second)
 constexpr int kMaxGroup = 64;  // matrices of one grouped launch
 
@@ -83,15 +88,21 @@ __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t saddr) {
   return d;
 }
 
-// Instruction descriptor: D f32, A/B tf32, both K-major, M = 128, N = 256.
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kTN >> 3) << 17) |
-                            ((uint32_t)(kTM >> 4) << 24);
+// Instruction descriptor: D f32, A/B tf32, both K-major, M = 128; bit 13 negates A.
+constexpr uint32_t idesc_tf32(int n, bool negate_a) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((negate_a ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(kTM >> 4) << 24);
+}
+constexpr uint32_t kIdescBoth = idesc_tf32(kTN, false);
+constexpr uint32_t kIdescHalf = idesc_tf32(kTNc, false);
+constexpr uint32_t kIdescHalfNeg = idesc_tf32(kTNc, true);
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -136,8 +147,13 @@ struct UpdateArgs {
   int b_row0;        // first operand row of the trailing block (Bop), = 2 * first complex column
   int c_row0;        // first row of the trailing block in C
   int c_col0;        // first complex column of the trailing block in C
-  int nk;            // K' / kKC
-  int nk0;           // chunks read from the first operand pair; the rest from the second
+  int nk;            // stages per tile: nseg x nchunk
+  int nchunk;        // stages per segment
+  int embedded;      // 1: no structure, A's one part against B's 256 rows
+  int a_im;          // of a segment's imaginary parts in an A row
+  int a_seg;         // between segments in an A row
+  int b_seg[3];      // of each segment in a B row
+  int second;        // 1: segment 1 reads the second operand pair (from its start)
   float* Cr;
   float* Ci;
   int64_t ldc;
@@ -254,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) cgemm_tf32_update_kernel(const __
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   unsigned char* ringA = smem;
-  unsigned char* ringB = smem + kStages * kABytes;
+  unsigned char* ringB = smem + 2 * kStages * kABytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;  // [2]
@@ -312,12 +328,15 @@ __global__ void __launch_bounds__(kThreads, 1) cgemm_tf32_update_kernel(const __
           const int s = (int)(g % kStages);
           const uint32_t use = (uint32_t)(g / kStages);
           if (g >= kStages && !(ok = mbar_wait_n(&empty[s], (use - 1) & 1, p.err, limit))) break;
-          mbar_expect_tx(&full[s], kStageBytes);
-          // K' chunks [0, nk0) from the first operand pair, the rest from the second
-          const bool first = kc < p.nk0;
-          const int kx = (first ? kc : kc - p.nk0) * kKC;
-          tma_load_3d(ringA + s * kABytes, first ? &mapA : &mapA1, kx, p.a_row0 + tm * kTM, b, &full[s]);
-          tma_load_3d(ringB + s * kBBytes, first ? &mapB : &mapB1, kx, p.b_row0 + tn * kTN, b, &full[s]);
+          mbar_expect_tx(&full[s], p.embedded ? kABytes + kBBytes : kStageBytes);
+          const int seg = kc / p.nchunk, kx = (kc - seg * p.nchunk) * kKC;
+          const bool other = p.second && seg == 1;
+          const CUtensorMap* ma = other ? &mapA1 : &mapA;
+          const int ax = kx + (other ? 0 : seg * p.a_seg), bx = kx + (other ? 0 : p.b_seg[seg]);
+          unsigned char* sa = ringA + s * 2 * kABytes;
+          tma_load_3d(sa, ma, ax, p.a_row0 + tm * kTM, b, &full[s]);
+          if (!p.embedded) tma_load_3d(sa + kABytes, ma, ax + p.a_im, p.a_row0 + tm * kTM, b, &full[s]);
+          tma_load_3d(ringB + s * kBBytes, other ? &mapB1 : &mapB, bx, p.b_row0 + tn * kTN, b, &full[s]);
         }
       }
       // drain: every issued copy must land before the CTA may exit
@@ -341,11 +360,18 @@ __global__ void __launch_bounds__(kThreads, 1) cgemm_tf32_update_kernel(const __
           const int s = (int)(g % kStages);
           if (!(ok = mbar_wait_n(&full[s], (uint32_t)(g / kStages) & 1, p.err, limit))) break;
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const uint32_t a0 = smem_u32(ringA + s * kABytes), b0 = smem_u32(ringB + s * kBBytes);
+          const uint32_t a0 = smem_u32(ringA + s * 2 * kABytes), b0 = smem_u32(ringB + s * kBBytes);
 #pragma unroll
           for (int kk = 0; kk < kKC / 8; ++kk) {
             // K = 8 tf32 = 32 bytes per instruction inside the 128-byte swizzle atom
-            mma_tf32(tacc, smem_desc_k_sw128(a0 + kk * 32), smem_desc_k_sw128(b0 + kk * 32), (kc | kk) != 0);
+            const uint64_t br = smem_desc_k_sw128(b0 + kk * 32);
+            mma_tf32(tacc, smem_desc_k_sw128(a0 + kk * 32), br, kIdescBoth, (kc | kk) != 0);
+            if (!p.embedded) {
+              const uint64_t ai = smem_desc_k_sw128(a0 + kABytes + kk * 32);
+              const uint64_t bi = smem_desc_k_sw128(b0 + kBBytes / 2 + kk * 32);
+              mma_tf32(tacc, ai, bi, kIdescHalfNeg, 1);
+              mma_tf32(tacc + kTNc, ai, br, kIdescHalf, 1);
+            }
           }
           mma_commit(&empty[s]);
         }
@@ -485,7 +511,7 @@ int num_sms(int* out) {
 // of 128) -= A' B' for `batch` matrices.  run > 0: tiles per CTA; 0: chosen
 // from the tile count (up to 32 while there are at least two runs per SM).
 int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float* Bop, int64_t b_rows, int b_row0,
-                      int kp, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
+                      const CgemmDepth& depth, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
                       int n, int batch, int* err, cudaStream_t stream, int store, const float* Aop1,
                       const float* Bop1, int run, long long wait_limit, const int* limit_host, float* pack,
                       int pack_mode, int64_t pack_stride, bool lshape, int reserve_sms) {
@@ -497,19 +523,20 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
       (pack_mode != kPackRows || !pack || n != kTNc || (reinterpret_cast<uintptr_t>(pack) & 15)))
     return set_error(BEM_ERR_INVALID_ARGUMENT,
                      "cgemm_tf32_update: a packed copy needs one tile column and a 16-byte aligned destination");
-  if (m % kTM || n % kTNc || kp % kKC || (a_row0 % 8) || (b_row0 % 8))
+  if (m % kTM || n % kTNc || depth.k <= 0 || depth.k % kKC || depth.ka % kKC || depth.kb % kKC || (a_row0 % 8) ||
+      (b_row0 % 8))
     return set_error(BEM_ERR_INVALID_ARGUMENT, "cgemm_tf32_update: sizes must be multiples of 128 (K' of 32)");
   if ((Aop1 == nullptr) != (Bop1 == nullptr))
     return set_error(BEM_ERR_INVALID_ARGUMENT, "cgemm_tf32_update: second operand pair incomplete");
   CUtensorMap mapA, mapB, mapA1, mapB1;
-  int st = make_operand_map(&mapA, Aop, kp, a_rows, batch, kTM);
+  int st = make_operand_map(&mapA, Aop, depth.ka, a_rows, batch, kTM);
   if (st) return st;
-  st = make_operand_map(&mapB, Bop, kp, b_rows, batch, kTN);
+  st = make_operand_map(&mapB, Bop, depth.kb, b_rows, batch, kTN);
   if (st) return st;
-  // second pair (same shapes, the next K' block): C -= A B - A1 B1 in one pass over C
-  st = make_operand_map(&mapA1, Aop1 ? Aop1 : Aop, kp, a_rows, batch, kTM);
+  // second pair (same shapes, one segment each): C -= A B + A1 B1 in one pass over C
+  st = make_operand_map(&mapA1, Aop1 ? Aop1 : Aop, depth.ka, a_rows, batch, kTM);
   if (st) return st;
-  st = make_operand_map(&mapB1, Bop1 ? Bop1 : Bop, kp, b_rows, batch, kTN);
+  st = make_operand_map(&mapB1, Bop1 ? Bop1 : Bop, depth.kb, b_rows, batch, kTN);
   if (st) return st;
   const int smem = kStages * kStageBytes + 1024 + 256;
   if (!g_tc_configured) {
@@ -518,15 +545,20 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
   }
   int sms = 0;
   if ((st = num_sms(&sms))) return st;
-  const int nk0 = kp / kKC;
+  const int nseg = Aop1 ? 2 : depth.nseg;
   const int tiles_m = m / kTM, tiles_n = n / kTNc;
   UpdateArgs p{};
   p.a_row0 = a_row0;
   p.b_row0 = b_row0;
   p.c_row0 = c_row0;
   p.c_col0 = c_col0;
-  p.nk = Aop1 ? 2 * nk0 : nk0;
-  p.nk0 = nk0;
+  p.nchunk = depth.k / kKC;
+  p.nk = nseg * p.nchunk;
+  p.embedded = depth.embedded ? 1 : 0;
+  p.a_im = depth.a_im;
+  p.a_seg = depth.a_seg;
+  for (int i = 0; i < 3; ++i) p.b_seg[i] = depth.b_seg[i];
+  p.second = Aop1 ? 1 : 0;
   p.Cr = Cr;
   p.Ci = Ci;
   p.ldc = ldc;
@@ -607,7 +639,11 @@ extern "C" int bem_cgemm_tf32_update(const float* Aop_dev, int64_t a_rows, int a
     return bem::set_error(BEM_ERR_INVALID_ARGUMENT, "bem_cgemm_tf32_update: operand rows out of range");
   if ((reinterpret_cast<uintptr_t>(Aop_dev) | reinterpret_cast<uintptr_t>(Bop_dev)) & 15)
     return bem::set_error(BEM_ERR_INVALID_ARGUMENT, "bem_cgemm_tf32_update: operands must be 16-byte aligned");
-  return bem::cgemm_tf32_update(Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, kp, Cr_dev, Ci_dev, ldc, c_stride,
+  // K' = 2k: the rows of B begin with Re B and Im B; an odd number of 16-deep
+  // steps (K' not a multiple of 64) takes the embedding as it stands
+  const bem::CgemmDepth depth = kp % 64 == 0 ? bem::CgemmDepth{kp / 2, kp, kp, 1, kp / 2, 0, {0, 0, 0}, false}
+                                             : bem::CgemmDepth{kp, kp, kp, 1, 0, 0, {0, 0, 0}, true};
+  return bem::cgemm_tf32_update(Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, depth, Cr_dev, Ci_dev, ldc, c_stride,
                                 c_row0, c_col0, m, n, batch, err_dev, (cudaStream_t)stream, 0, nullptr, nullptr, 0, 0,
                                 nullptr, nullptr, bem::kPackNone, 0, false, 0);
 }
