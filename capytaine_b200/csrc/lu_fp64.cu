@@ -500,6 +500,7 @@ __global__ void __launch_bounds__(256, 2) zlu_panel_kernel(double2* __restrict__
 // where these are long, and costs no launch.  Those CTAs come first in the
 // grid.
 constexpr int kTile = 64, kDepth = 16, kStages = 3;
+constexpr int kResident = 2 * 148;  // CTAs that the GPU holds at a time
 constexpr int kLdTA = kTile + 2, kLdTB = kDepth + 4;
 constexpr int kStageElems = kDepth * kLdTA + kTile * kLdTB;
 constexpr int kGemmSmem = kStages * kStageElems * (int)sizeof(double2);
@@ -563,6 +564,19 @@ __global__ void __launch_bounds__(256, 2)
         re[j][e] = -c.x;
         im[j][e] = -c.y;
       }
+    // meanwhile the tile of the CTA that follows in this place comes into L2: its loads
+    // are the only ones that otherwise wait for DRAM (2688 x 4: 9.66 -> 9.28 ms)
+    const int next = (int)blockIdx.x + kResident;
+    if (next >= batch && next < tiles * batch) {  // the first `batch` CTAs take the first tiles
+      const int tn = 1 + (next - batch) % (tiles - 1), bn = (next - batch) / (tiles - 1);
+      const double2* Cn = C + (int64_t)(bn - b) * strideC + (tn % tiles_m) * kTile +
+                          (int64_t)(tn / tiles_m) * kTile * ldc;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int line = tid + 256 * i;  // 8 lines of 128 bytes per column
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(Cn + 8 * (line & 7) + (int64_t)(line >> 3) * ldc));
+      }
+    }
   }
 #pragma unroll 1
   for (int q = 0; q < nk; ++q) {
