@@ -122,11 +122,15 @@ struct CgemmDepth {
   bool embedded;
 };
 
+// Tiles of a block that a product covers: all, all but the first, or the first
+// row and column of a square block without their common tile.
+enum TileRegion { kTilesAll = 0, kTilesL = 1, kTilesNoCorner = 2 };
+
 // C (m x n complex in two float32 planes) -= A' B' (store = 0) or = A' B'
 // (store = 1) on the tensor cores from packed operands; an optional second
 // operand pair adds a second segment in the same pass over C; limit_host: per-matrix
-// active sizes (grouped launches); pack: a packed copy of the result; lshape:
-// only the first tile row and column of the square block, corner excluded;
+// active sizes (grouped launches); pack: a packed copy of the result; region:
+// which tiles of the block;
 // reserve_sms: SMs that a kernel beside this one holds (left out of the
 // launch's width).
 int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float* Bop, int64_t b_rows, int b_row0,
@@ -134,7 +138,7 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
                       int n, int batch, int* err, cudaStream_t stream, int store = 0, const float* Aop1 = nullptr,
                       const float* Bop1 = nullptr, int run = 0, long long wait_limit = 0,
                       const int* limit_host = nullptr, float* pack = nullptr, int pack_mode = kPackNone,
-                      int64_t pack_stride = 0, bool lshape = false, int reserve_sms = 0);
+                      int64_t pack_stride = 0, TileRegion region = kTilesAll, int reserve_sms = 0);
 
 }  // namespace bem
 

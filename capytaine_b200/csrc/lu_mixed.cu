@@ -556,6 +556,94 @@ __global__ void __launch_bounds__(256) clu_pack_kernel(Planes W, int npad, int k
   }
 }
 
+// The next diagonal block's update by block step kk in one launch of its own,
+// D -= A21 (A_kk^{-1} A12) in float32 from the unpacked blocks, as soon as the
+// inverse is there: the chain of diagonal blocks need not wait for the packed
+// inverse, the panel product over the whole block column (one 128 x 128 tile
+// takes it 19 us whatever the column's height) and a tensor-core tile, which
+// follow beside the next inverse.
+// A CTA takes 4 columns: first A_kk^{-1} times theirs of A12, then A21 times
+// that; a thread two rows of all four over a quarter of the depth (the quarters
+// meet in shared memory).  Bound: the two 128 x 128 factors that every CTA
+// reads from L2 (256 KB), 9.5 us in place of 34 between two inverses (packing
+// 2.4, panel 19.4, tile 10-13 and their launches): one 3840 3.74 -> 2.97 ms.
+constexpr int kNextCols = 4;
+__global__ void __launch_bounds__(256) clu_next_diagonal_kernel(Planes W, int kk, const float2* __restrict__ inv,
+                                                               int nblk) {
+  __shared__ float4 rhs[kB][kNextCols];  // (re, re, im, im)
+  __shared__ float2 part[4][2][kNextCols][kB / 2];
+  const int b = blockIdx.y, tid = threadIdx.x, rp = tid & 63, quarter = tid >> 6;
+  const int kn = kk + kB, c0 = kn + kNextCols * blockIdx.x;
+  float* re = W.re + (size_t)b * W.stride;
+  float* im = W.im + (size_t)b * W.stride;
+  for (int idx = tid; idx < kB * kNextCols; idx += 256) {
+    const int k = idx & (kB - 1), c = idx / kB;
+    const size_t g = (size_t)(c0 + c) * W.ld + kk + k;
+    const float x = re[g], y = im[g];
+    rhs[k][c] = make_float4(x, x, y, y);
+  }
+  float2 ar[kNextCols], ai[kNextCols];
+  auto clear = [&]() {
+#pragma unroll
+    for (int c = 0; c < kNextCols; ++c) ar[c] = ai[c] = make_float2(0.0f, 0.0f);
+  };
+  auto step = [&](int k, float2 xr, float2 xi) {
+    const float2 ni = make_float2(-xi.x, -xi.y);
+#pragma unroll
+    for (int c = 0; c < kNextCols; ++c) {
+      const float4 y = rhs[k][c];
+      const float2 yr = make_float2(y.x, y.y), yi = make_float2(y.z, y.w);
+      ar[c] = fma2(ni, yi, fma2(xr, yr, ar[c]));
+      ai[c] = fma2(xi, yr, fma2(xr, yi, ai[c]));
+    }
+  };
+  // the sum over the quarters: thread (rp, c) has the two rows of column c = quarter
+  auto total = [&](float2& r, float2& i) {
+#pragma unroll
+    for (int c = 0; c < kNextCols; ++c) {
+      part[quarter][0][c][rp] = ar[c];
+      part[quarter][1][c][rp] = ai[c];
+    }
+    __syncthreads();
+    r = i = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 u = part[q][0][quarter][rp], v = part[q][1][quarter][rp];
+      r.x += u.x;
+      r.y += u.y;
+      i.x += v.x;
+      i.y += v.y;
+    }
+  };
+  __syncthreads();
+  const int k0 = quarter * (kB / 4);
+  clear();
+  const float4* X = reinterpret_cast<const float4*>(inv + ((size_t)b * nblk + kk / kB) * kB * kB) + rp;
+#pragma unroll 16
+  for (int k = k0; k < k0 + kB / 4; ++k) {
+    const float4 v = __ldcg(X + (size_t)k * (kB / 2));
+    step(k, make_float2(v.x, v.z), make_float2(v.y, v.w));
+  }
+  float2 yr, yi;
+  total(yr, yi);
+  rhs[2 * rp][quarter] = make_float4(yr.x, yr.x, yi.x, yi.x);
+  rhs[2 * rp + 1][quarter] = make_float4(yr.y, yr.y, yi.y, yi.y);
+  __syncthreads();
+  clear();
+  const size_t a21 = (size_t)kk * W.ld + kn + 2 * rp;
+#pragma unroll 16
+  for (int k = k0; k < k0 + kB / 4; ++k)
+    step(k, *reinterpret_cast<const float2*>(re + a21 + (size_t)k * W.ld),
+         *reinterpret_cast<const float2*>(im + a21 + (size_t)k * W.ld));
+  total(yr, yi);
+  const size_t d = (size_t)(c0 + quarter) * W.ld + kn + 2 * rp;
+  float2* dr = reinterpret_cast<float2*>(re + d);
+  float2* di = reinterpret_cast<float2*>(im + d);
+  const float2 or_ = *dr, oi = *di;
+  *dr = make_float2(or_.x - yr.x, or_.y - yr.y);
+  *di = make_float2(oi.x - yi.x, oi.y - yi.y);
+}
+
 // 16-byte asynchronous global -> shared copy and its completion wait.
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
@@ -935,16 +1023,20 @@ Planes planes_of(const MixedWork& w, int npad) {
 // Streams and events of the lookahead in the block LU, one set per (device,
 // caller stream): factorisations enqueued on different streams (concurrent
 // requests of a server) overlap on the device without sharing a side stream.
-// `side` (highest priority) runs the chain of the next block (inverse,
-// panel), `upper` (lowest priority) the block rows of U' that only the solves
-// need.  The mutex is held
-// while a factorisation is enqueued, so the events are never re-recorded by
+// `chain` and `side` (highest priority) run the diagonal blocks (update,
+// inverse) and the panels, `upper` (lowest priority) the block rows of U' that
+// only the solves need.  The mutex is held while a factorisation is enqueued, so the events are never re-recorded by
 // another caller in between.
 struct Lookahead {
   std::mutex mu;
+  cudaStream_t chain = nullptr;
   cudaStream_t side = nullptr;
   cudaStream_t upper = nullptr;
+  cudaEvent_t inverse = nullptr;
   cudaEvent_t diag = nullptr;
+  cudaEvent_t pre = nullptr;
+  cudaEvent_t rows = nullptr;
+  cudaEvent_t big = nullptr;
   cudaEvent_t strips = nullptr;
   cudaEvent_t colpack = nullptr;
   cudaEvent_t panel = nullptr;
@@ -961,13 +1053,12 @@ int lookahead_for(cudaStream_t caller, Lookahead** out) {
     auto fresh = std::make_unique<Lookahead>();
     int least = 0, greatest = 0;
     BEM_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    BEM_CUDA_CHECK(cudaStreamCreateWithPriority(&fresh->chain, cudaStreamNonBlocking, greatest));
     BEM_CUDA_CHECK(cudaStreamCreateWithPriority(&fresh->side, cudaStreamNonBlocking, greatest));
     BEM_CUDA_CHECK(cudaStreamCreateWithPriority(&fresh->upper, cudaStreamNonBlocking, least));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fresh->diag, cudaEventDisableTiming));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fresh->strips, cudaEventDisableTiming));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fresh->colpack, cudaEventDisableTiming));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fresh->panel, cudaEventDisableTiming));
-    for (auto& e : fresh->upper_done) BEM_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (cudaEvent_t* e : {&fresh->inverse, &fresh->diag, &fresh->pre, &fresh->rows, &fresh->big, &fresh->strips,
+                           &fresh->colpack, &fresh->panel, &fresh->upper_done[0], &fresh->upper_done[1]})
+      BEM_CUDA_CHECK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     la = std::move(fresh);
   }
   *out = la.get();
@@ -1079,14 +1170,18 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
   float* Bop[kOpBuffers] = {w.Bop, w.Bop + bbuf, w.Bop + 2 * bbuf};
   const size_t ainv_buf = (size_t)batch * kB * 2 * kB;
   const int64_t a_stride = (int64_t)npad * 2 * kB;
-  // Inverse of diagonal block kk (its A operand copy in ainv buffer of the
-  // block's parity).
   auto inverse = [&](int kk, cudaStream_t on) {
     TimedLaunch tl(kKCluGj, on);
     clu_gj_kernel<<<batch, 32 * kGjWarps, kGjSmem, on>>>(W, kk, info_dev, w.inv, nblk, err_dev);
+    ++launches;
+  };
+  // its copies as the operands of the panel product and of U' (ainv buffer of
+  // the block's parity)
+  auto inverse_pack = [&](int kk, cudaStream_t on) {
+    TimedLaunch tl(kKCluPanel, on);
     clu_inverse_pack_kernel<<<dim3(kB / 8, batch), 256, 0, on>>>(w.inv, nblk, kk, w.binv,
                                                                  w.ainv + ((kk / kB) & 1) * ainv_buf);
-    launches += 2;
+    ++launches;
   };
   // L21 = A21 A_kk^{-1} (split TF32: A_hi B_hi + A_lo B_hi + A_hi B_lo,
   // float32-level multipliers) into the working matrix and, packed, into the
@@ -1112,94 +1207,143 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
   // C rows r0.. (m), complex columns c0.. (nc) -= L21 U12 of the block step whose
   // packed operands are in buffer buf, and of a second step (buffer buf2 >= 0)
   // in the same pass over C (depth 256); optionally a packed copy of the result.
-  auto update = [&](int buf, int r0, int c0, int m, int nc, int buf2, int run, bool lshape = false,
-                    int reserve = 0) -> int {
+  auto update = [&](int buf, int r0, int c0, int m, int nc, int buf2, int run, cudaStream_t on,
+                    TileRegion region = kTilesAll, int reserve = 0) -> int {
     if (m <= 0 || nc <= 0) return BEM_OK;
     return cgemm_tf32_update(Aop[buf], npad, r0, Bop[buf], 2 * (int64_t)npad, 2 * c0, kUpdateDepth, W.re, W.im, npad,
-                             W.stride, r0, c0, m, nc, batch, err_dev, s, 0, buf2 >= 0 ? Aop[buf2] : nullptr,
-                             buf2 >= 0 ? Bop[buf2] : nullptr, run, 0, act, nullptr, kPackNone, 0, lshape, reserve);
+                             W.stride, r0, c0, m, nc, batch, err_dev, on, 0, buf2 >= 0 ? Aop[buf2] : nullptr,
+                             buf2 >= 0 ? Bop[buf2] : nullptr, run, 0, act, nullptr, kPackNone, 0, region, reserve);
   };
   Lookahead* la = nullptr;
   if ((st = lookahead_for(s, &la))) return st;
   std::lock_guard<std::mutex> lock(la->mu);
-  // Right-looking block LU with a lookahead of one block, the trailing updates
-  // of two consecutive block steps applied in one pass over C (depth 256: the
-  // update is bound by reading and writing C).  Step k, on the caller's
-  // stream: the diagonal block k+1 gets every update still pending on it and
-  // its inverse starts on the side stream; then block row and block column
-  // k+1 get theirs (one L-shaped launch) and are packed as the operands of
-  // step k+1 (A12 as the B operand, A21 split for the panel product) while
-  // the inverse runs; the panel L21 follows on the side stream (its epilogue
-  // packs the A operand), U' on the third stream.  Meanwhile, at every
-  // second step, the rest of the trailing matrix gets the updates of steps
-  // k-1 and k together.
+  auto record = [](cudaEvent_t e, cudaStream_t on) -> int {
+    BEM_CUDA_CHECK(cudaEventRecord(e, on));
+    return BEM_OK;
+  };
+  auto wait = [](cudaStream_t on, cudaEvent_t e) -> int {
+    BEM_CUDA_CHECK(cudaStreamWaitEvent(on, e, 0));
+    return BEM_OK;
+  };
+#define BEM_TRY(call) \
+  if ((st = (call))) return st
+  // Right-looking block LU with a lookahead, the trailing updates of two
+  // consecutive block steps applied in one pass over C (depth 256: the update
+  // is bound by reading and writing C).  Step k, its inverse and operands
+  // (A12 as the B operand, A21 split for the panel product) given:
+  //   chain (highest priority): the diagonal block k+1 gets the update of step
+  //     k and is inverted;
+  //   side (highest priority): the panel product L21 (its epilogue packs the A
+  //     operand), then the updates pending on the diagonal block k+2;
+  //   upper (lowest priority): U', which only the solves need;
+  //   the caller's stream: block row and block column k+1 get their updates
+  //     (one L-shaped launch) and are packed as the operands of step k+1; at
+  //     every second step the rest of the trailing matrix gets the updates of
+  //     steps k-1 and k together.
+  // direct: the diagonal block k+1 gets step k's update straight from A12, A21
+  // and the inverse (clu_next_diagonal_kernel), what is pending on it having
+  // been applied before; otherwise all of it as a tile behind the panel product.
   // Operands of steps k-1, k, k+1 live in three buffers; A_kk^{-1} for U' in
   // two.
-  // Block 0: the operands come straight from the converted matrix.
-  inverse(0, s);
-  if (npad > kB) {
+  // direct while the chain is the bound: fewer than 200 blocks below block k+1
+  // in all matrices together (8 x 3072: 4.13 -> 3.70 ms with 200, 3.88 with 100;
+  // 15 x 6144 the same with 100, 200 and 400), and up to 24 matrices, whose
+  // next blocks still fit the GPU at once (24 x 1024 1.18 -> 1.13 ms, but
+  // 32 x 1536 2.41 -> 2.46, 60 x 1536 3.81 -> 3.95)
+  auto direct = [&](int kk) {
+    return batch <= 24 && (long long)batch * (npad - kk - 2 * kB) < 200ll * kB;
+  };
+  BEM_TRY(record(la->rows, s));
+  BEM_TRY(wait(la->chain, la->rows));
+  inverse(0, la->chain);
+  BEM_TRY(record(la->inverse, la->chain));
+  if (npad > kB) {  // the operands of block 0 come straight from the converted matrix
     const int m = npad - kB;
     TimedLaunch tl(kKCluPanel, s);
     clu_pack_kernel<<<dim3(m / kPT + m / 32, batch), 256, 0, s>>>(W, npad, 0, m / kPT, kB, 0, Bop[0], w.a3, 0);
     ++launches;
+    BEM_TRY(record(la->colpack, s));
+    BEM_TRY(record(la->strips, s));
   }
-  if ((st = panel(0, 0, s))) return st;
-  BEM_CUDA_CHECK(cudaEventRecord(la->panel, s));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(la->upper, la->panel, 0));
-  if ((st = upper(0, 0, la->upper))) return st;
-  BEM_CUDA_CHECK(cudaEventRecord(la->upper_done[0], la->upper));
   for (int kk = 0, step = 0; kk + kB < npad; kk += kB, ++step) {
     const int cur = step % kOpBuffers, prev = (step + kOpBuffers - 1) % kOpBuffers;
     const int nxt = (step + 1) % kOpBuffers;
     const int kn = kk + kB, rest = npad - kn - kB;
     const int pend = (step & 1) ? prev : -1;  // step k-1 still pending beyond block k
-    // U' of block k-1 (third stream) has read the A_kk^{-1} copy that the
-    // inverse of block k+1 overwrites (and, before it, U' of block k-2 the
-    // operand buffer that the strips below overwrite)
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(s, la->upper_done[(step + 1) & 1], 0));
-    if ((st = update(cur, kn, kn, kB, kB, pend, kSideRun))) return st;  // diagonal block kn
-    BEM_CUDA_CHECK(cudaEventRecord(la->diag, s));
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(la->side, la->diag, 0));
-    inverse(kn, la->side);
-    // block row kn and block column kn below the diagonal (one L-shaped
-    // launch), then their packed copies (A12 as the B operand, A21 split for
-    // the panel product), beside the inverse.  (Packing behind the inverse on
-    // the side stream at the steps with a big update, so that the big update
-    // starts right after the strips, measured slower: the pack then shares
-    // the SMs and HBM with the big update.)
-    const bool big_step = (step & 1) && rest > 0;
-    if (rest > 0) {
-      // the inverse of block kn holds one SM per matrix meanwhile
-      if ((st = update(cur, kn, kn, rest + kB, rest + kB, pend, 0, true, batch))) return st;
-      // the block column's split copy first: the panel product starts on it
-      // while the block row is packed as the next step's B operand
+    if (step >= 2) {
+      // U' of block k-2 has read the A^{-1} copy that this block's overwrites
+      // and the operand buffer that the strips below overwrite
+      BEM_TRY(wait(la->side, la->upper_done[step & 1]));
+      BEM_TRY(wait(s, la->upper_done[step & 1]));
+    }
+    BEM_TRY(wait(la->side, la->inverse));
+    inverse_pack(kk, la->side);
+    if (direct(kk)) {
+      BEM_TRY(wait(la->chain, la->rows));
+      if (step > 0) BEM_TRY(wait(la->chain, la->pre));
+      {
+        TimedLaunch tl(kKCluPanel, la->chain);
+        clu_next_diagonal_kernel<<<dim3(kB / kNextCols, batch), 256, 0, la->chain>>>(W, kk, w.inv, nblk);
+        ++launches;
+      }
+      BEM_TRY(record(la->diag, la->chain));
+      inverse(kn, la->chain);
+      BEM_TRY(record(la->inverse, la->chain));
+      BEM_TRY(wait(la->side, la->diag));  // the panel product overwrites A21
+    }
+    BEM_TRY(wait(la->side, la->colpack));
+    BEM_TRY(panel(kk, cur, la->side));
+    BEM_TRY(record(la->panel, la->side));
+    // U' reads the block row's B operand and the inverse, and overwrites A12
+    BEM_TRY(wait(la->upper, la->strips));
+    BEM_TRY(wait(la->upper, la->panel));
+    BEM_TRY(upper(kk, cur, la->upper));
+    BEM_TRY(record(la->upper_done[step & 1], la->upper));
+    BEM_TRY(wait(s, la->panel));
+    if (!direct(kk)) {
+      BEM_TRY(update(cur, kn, kn, kB, kB, pend, kSideRun, s));
+      BEM_TRY(record(la->diag, s));
+      BEM_TRY(wait(la->chain, la->diag));
+      inverse(kn, la->chain);
+      BEM_TRY(record(la->inverse, la->chain));
+    }
+    if (rest == 0) break;
+    const bool ahead = direct(kn);
+    if (ahead) {  // what is pending on the next step's diagonal block
+      BEM_TRY(wait(la->side, la->strips));
+      if (step >= 2) BEM_TRY(wait(la->side, la->big));
+      BEM_TRY(update(cur, kn + kB, kn + kB, kB, kB, pend, kSideRun, la->side));
+      BEM_TRY(record(la->pre, la->side));
+    }
+    // block row kn and block column kn below the diagonal; the inverse of
+    // block kn holds one SM per matrix meanwhile
+    BEM_TRY(update(cur, kn, kn, rest + kB, rest + kB, pend, 0, s, kTilesL, batch));
+    BEM_TRY(record(la->rows, s));
+    // the block column's split copy first: the panel product starts on it
+    // while the block row is packed as the next step's B operand.  (Strips and
+    // packs on a stream of their own beside the big update: 15 x 6144 29.4 ->
+    // 30.4 ms; they share its SMs and HBM.)
+    {
       TimedLaunch tl(kKCluPanel, s);
       clu_pack_kernel<<<dim3(rest / 32, batch), 256, 0, s>>>(W, npad, kn, rest / kPT, kn + kB, kn, Bop[nxt], w.a3,
                                                             rest / kPT);
-      BEM_CUDA_CHECK(cudaEventRecord(la->colpack, s));
+      BEM_TRY(record(la->colpack, s));
       clu_pack_kernel<<<dim3(rest / kPT, batch), 256, 0, s>>>(W, npad, kn, rest / kPT, kn + kB, kn, Bop[nxt], w.a3,
                                                              0);
       launches += 2;
-    } else {
-      BEM_CUDA_CHECK(cudaEventRecord(la->colpack, s));
     }
-    BEM_CUDA_CHECK(cudaEventRecord(la->strips, s));
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(la->side, la->colpack, 0));
-    if ((st = panel(kn, nxt, la->side))) return st;
-    BEM_CUDA_CHECK(cudaEventRecord(la->panel, la->side));
-    // U' reads the block row's B operand and the inverse
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(la->upper, la->strips, 0));
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(la->upper, la->panel, 0));
-    if ((st = upper(kn, nxt, la->upper))) return st;
-    BEM_CUDA_CHECK(cudaEventRecord(la->upper_done[(step + 1) & 1], la->upper));
-    if (big_step) {
-      if ((st = update(cur, kn + kB, kn + kB, rest, rest, prev, kBigRun))) return st;
+    BEM_TRY(record(la->strips, s));
+    if (step & 1) {
+      BEM_TRY(update(cur, kn + kB, kn + kB, rest, rest, prev, kBigRun, s, ahead ? kTilesNoCorner : kTilesAll));
+      BEM_TRY(record(la->big, s));
     }
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(s, la->panel, 0));
   }
-  // the last block rows of U' are part of the factors
-  BEM_CUDA_CHECK(cudaEventRecord(la->upper_done[0], la->upper));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(s, la->upper_done[0], 0));
+  BEM_TRY(wait(s, la->inverse));
+  if (npad > kB) {  // the last block rows of U' are part of the factors
+    BEM_TRY(record(la->upper_done[0], la->upper));
+    BEM_TRY(wait(s, la->upper_done[0]));
+  }
+#undef BEM_TRY
   count_launches(launches);
   BEM_CUDA_CHECK(cudaGetLastError());
   return BEM_OK;

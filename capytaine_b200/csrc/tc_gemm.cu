@@ -175,10 +175,10 @@ struct UpdateArgs {
   float* pack;
   int64_t pack_stride;  // floats between matrices
   int pack_mode;
-  // L-shaped launch: only the first tile row and the first tile column of the
-  // m x n block, without the corner tile (R = tiles_m - 1 of each; grouped:
-  // R of matrix b in gtm[b])
-  int lshape;
+  // kTilesL: only the first tile row and the first tile column of the m x n
+  // block, without the corner tile (R = tiles_m - 1 of each; grouped: R of
+  // matrix b in gtm[b]); kTilesNoCorner: all tiles but the corner
+  int region;
   int gstart[kMaxGroup + 1];
   short gtm[kMaxGroup];
   short gtn[kMaxGroup];
@@ -186,7 +186,7 @@ struct UpdateArgs {
 
 // Matrix and tile coordinates of tile t of the launch.
 __device__ __forceinline__ void decode_tile(const UpdateArgs& p, int t, int& b, int& tm, int& tn) {
-  if (p.lshape) {
+  if (p.region == kTilesL) {
     int R, r;
     if (p.ngroup > 0) {
       b = 0;
@@ -207,17 +207,18 @@ __device__ __forceinline__ void decode_tile(const UpdateArgs& p, int t, int& b, 
     }
     return;
   }
+  const int first = p.region == kTilesNoCorner ? 1 : 0;
   if (p.ngroup > 0) {
     b = 0;
     while (b + 1 < p.ngroup && p.gstart[b + 1] <= t) ++b;
-    const int r = t - p.gstart[b];
+    const int r = t - p.gstart[b] + first;
     tn = r / p.gtm[b];
     tm = r - tn * p.gtm[b];
     return;
   }
-  const int per_matrix = p.tiles_m * p.tiles_n;
+  const int per_matrix = p.tiles_m * p.tiles_n - first;
   b = t / per_matrix;
-  const int r = t - b * per_matrix;
+  const int r = t - b * per_matrix + first;
   tn = r / p.tiles_m;
   tm = r - tn * p.tiles_m;
 }
@@ -514,9 +515,9 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
                       const CgemmDepth& depth, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
                       int n, int batch, int* err, cudaStream_t stream, int store, const float* Aop1,
                       const float* Bop1, int run, long long wait_limit, const int* limit_host, float* pack,
-                      int pack_mode, int64_t pack_stride, bool lshape, int reserve_sms) {
+                      int pack_mode, int64_t pack_stride, TileRegion region, int reserve_sms) {
   if (m <= 0 || n <= 0) return BEM_OK;
-  if (lshape && (m != n || m <= kTM || pack_mode != kPackNone))
+  if (region == kTilesL && (m != n || m <= kTM || pack_mode != kPackNone))
     return set_error(BEM_ERR_INVALID_ARGUMENT, "cgemm_tf32_update: an L-shaped update needs a square block of "
                                                "more than one tile and no packed copy");
   if (pack_mode != kPackNone &&
@@ -571,13 +572,14 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
   p.pack = pack;
   p.pack_stride = pack_stride;
   p.pack_mode = pack_mode;
-  p.lshape = lshape ? 1 : 0;
+  p.region = region;
   int launches = 0;
   // Grouped: matrix b covers only rows and columns below limit_host[b] (its
   // active size), launches of at most kMaxGroup matrices
   for (int b0 = 0; b0 < batch; b0 += limit_host ? kMaxGroup : batch) {
     const int nb = limit_host ? std::min(kMaxGroup, batch - b0) : batch;
-    long long ntiles = lshape ? 2ll * (tiles_m - 1) * nb : (long long)tiles_m * tiles_n * nb;
+    const int corner = region == kTilesNoCorner ? 1 : 0;
+    long long ntiles = region == kTilesL ? 2ll * (tiles_m - 1) * nb : ((long long)tiles_m * tiles_n - corner) * nb;
     if (limit_host) {
       p.ngroup = nb;
       ntiles = 0;
@@ -586,7 +588,7 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
         const int mb = std::max(0, std::min(m, lim - c_row0)) / kTM;
         const int nbc = std::max(0, std::min(n, lim - c_col0)) / kTNc;
         p.gstart[i] = (int)ntiles;
-        if (lshape) {  // R tiles in the row and R in the column beyond the corner
+        if (region == kTilesL) {  // R tiles in the row and R in the column beyond the corner
           const int R = std::max(0, mb - 1);
           p.gtm[i] = (short)R;
           p.gtn[i] = 0;
@@ -595,7 +597,7 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
         }
         p.gtm[i] = (short)std::max(mb, 1);  // never divides by zero; no tile when gtn is 0
         p.gtn[i] = (short)(mb > 0 ? nbc : 0);
-        ntiles += (long long)(mb > 0 ? mb : 0) * (mb > 0 ? nbc : 0);
+        ntiles += std::max(0ll, (long long)mb * nbc - corner);
       }
       p.gstart[nb] = (int)ntiles;
     }
@@ -645,5 +647,5 @@ extern "C" int bem_cgemm_tf32_update(const float* Aop_dev, int64_t a_rows, int a
                                              : bem::CgemmDepth{kp, kp, kp, 1, 0, 0, {0, 0, 0}, true};
   return bem::cgemm_tf32_update(Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, depth, Cr_dev, Ci_dev, ldc, c_stride,
                                 c_row0, c_col0, m, n, batch, err_dev, (cudaStream_t)stream, 0, nullptr, nullptr, 0, 0,
-                                nullptr, nullptr, bem::kPackNone, 0, false, 0);
+                                nullptr, nullptr, bem::kPackNone, 0, bem::kTilesAll, 0);
 }
