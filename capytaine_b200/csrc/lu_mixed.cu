@@ -304,7 +304,8 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
 // Bound: the chain of panels on one SM, 8000 cycles each: the factorisation 4400
 // (540 a column: shuffles of the pivot row, reciprocal, multipliers, the key and
 // its reduction), the next warp's rank-8 update 2050, the exchange 1300; the
-// other warps' updates (5000 a scheduler) run beside it.  80 us per block.  One
+// other warps' updates (5000 a scheduler) run beside it.  77 us per block (80
+// with a pass of its own for the scaling and a serial loop of the stores).  One
 // step per exchange took 1800 cycles a column (121 us per block with the packed
 // copies written by the same CTA): a pivot search, two trips through shared
 // memory and a barrier each.  Row pairs and duplicated pivot entries feed the
@@ -421,30 +422,23 @@ __global__ void __launch_bounds__(32 * kGjWarps, 1) clu_gj_kernel(Planes W, int 
   __syncthreads();
   if (sh.abort) return;
   if (tid < kB) sh.jinv[sh.piv_row[tid]] = tid;
-  // rows scaled by their pivots' reciprocals
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float2 s0 = sh.rowscale[r0 + 64 * h], s1 = sh.rowscale[r0 + 1 + 64 * h];
-#pragma unroll
-    for (int m = 0; m < kGjPanel; ++m) {
-      float2* pr = reinterpret_cast<float2*>(mr + m * kGjLd + 64 * h);
-      float2* pi = reinterpret_cast<float2*>(mi + m * kGjLd + 64 * h);
-      const float2 re = *pr, im = *pi;
-      const float2 v0 = fmul(make_float2(re.x, im.x), s0), v1 = fmul(make_float2(re.y, im.y), s1);
-      *pr = make_float2(v0.x, v1.x);
-      *pi = make_float2(v0.y, v1.y);
-    }
-  }
   __syncthreads();
-  // A_kk^{-1}(row, col) = a(piv_row[row], jinv[col]): column-major 128 x 128, four
-  // rows per thread
-  float4* out = reinterpret_cast<float4*>(inv + ((size_t)b * nblk + kk / kB) * kB * kB);
-#pragma unroll 1
-  for (int col = w; col < kB; col += kGjWarps) {
-    const int o = sh.jinv[col] * kGjLd;
-    const int4 p = *reinterpret_cast<const int4*>(sh.piv_row + 4 * lane);
-    out[col * (kB / 2) + 2 * lane] = make_float4(Mre[o + p.x], Mim[o + p.x], Mre[o + p.y], Mim[o + p.y]);
-    out[col * (kB / 2) + 2 * lane + 1] = make_float4(Mre[o + p.z], Mim[o + p.z], Mre[o + p.w], Mim[o + p.w]);
+  // A_kk^{-1}(row, col) = a(piv_row[row], jinv[col]) / pivot of the row: column-major
+  // 128 x 128, a lane's four rows 32 apart
+  int p[4];
+  float2 scale[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    p[u] = sh.piv_row[lane + 32 * u];
+    scale[u] = sh.rowscale[p[u]];
+  }
+  float2* out = inv + ((size_t)b * nblk + kk / kB) * kB * kB + lane;
+#pragma unroll 4
+  for (int m = 0; m < kGjPanel; ++m) {
+    const int col = w + kGjWarps * m, o = sh.jinv[col] * kGjLd;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      out[col * kB + 32 * u] = fmul(make_float2(Mre[o + p[u]], Mim[o + p[u]]), scale[u]);
   }
 }
 
@@ -639,9 +633,9 @@ __global__ void __launch_bounds__(256) clu_next_diagonal_kernel(Planes W, int kk
   const size_t d = (size_t)(c0 + quarter) * W.ld + kn + 2 * rp;
   float2* dr = reinterpret_cast<float2*>(re + d);
   float2* di = reinterpret_cast<float2*>(im + d);
-  const float2 or_ = *dr, oi = *di;
-  *dr = make_float2(or_.x - yr.x, or_.y - yr.y);
-  *di = make_float2(oi.x - yi.x, oi.y - yi.y);
+  const float2 oldr = *dr, oldi = *di;
+  *dr = make_float2(oldr.x - yr.x, oldr.y - yr.y);
+  *di = make_float2(oldi.x - yi.x, oldi.y - yi.y);
 }
 
 // 16-byte asynchronous global -> shared copy and its completion wait.
