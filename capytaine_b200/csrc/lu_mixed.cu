@@ -43,7 +43,6 @@ constexpr int kRhs = 16;       // right-hand sides per solve launch
 constexpr int kOpBuffers = 3;  // packed operands of the current, previous and next block steps
 
 __device__ __forceinline__ float2 fmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-__device__ __forceinline__ float fabs1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 // a b + c on a pair of floats in one instruction (fma.rn.f32x2: per element the
 // correctly rounded fused multiply-add of fmaf)
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -66,10 +65,6 @@ struct Planes {
 // exact in float32 and is the "lo" part of the split product.
 __device__ __forceinline__ float tf32_hi(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
 
-__device__ __forceinline__ float2 ldp(const Planes& W, int b, int r, int c) {
-  const size_t o = (size_t)b * W.stride + (size_t)r + (size_t)c * W.ld;
-  return make_float2(W.re[o], W.im[o]);
-}
 __device__ __forceinline__ void stp(const Planes& W, int b, int r, int c, float2 v) {
   const size_t o = (size_t)b * W.stride + (size_t)r + (size_t)c * W.ld;
   W.re[o] = v.x;
