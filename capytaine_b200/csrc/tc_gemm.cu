@@ -15,15 +15,19 @@
 // columns: real parts then imaginary parts).  Warp 0 streams operand slices with
 // TMA (128-byte swizzle) through a three-stage shared-memory ring, 32 values of
 // depth per stage of both parts of A (32 KB) and of B (32 KB); one thread of warp
-// 1 issues, per 8 of depth, one tcgen05.mma of N = 256 (Re A against [Re B; Im B])
-// and two of N = 128 (Im A against Im B, negated, and against Re B).  Every
-// operand byte crosses from L2 once per tile: with the real embedding [[Br, Bi],
+// 1 issues, per 8 of depth, four tcgen05.mma of M = N = 128: Re A and Im A (negated)
+// against Re B and Im B into the real columns, against Im B and Re B into the
+// imaginary ones.  All have one shape: two tcgen05.mma of a thread are ordered
+// when their accumulator and shape agree, so one of N = 256 over both halves of
+// the accumulator (Re A against [Re B; Im B]: 505 TF/s) must not be mixed in.
+// Every operand byte crosses from L2 once per tile: with the real embedding [[Br, Bi],
 // [-Bi, Br]] stored as such, each part of B came twice, 786 KB per tile of depth
 // 256 against 524, and had to be packed twice.
-// Bound: shared-memory bandwidth.  Per 8 of depth the MMAs read 28 KB in what would
-// be 262 clocks and TMA writes 16 KB, 169 bytes per clock of the 128 there are
-// (with the embedding 184).  15 x 5888^2, depth 256: 469 -> 505 TF/s, 0.69 of cuBLAS
-// on plain TF32 matrices; a pair of SMs sharing B (cta_group::2) would read less.
+// Bound: shared-memory bandwidth.  Per 8 of depth the MMAs read 32 KB and TMA
+// writes 16 KB in what would be 256 clocks, 192 bytes per clock of the 128 there
+// are.  15 x 5888^2, depth 256: 490 TF/s (469 with the embedding and N = 256),
+// 0.67 of cuBLAS on plain TF32 matrices; the order of the four makes no difference
+// (489 to 490); a pair of SMs sharing B (cta_group::2) would read less.
 // Sixteen warps read the accumulator back with tcgen05.ld and apply C -= acc in
 // place, the loads of C running ahead of the accumulator reads.
 // Every mbarrier wait is bounded; on timeout the kernel records an error and
@@ -38,7 +42,7 @@ namespace {
 
 constexpr int kTM = 128;            // tile rows
 constexpr int kTNc = 128;           // tile complex columns
-constexpr int kTN = 2 * kTNc;       // accumulator columns (MMA N)
+constexpr int kTN = 2 * kTNc;       // accumulator columns (two halves of MMA N = kTNc)
 constexpr int kKC = 32;             // values of depth per stage (128 bytes of fp32)
 constexpr int kStages = 3;
 constexpr int kABytes = kTM * kKC * 4;   // 16 KiB: one part of A
@@ -88,14 +92,13 @@ __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t saddr) {
   return d;
 }
 
-// Instruction descriptor: D f32, A/B tf32, both K-major, M = 128; bit 13 negates A.
-constexpr uint32_t idesc_tf32(int n, bool negate_a) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((negate_a ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) |
+// Instruction descriptor: D f32, A/B tf32, both K-major, M = N = 128; bit 13 negates A.
+constexpr uint32_t idesc_tf32(bool negate_a) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((negate_a ? 1u : 0u) << 13) | ((uint32_t)(kTNc >> 3) << 17) |
          ((uint32_t)(kTM >> 4) << 24);
 }
-constexpr uint32_t kIdescBoth = idesc_tf32(kTN, false);
-constexpr uint32_t kIdescHalf = idesc_tf32(kTNc, false);
-constexpr uint32_t kIdescHalfNeg = idesc_tf32(kTNc, true);
+constexpr uint32_t kIdesc = idesc_tf32(false);
+constexpr uint32_t kIdescNeg = idesc_tf32(true);
 
 __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -350,13 +353,15 @@ __global__ void __launch_bounds__(kThreads, 1) cgemm_tf32_update_kernel(const __
 #pragma unroll
           for (int kk = 0; kk < kKC / 8; ++kk) {
             // K = 8 tf32 = 32 bytes per instruction inside the 128-byte swizzle atom
+            const uint64_t ar = smem_desc_k_sw128(a0 + kk * 32);
             const uint64_t br = smem_desc_k_sw128(b0 + kk * 32);
-            mma_tf32(tacc, smem_desc_k_sw128(a0 + kk * 32), br, kIdescBoth, (kc | kk) != 0);
+            const uint64_t bi = smem_desc_k_sw128(b0 + kBBytes / 2 + kk * 32);
+            mma_tf32(tacc, ar, br, kIdesc, (kc | kk) != 0);
+            mma_tf32(tacc + kTNc, ar, bi, kIdesc, (kc | kk) != 0);
             if (!p.embedded) {
               const uint64_t ai = smem_desc_k_sw128(a0 + kABytes + kk * 32);
-              const uint64_t bi = smem_desc_k_sw128(b0 + kBBytes / 2 + kk * 32);
-              mma_tf32(tacc, ai, bi, kIdescHalfNeg, 1);
-              mma_tf32(tacc + kTNc, ai, br, kIdescHalf, 1);
+              mma_tf32(tacc, ai, bi, kIdescNeg, 1);
+              mma_tf32(tacc + kTNc, ai, br, kIdesc, 1);
             }
           }
           mma_commit(&empty[s]);
