@@ -1155,9 +1155,10 @@ def _raise_on_timeout(err):
 
 def _column_major(t):
     """The (n, K) tensor t as a (K, n) contiguous complex128 one: its own memory
-    when it is column-major already (the engine's matrices are)."""
+    when it is column-major already (the engine's matrices are) and holds the
+    values themselves (torch conjugates and negates lazily)."""
     import torch
-    a = t.T
+    a = t.T.resolve_conj().resolve_neg()
     return a.contiguous() if a.dtype == torch.complex128 else a.to(torch.complex128).contiguous()
 
 
