@@ -1224,9 +1224,12 @@ class DeviceMatrix:
                                       _lib.stream_ptr()))
         if int(info.item()) != 0:
             raise _lib.SingularMatrixError(_lib.BEM_ERR_SINGULAR, f"zero pivot at column {int(info.item())}")
-        # the unfactored matrix, column-major complex128, for the residual checks
+        # the matrix that was factored, column-major complex128, for the residual
+        # checks: a copy, since t may change in place between two solves
+        Kcm = torch.empty((n, n), dtype=torch.complex128, device=dev)  # Kcm[j, i] = K[i, j]
+        Kcm.copy_(self.t.T)
+        self._kcm = Kcm
         self._lu = (Kf, piv, work, npad)
-        self._kcm = _column_major(self.t)  # _kcm[j, i] = K[i, j]
         return self._lu
 
     def gmres(self, b: np.ndarray, *, atol=1e-6, rtol=1e-5, restart=20, maxiter=None) -> np.ndarray:

@@ -42,3 +42,17 @@ def test_products_and_solves(n, m, form):
             for got in solutions:
                 assert got.shape == x.shape
                 assert np.all(np.abs(got - x) <= 10 * tol * max(1.0, np.abs(x).max(initial=0)))
+
+
+def test_solves_keep_to_the_matrix_that_was_factored():
+    import torch
+    from capytaine_b200.engine import B200Engine, DeviceMatrix
+    rng = np.random.default_rng(5)
+    n = 100
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 4 * n * np.eye(n)
+    b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    M = DeviceMatrix(torch.as_tensor(A.T.copy(), device="cuda").T, B200Engine())
+    first = M.solve(b)
+    M.t.mul_(3.0)
+    assert np.array_equal(M.solve(b), first)
+    assert np.allclose(M @ first, 3 * b, rtol=0, atol=1e-11)  # products are of the matrix as it is
