@@ -189,6 +189,30 @@ __device__ __forceinline__ unsigned gj_key(float re, float im, int row, unsigned
   return (((__float_as_uint(m) + 128u) & ~127u) | (unsigned)(127 - row)) & left;
 }
 
+// 1 / (re + i im) for any pivot: where the square of its modulus is far inside
+// the range of float32, conj(pivot) times the hardware's estimate of 1 / d
+// (rcp.approx, which flushes) and one step of Newton-Raphson for 1 / d,
+// r + r (1 - d r); elsewhere quotients of the pivot scaled by the power of two of
+// its larger part (out of line: the range costs 2 us per block, in line 3).  0 for a
+// zero pivot, infinite for one below 2^-128.
+__device__ __noinline__ float2 gj_reciprocal_scaled(float re, float im) {
+  const float m = fmaxf(fabsf(re), fabsf(im));
+  if (!(m > 0.0f)) return make_float2(0.0f, 0.0f);
+  const int e = ilogbf(m);
+  const float x = scalbnf(re, -e), y = scalbnf(im, -e), n = x * x + y * y;
+  return make_float2(scalbnf(x / n, -e), scalbnf(-y / n, -e));
+}
+__device__ __forceinline__ float2 gj_reciprocal(float re, float im) {
+  const float d = re * re + im * im;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(r, fmaf(-d, r, 1.0f), r);
+  float2 out = make_float2(re * r, -im * r);
+  // the pivot is the same in every lane: no divergence
+  if (!(d > 0x1p-100f && d < 0x1p100f)) out = gj_reciprocal_scaled(re, im);
+  return out;
+}
+
 // A warp's columns in registers: [pair of rows][column], planes apart.
 struct GjColumns {
   float2 re[2][kGjPanel], im[2][kGjPanel];
@@ -218,7 +242,7 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
                             gj_key(a.re[1][0].y, a.im[1][0].y, r0 + 65, left[3]));
     return __reduce_max_sync(0xffffffffu, max(k0, k1));
   };
-  unsigned key = column_key(), zeros = 0u;
+  unsigned key = column_key();
   int my_p = 0;  // of step s in lane s: stored once at the end
   float2 my_scale = make_float2(0.0f, 0.0f);
 #pragma unroll 1
@@ -237,11 +261,8 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
       if (p & 1) { BEM_GJ_ROW(0, y) } else { BEM_GJ_ROW(0, x) }
     }
 #undef BEM_GJ_ROW
-    const float d = ur[0] * ur[0] + ui[0] * ui[0];
-    float rd;  // 1 / d: the hardware's estimate and a Newton step
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rd) : "f"(d));
-    rd = d > 0.0f ? fmaf(rd, fmaf(-d, rd, 1.0f), rd) : 0.0f;
-    const float dr = ur[0] * rd, di = -ui[0] * rd;
+    const float2 recip = gj_reciprocal(ur[0], ui[0]);
+    const float dr = recip.x, di = recip.y;
     const bool own[4] = {p == r0, p == r0 + 1, p == r0 + 64, p == r0 + 65};
 #pragma unroll
     for (int i = 0; i < 4; ++i) left[i] = own[i] ? 0u : left[i];
@@ -280,14 +301,15 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
       my_p = p;
       my_scale = make_float2(dr, di);
     }
-    zeros |= (fabsf(ur[0]) + fabsf(ui[0]) > 0.0f ? 0u : 1u) << s;
   }
   if (lane < kGjPanel) {
     sh.piv_row[kGjPanel * q + lane] = my_p;
     sh.rowscale[my_p] = my_scale;
     sh.used[my_p] = 1;
   }
-  if (zeros && lane == 0 && info[b] == 0) info[b] = kk + kGjPanel * q + __ffs(zeros);
+  const bool sound = isfinite(my_scale.x) && isfinite(my_scale.y) && (my_scale.x != 0.0f || my_scale.y != 0.0f);
+  const unsigned bad = __ballot_sync(0xffffffffu, lane < kGjPanel && !sound);
+  if (bad && lane == 0 && info[b] == 0) info[b] = kk + kGjPanel * q + __ffs(bad);
 }
 
 // Inverse of the diagonal block A_kk by Gauss-Jordan elimination with partial
@@ -299,15 +321,15 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
 // Bound: the chain of panels on one SM, 8000 cycles each: the factorisation 4400
 // (540 a column: shuffles of the pivot row, reciprocal, multipliers, the key and
 // its reduction), the next warp's rank-8 update 2050, the exchange 1300; the
-// other warps' updates (5000 a scheduler) run beside it.  77 us per block (80
+// other warps' updates (5000 a scheduler) run beside it.  79 us per block (82
 // with a pass of its own for the scaling and a serial loop of the stores).  One
 // step per exchange took 1800 cycles a column (121 us per block with the packed
 // copies written by the same CTA): a pivot search, two trips through shared
 // memory and a barrier each.  Row pairs and duplicated pivot entries feed the
 // pair instructions without moves; interleaved complex entries in registers
 // spent as much on moves and divergent row extraction as panels saved (170 us).
-// Output: inv (128 x 128, column-major) = A_kk^{-1}; info flags an exactly zero
-// pivot; err is set when a bounded wait runs out.
+// Output: inv (128 x 128, column-major) = A_kk^{-1}; info flags a pivot without a
+// finite reciprocal; err is set when a bounded wait runs out.
 __global__ void __launch_bounds__(32 * kGjWarps, 1) clu_gj_kernel(Planes W, int kk, int* __restrict__ info,
                                                                  float2* __restrict__ inv, int nblk,
                                                                  int* __restrict__ err) {

@@ -62,3 +62,25 @@ def test_zero_column_is_reported(column):
     m[:, column] = 0.0
     _, info = _solve_block([np.eye(128, dtype=complex), m])
     assert info.tolist() == [0, column + 1]
+
+
+@pytest.mark.parametrize("scale", [1e-36, 1e-30, 1e-19, 2.0 ** -50, 2.0 ** 50, 1e19, 1e30, 1e36])
+def test_inverse_at_every_scale(scale):
+    # squares of these pivots leave the range of float32, their reciprocals do not
+    rng = np.random.default_rng(13)
+    n = 128
+    m = 0.5 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    m[np.arange(n), np.arange(n)] += np.exp(1j * rng.uniform(0, 6, n))
+    m[:, ::3] *= 3.0  # columns on both sides of a range's edge
+    X, info = _solve_block([m * scale])
+    assert info.tolist() == [0]
+    ref = np.linalg.inv(m * scale)
+    assert np.abs(X[0] - ref).max() < 1e-4 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("pivot", [1e-40, 1e-42j, np.inf])
+def test_pivot_without_a_finite_reciprocal_is_reported(pivot):
+    m = np.eye(128, dtype=complex)
+    m[41, 41] = pivot
+    _, info = _solve_block([m])
+    assert info.tolist() == [42]
