@@ -62,12 +62,16 @@ struct DiagShared {
 __device__ __forceinline__ double2 shfl2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-__device__ __forceinline__ double2 cinv(double2 a) {  // 1 / a
-  const double d = 1.0 / (a.x * a.x + a.y * a.y);
-  return make_double2(a.x * d, -a.y * d);
+// 1 / a, a != 0, by quotients of a scaled by the power of two of its larger part
+// (out of line: 1% of an 800-panel sweep, in line 2.5%).
+__device__ __noinline__ double2 cinv(double2 a) {
+  const int e = ilogb(fmax(fabs(a.x), fabs(a.y)));
+  const double x = scalbn(a.x, -e), y = scalbn(a.y, -e), n = x * x + y * y;
+  return make_double2(scalbn(x / n, -e), scalbn(-y / n, -e));
 }
-// The same without a branch, for moduli well inside the exponent range: the
-// hardware's estimate of the reciprocal and two Newton steps.
+// The same without a branch where the square of the modulus is well inside the
+// range of float64: the hardware's estimate of the reciprocal and two steps of
+// Newton-Raphson for 1 / d, r + r (1 - d r).
 __device__ __forceinline__ double2 cinv_fast(double2 a, bool& in_range) {
   const double d = a.x * a.x + a.y * a.y;
   in_range = d > 1e-280 && d < 1e280;
@@ -200,7 +204,9 @@ __device__ __forceinline__ void invert_lower16(double2* T, int base, int lane) {
 __device__ __forceinline__ void invert_upper16(double2* T, int base, int lane) {
   const int c = lane & 15;
   const double2 d = T[(base + c) * kLdD + base + c];
-  const double2 mine = cabs1(d) > 0.0 ? cinv(d) : make_double2(0.0, 0.0);
+  bool in_range;
+  double2 mine = cinv_fast(d, in_range);
+  if (!in_range) mine = cabs1(d) > 0.0 ? cinv(d) : make_double2(0.0, 0.0);
   double2 x[16];
 #pragma unroll
   for (int r = 0; r < 16; ++r) x[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);

@@ -321,7 +321,7 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
 // Bound: the chain of panels on one SM, 8000 cycles each: the factorisation 4400
 // (540 a column: shuffles of the pivot row, reciprocal, multipliers, the key and
 // its reduction), the next warp's rank-8 update 2050, the exchange 1300; the
-// other warps' updates (5000 a scheduler) run beside it.  79 us per block (82
+// other warps' updates (5000 a scheduler) run beside it.  79 us per block (80
 // with a pass of its own for the scaling and a serial loop of the stores).  One
 // step per exchange took 1800 cycles a column (121 us per block with the packed
 // copies written by the same CTA): a pivot search, two trips through shared

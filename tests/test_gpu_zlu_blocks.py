@@ -48,3 +48,28 @@ def test_factors_reproduce_the_matrix(n, batch):
             s = slice(64 * i, 64 * i + 64)
             for tri, x in ((L[s, s], inv[b, i, 0].T), (U[s, s], inv[b, i, 1].T)):
                 assert np.abs(tri @ x - np.eye(64)).max() < 1e-11
+
+
+@pytest.mark.parametrize("scale", [1e-300, 1e-200, 1e-158, 1e-139, 1e139, 1e158, 1e200, 1e290])
+def test_factors_at_every_scale(scale):
+    # squares of these pivots leave the range of float64, their reciprocals do not
+    import torch
+    lib = _lib.load()
+    rng = np.random.default_rng(17)
+    n = 192
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3 * np.sqrt(n) * np.eye(n)
+    A *= scale
+    B = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    At = torch.as_tensor(np.ascontiguousarray(A.T), device="cuda")
+    Bt = torch.as_tensor(np.ascontiguousarray(B.T), device="cuda")
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(lib.bem_zlu_workspace_bytes(n, 1)), dtype=torch.uint8, device="cuda")
+    s = _lib.stream_ptr()
+    _lib.check(lib.bem_zlu_factor(_vp(At), n, n, n * n, 1, _vp(piv), _vp(info), _vp(work), s))
+    _lib.check(lib.bem_zlu_solve(_vp(At), n, n, n * n, 1, _vp(piv), _vp(work), _vp(Bt), n, n * 2, 2, _vp(err), s))
+    assert int(info.item()) == 0 and int(err.item()) == 0
+    X = Bt.cpu().numpy().T * scale  # X of the unscaled matrix
+    want = np.linalg.solve(A / scale, B)
+    assert np.abs(X - want).max() < 1e-12 * np.abs(want).max()
