@@ -43,10 +43,11 @@ struct FaceRec {
 // Plain Euclidean norm, used inside the exact integrals (last-ulp differences only).
 __device__ __forceinline__ double dnorm3(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
 
-// 1 / sqrt(x) for positive normal x: the hardware's estimate (rsqrt.approx) and
-// one step of third order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2, which
-// takes an error of 2^-19 below that of the roundings.  No branch and about
-// half the operations of rsqrt(); within 2 ulp.
+// 1 / sqrt(x) for positive normal x: the hardware's estimate y (rsqrt.approx)
+// and the first two terms of the binomial series of 1 / sqrt(x) =
+// y (1 - e)^(-1/2) with e = 1 - x y^2, y + y e (1/2 + 3/8 e), which take an error
+// of 2^-19 below that of the roundings: within 2 ulp.  0, subnormal and infinite
+// x give NaN: the callers keep them out.
 __device__ __forceinline__ double rsqrt_pos(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -1488,7 +1489,9 @@ __global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_as
             I[2] = I5[3];
             I[3] = I5[4];
           }
-          const double inv_r1 = rsqrt_pos(rr * rr + zz * zz);
+          // infinite where the point meets a quadrature point of the free surface
+          const double r2 = rr * rr + zz * zz;
+          const double inv_r1 = r2 > 1e-300 ? rsqrt_pos(r2) : 1.0 / hypot(rr, zz);
           double hr = I[2], vr = I[0];
           if (high) {
             const double s3 = 2 * inv_r1 * inv_r1 * inv_r1;
