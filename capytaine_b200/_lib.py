@@ -128,6 +128,7 @@ _SIGNATURES = {
                       c_double, c_double, c_void_p, c_i64, c_i64, c_int, c_void_p, c_void_p], c_int),
     "bem_integrate_pressure": ([c_int, c_int, c_int, c_int, c_void_p, c_i64, c_i64, c_void_p, c_double, c_void_p,
                                 c_void_p, c_void_p], c_int),
+    "bem_reciprocals": ([c_int, c_i64, c_void_p, c_void_p, c_void_p], c_int),
     "bem_cgemm_tf32_update": ([c_void_p, c_i64, c_int, c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p, c_i64,
                                c_i64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "bem_clu_workspace_bytes": ([c_int, c_int], c_i64),

@@ -23,6 +23,7 @@
 #include <cmath>
 #include "integrals.cuh"
 #include "packed_table.cuh"
+#include "reciprocals.cuh"
 
 namespace bem {
 namespace {
@@ -42,18 +43,6 @@ struct FaceRec {
 
 // Plain Euclidean norm, used inside the exact integrals (last-ulp differences only).
 __device__ __forceinline__ double dnorm3(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
-
-// 1 / sqrt(x) for positive normal x: the hardware's estimate y (rsqrt.approx)
-// and the first two terms of the binomial series of 1 / sqrt(x) =
-// y (1 - e)^(-1/2) with e = 1 - x y^2, y + y e (1/2 + 3/8 e), which take an error
-// of 2^-19 below that of the roundings: within 2 ulp.  0, subnormal and infinite
-// x give NaN: the callers keep them out.
-__device__ __forceinline__ double rsqrt_pos(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
 
 // Fortran NORM2 with gfortran's scaled accumulation, every operation rounded
 // on its own.  The near/far switch `r0 > 7*radius` (Green_Rankine.f90:50,227)

@@ -22,6 +22,7 @@
 // row whose CTA is already running; waits are bounded and report a timeout.
 #include <algorithm>
 #include "dmma.cuh"
+#include "reciprocals.cuh"
 
 namespace bem {
 namespace {
@@ -61,25 +62,6 @@ struct DiagShared {
 
 __device__ __forceinline__ double2 shfl2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-// 1 / a, a != 0, by quotients of a scaled by the power of two of its larger part
-// (out of line: 1% of an 800-panel sweep, in line 2.5%).
-__device__ __noinline__ double2 cinv(double2 a) {
-  const int e = ilogb(fmax(fabs(a.x), fabs(a.y)));
-  const double x = scalbn(a.x, -e), y = scalbn(a.y, -e), n = x * x + y * y;
-  return make_double2(scalbn(x / n, -e), scalbn(-y / n, -e));
-}
-// The same without a branch where the square of the modulus is well inside the
-// range of float64: the hardware's estimate of the reciprocal and two steps of
-// Newton-Raphson for 1 / d, r + r (1 - d r).
-__device__ __forceinline__ double2 cinv_fast(double2 a, bool& in_range) {
-  const double d = a.x * a.x + a.y * a.y;
-  in_range = d > 1e-280 && d < 1e280;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
-  r = fma(r, fma(-d, r, 1.0), r);
-  return make_double2(a.x * r, -a.y * r);
 }
 __device__ __forceinline__ int nth_bit(unsigned long long m, int n) {
   for (; n > 0; --n) m &= m - 1;

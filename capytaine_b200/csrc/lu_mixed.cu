@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 #include "common.cuh"
+#include "reciprocals.cuh"
 
 namespace bem {
 
@@ -187,30 +188,6 @@ __device__ __forceinline__ bool gj_wait(uint64_t* bar, uint32_t parity, GjShared
 __device__ __forceinline__ unsigned gj_key(float re, float im, int row, unsigned left) {
   const float m = fmaxf(fabsf(re) + fabsf(im), 0.0f);
   return (((__float_as_uint(m) + 128u) & ~127u) | (unsigned)(127 - row)) & left;
-}
-
-// 1 / (re + i im) for any pivot: where the square of its modulus is far inside
-// the range of float32, conj(pivot) times the hardware's estimate of 1 / d
-// (rcp.approx, which flushes) and one step of Newton-Raphson for 1 / d,
-// r + r (1 - d r); elsewhere quotients of the pivot scaled by the power of two of
-// its larger part (out of line: the range costs 2 us per block, in line 3).  0 for a
-// zero pivot, infinite for one below 2^-128.
-__device__ __noinline__ float2 gj_reciprocal_scaled(float re, float im) {
-  const float m = fmaxf(fabsf(re), fabsf(im));
-  if (!(m > 0.0f)) return make_float2(0.0f, 0.0f);
-  const int e = ilogbf(m);
-  const float x = scalbnf(re, -e), y = scalbnf(im, -e), n = x * x + y * y;
-  return make_float2(scalbnf(x / n, -e), scalbnf(-y / n, -e));
-}
-__device__ __forceinline__ float2 gj_reciprocal(float re, float im) {
-  const float d = re * re + im * im;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(r, fmaf(-d, r, 1.0f), r);
-  float2 out = make_float2(re * r, -im * r);
-  // the pivot is the same in every lane: no divergence
-  if (!(d > 0x1p-100f && d < 0x1p100f)) out = gj_reciprocal_scaled(re, im);
-  return out;
 }
 
 // A warp's columns in registers: [pair of rows][column], planes apart.

@@ -378,6 +378,12 @@ int bem_clu_factor_planes(int n, int npad, int batch, int* piv_dev, int* info_de
 int bem_clu_solve(void* work_dev, int npad, int batch, const int* piv_dev, void* B_dev, int64_t ldb,
                   int64_t strideB, int nrhs, int* err_dev, void* stream);
 
+/* No counterpart in the reference: a test of the refined reciprocals of the
+ * kernels over n values.  kind 0: out[i] = 1 / sqrt(in[i]) in float64 (positive
+ * normal values); 1 and 2: complex values (2 n doubles), 1 / in[i] in float64 and in
+ * float32. */
+int bem_reciprocals(int kind, int64_t n, const double* in_dev, double* out_dev, void* stream);
+
 /* No counterpart in the reference: a test of the bounded waits.  bem_clu_solve
  * with the iteration limit of the flag waits of its block substitutions given
  * (spin_limit > 0 polls of ~64 ns; bem_clu_solve uses 4e6) and, when
