@@ -58,7 +58,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     nvcc = _nvcc()
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    headers = [h for d, p in ((CSRC, "*.cuh"), (CSRC, "*.h"), (os.path.join(ROOT, "include"), "*.h"))
+               for h in glob.glob(os.path.join(d, p))]
     extra = _cutlass_include()
     jobs = []
     objs = []

@@ -5,6 +5,7 @@
 #include <cstdio>
 
 #include "../../include/capytaine_b200.h"
+#include "per_device.h"
 
 namespace bem {
 
@@ -147,3 +148,13 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
     cudaError_t _e = (call);                                  \
     if (_e != cudaSuccess) return bem::set_cuda_error(_e, #call); \
   } while (0)
+
+namespace bem {
+// configure() once on the current device (see OncePerDevice).
+template <class Configure>
+int configure_device(OncePerDevice& once, Configure&& configure) {
+  int dev = 0;
+  BEM_CUDA_CHECK(cudaGetDevice(&dev));
+  return once(dev, configure);
+}
+}  // namespace bem

@@ -831,9 +831,7 @@ int check_lu_args(const void* A, int n, int64_t lda, int batch) {
   if (batch <= 0) return set_error(BEM_ERR_INVALID_ARGUMENT, "batch <= 0");
   return BEM_OK;
 }
-bool g_smem_configured = false;
-int configure_smem() {
-  if (g_smem_configured) return BEM_OK;
+int opt_in_smem() {
   BEM_CUDA_CHECK(cudaFuncSetAttribute(zlu_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
   BEM_CUDA_CHECK(
       cudaFuncSetAttribute(zgemm_dmma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
@@ -846,9 +844,10 @@ int configure_smem() {
       cudaFuncSetAttribute(ztrsm_persistent_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem(8)));
   BEM_CUDA_CHECK(
       cudaFuncSetAttribute(ztrsm_persistent_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem(16)));
-  g_smem_configured = true;
   return BEM_OK;
 }
+OncePerDevice g_smem;
+int configure_smem() { return configure_device(g_smem, opt_in_smem); }
 }  // namespace
 
 extern "C" int bem_zpad_identity(void* A_dev, int64_t lda, int64_t stride, int batch, int n, int npad, void* stream) {

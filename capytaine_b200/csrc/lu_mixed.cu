@@ -946,9 +946,7 @@ __global__ void refine_check_kernel(const double* __restrict__ bn, const double*
   }
 }
 
-bool g_mixed_configured = false;
-int configure_mixed() {
-  if (g_mixed_configured) return BEM_OK;
+int opt_in_mixed() {
   BEM_CUDA_CHECK(cudaFuncSetAttribute(clu_gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmem));
   BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       trsm_smem_bytes(8)));
@@ -956,9 +954,10 @@ int configure_mixed() {
                                       trsm_smem_bytes(8)));
   BEM_CUDA_CHECK(cudaFuncSetAttribute(ctrsm_persistent_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       trsm_smem_bytes(16)));
-  g_mixed_configured = true;
   return BEM_OK;
 }
+OncePerDevice g_mixed;
+int configure_mixed() { return configure_device(g_mixed, opt_in_mixed); }
 
 // Streaming multiprocessors of the current device (cached per device).
 int sm_count(int* out) {

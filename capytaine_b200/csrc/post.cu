@@ -302,14 +302,15 @@ int zgemm_ts_enqueue(int M, int K, int nrhs, double alpha_re, double alpha_im, c
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_zgemm_ts: bad arguments (nrhs must be <= 16)");
   const int nsplit = ts_nsplit(M, K, batch), kchunk = ceil_div(K, nsplit);
   cudaStream_t s = (cudaStream_t)stream;
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice once;
+  const int st = configure_device(once, [] {
     BEM_CUDA_CHECK(
         cudaFuncSetAttribute(zgemm_ts_partial_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmem));
     BEM_CUDA_CHECK(
         cudaFuncSetAttribute(zgemm_ts_partial_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsSmem));
-    configured = true;
-  }
+    return BEM_OK;
+  });
+  if (st) return st;
   TimedLaunch tl(kKZgemmTs, s);
   auto* kernel = nrhs <= 8 ? zgemm_ts_partial_kernel<1> : zgemm_ts_partial_kernel<2>;
   kernel<<<dim3(ceil_div(M, kTsRows), nsplit, batch), 256, kTsSmem, s>>>(

@@ -484,7 +484,7 @@ int make_operand_map(CUtensorMap* map, const float* base, int kp, int64_t rows, 
   return BEM_OK;
 }
 
-bool g_tc_configured = false;
+OncePerDevice g_tc;
 int g_num_sms[64] = {0};
 
 int num_sms(int* out) {
@@ -530,10 +530,11 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
   st = make_operand_map(&mapB1, Bop1 ? Bop1 : Bop, depth.kb, b_rows, batch, kTN);
   if (st) return st;
   const int smem = kStages * kStageBytes + 1024 + 256;
-  if (!g_tc_configured) {
+  st = configure_device(g_tc, [&] {
     BEM_CUDA_CHECK(cudaFuncSetAttribute(cgemm_tf32_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    g_tc_configured = true;
-  }
+    return BEM_OK;
+  });
+  if (st) return st;
   int sms = 0;
   if ((st = num_sms(&sms))) return st;
   const int nseg = Aop1 ? 2 : depth.nseg;
