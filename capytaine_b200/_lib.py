@@ -25,6 +25,7 @@ BEM_ERR_UNSUPPORTED = 7
 BEM_ERR_TIMEOUT = 8
 
 BEM_GRID_LEGACY, BEM_GRID_SCALED_NEMOH3 = 0, 1
+BEM_GRID_PACKED_TABLE = 256  # or-ed to the grid shape: packed_table_dev is set
 BEM_GF_HIGH_FREQ, BEM_GF_LOW_FREQ, BEM_GF_LOW_FREQ_WITH_RANKINE_PART = 0, 1, 2
 BEM_DTYPE_C128, BEM_DTYPE_C64 = 0, 1
 BEM_PREC_FP64, BEM_PREC_MIXED = 0, 1

@@ -21,6 +21,8 @@
 // O(k)-small imaginary part of the source strengths (radiation damping at low
 // frequency) beyond 1e-5 relative.
 #include <cmath>
+#include <cstddef>
+#include <cstring>
 #include "integrals.cuh"
 #include "packed_table.cuh"
 #include "reciprocals.cuh"
@@ -1583,12 +1585,22 @@ int launch_entries(const bem_assembly_args& a, EntryParams e, const TabView& T, 
   return BEM_OK;
 }
 
+// The caller's struct without what it does not have: a program built before
+// packed_table_dev was appended passes a shorter one, without the flag.
+bem_assembly_args read_args(const bem_assembly_args& caller) {
+  bem_assembly_args a{};
+  std::memcpy(&a, &caller, offsetof(bem_assembly_args, packed_table_dev));
+  if (a.tabulation_grid_shape & BEM_GRID_PACKED_TABLE) a.packed_table_dev = caller.packed_table_dev;
+  return a;
+}
+int grid_shape(const bem_assembly_args& a) { return a.tabulation_grid_shape & ~BEM_GRID_PACKED_TABLE; }
+
 PackedTab packed_tab(const bem_assembly_args& a) {
   PackedTab P{};
   P.base = a.nr > 2 && a.nz > 2 ? a.packed_table_dev : nullptr;
   P.nr = a.nr;
   P.nz = a.nz;
-  P.grid = a.tabulation_grid_shape;
+  P.grid = grid_shape(a);
   return P;
 }
 
@@ -1598,7 +1610,7 @@ PackedTab packed_tab(const bem_assembly_args& a) {
 extern "C" int bem_assemble(const bem_assembly_args* args, void* stream) {
   using namespace bem;
   if (!args) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble: null args");
-  const bem_assembly_args& a = *args;
+  const bem_assembly_args a = read_args(*args);
   if (a.n < 0 || a.nb_faces < 0) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble: negative size");
   if (a.n == 0 || a.nb_faces == 0) return BEM_OK;
   if (!a.points_dev || !a.vertices_dev || !a.faces_dev || !a.centers_dev || !a.normals_dev || !a.areas_dev ||
@@ -1621,7 +1633,7 @@ extern "C" int bem_assemble(const bem_assembly_args* args, void* stream) {
     if (a.precision == BEM_PREC_MIXED && tabulated && !a.table32_dev)
       return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble: mixed precision needs the float32 table");
   }
-  const TabView T{a.tabulation_nb_integration_points, a.tabulation_grid_shape, a.nr, a.nz, a.r_range_dev,
+  const TabView T{a.tabulation_nb_integration_points, grid_shape(a), a.nr, a.nz, a.r_range_dev,
                   a.z_range_dev, a.table_dev, a.table32_dev, 0.0, 0.0, a.r_inv_den_dev, a.z_inv_den_dev, 0.0};
   int gf_sing = a.gf_singularities;
   // Singularity variant overrides of delhommeau.py:472-487.
@@ -1681,7 +1693,7 @@ int check_common(const bem_assembly_args& a, const char* who) {
 extern "C" int bem_assemble_rankine_part(const bem_assembly_args* args, void* out_dev, int64_t ld, void* stream) {
   using namespace bem;
   if (!args || !out_dev) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_rankine_part: null pointer");
-  const bem_assembly_args& a = *args;
+  const bem_assembly_args a = read_args(*args);
   int st = check_common(a, "bem_assemble_rankine_part");
   if (st) return st;
   if (ld < a.n) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_rankine_part: ld < n");
@@ -1716,7 +1728,7 @@ int wave_symmetric_launch(const bem_assembly_args* args, const void* rankine_dev
     std::snprintf(msg, sizeof(msg), "%s: null pointer or no wavenumber", who);
     return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
   }
-  const bem_assembly_args& a = *args;
+  const bem_assembly_args a = read_args(*args);
   int st = check_common(a, who);
   if (st) return st;
   if (!a.S_dev || !a.K_dev) {
@@ -1771,7 +1783,7 @@ int wave_symmetric_launch(const bem_assembly_args* args, const void* rankine_dev
     std::snprintf(msg, sizeof(msg), "%s: mixed precision needs table32_dev", who);
     return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
   }
-  const TabView T{a.tabulation_nb_integration_points, a.tabulation_grid_shape, a.nr, a.nz, a.r_range_dev,
+  const TabView T{a.tabulation_nb_integration_points, grid_shape(a), a.nr, a.nz, a.r_range_dev,
                   a.z_range_dev, a.table_dev, a.table32_dev, 0.0, 0.0, a.r_inv_den_dev, a.z_inv_den_dev, 0.0};
   const int nbi = ceil_div(a.n, kSymT), nbj = ceil_div(general ? a.nb_faces : a.n, kSymT);
   cudaStream_t s = (cudaStream_t)stream;
@@ -1878,7 +1890,7 @@ extern "C" int bem_assemble_wave_cached(const bem_assembly_args* args, const voi
 extern "C" int bem_assemble_symmetric(const bem_assembly_args* args, void* stream) {
   using namespace bem;
   if (!args || !args->K_dev) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_symmetric: null pointer");
-  const bem_assembly_args& a = *args;
+  const bem_assembly_args a = read_args(*args);
   if (a.n != a.nb_faces || a.nb_quad_points != 1 || a.points_dev != a.quad_points_dev ||
       a.centers_dev != a.quad_points_dev)
     return set_error(BEM_ERR_INVALID_ARGUMENT,
@@ -1899,7 +1911,7 @@ extern "C" int bem_assemble_finite_depth(const bem_assembly_args* args, double d
                                          const double* prony_dev, int nexp, void* stream) {
   using namespace bem;
   if (!args) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: null args");
-  const bem_assembly_args& a = *args;
+  const bem_assembly_args a = read_args(*args);
   if (a.n < 0 || a.nb_faces < 0) return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: negative size");
   if (a.n == 0 || a.nb_faces == 0) return BEM_OK;
   if (!a.points_dev || !a.vertices_dev || !a.faces_dev || !a.centers_dev || !a.normals_dev || !a.areas_dev ||
@@ -1929,7 +1941,7 @@ extern "C" int bem_assemble_finite_depth(const bem_assembly_args* args, double d
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: tabulation pointers missing");
   if (finite_k && !tabulated && a.tabulation_nb_integration_points <= 0)
     return set_error(BEM_ERR_INVALID_ARGUMENT, "bem_assemble_finite_depth: nb_integration_points <= 0");
-  const TabView T{a.tabulation_nb_integration_points, a.tabulation_grid_shape, a.nr, a.nz, a.r_range_dev,
+  const TabView T{a.tabulation_nb_integration_points, grid_shape(a), a.nr, a.nz, a.r_range_dev,
                   a.z_range_dev, a.table_dev, a.table32_dev, 0.0, 0.0, a.r_inv_den_dev, a.z_inv_den_dev, 0.0};
   // the caller picks the variant (delhommeau.py:467-487: the legacy method
   // takes low_freq before the wavenumber rules apply)

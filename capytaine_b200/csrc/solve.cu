@@ -158,7 +158,10 @@ bem_assembly_args base_args(const bem_context* ctx, int n, const double* centers
   a.z_range_dev = ctx->z_dev;
   a.table_dev = ctx->table_dev;
   a.table32_dev = nullptr;
-  a.packed_table_dev = ctx->table_dev ? ctx->packed_dev : nullptr;
+  if (ctx->table_dev && ctx->packed_dev) {
+    a.packed_table_dev = ctx->packed_dev;
+    a.tabulation_grid_shape |= BEM_GRID_PACKED_TABLE;
+  }
   a.wavenumber = 1.0;
   a.free_surface = 0.0;
   a.gf_singularities = variant;

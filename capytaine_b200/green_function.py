@@ -302,6 +302,11 @@ class Delhommeau:
         return (self.tabulation_nb_integration_points, self.tabulation_grid_shape_index,
                 self.tabulated_r_range, self.tabulated_z_range, self.tabulated_integrals)
 
+    def _grid_shape_flags(self, table):
+        """The grid's shape, with the flag of the packed table where a call passes one."""
+        packed = table is not None and self._dev_tab_packed
+        return self.tabulation_grid_shape_index | (_lib.BEM_GRID_PACKED_TABLE if packed else 0)
+
     # ---- meshes -------------------------------------------------------------
     def device_mesh(self, mesh) -> DeviceMesh:
         key = mesh.content_hash
@@ -411,7 +416,7 @@ class Delhommeau:
             areas_dev=dm2.areas.data_ptr(), radii_dev=dm2.radii.data_ptr(), nb_quad_points=dm2.nb_quad_points,
             quad_points_dev=dm2.quad_points.data_ptr(), quad_weights_dev=dm2.quad_weights.data_ptr(),
             tabulation_nb_integration_points=self.tabulation_nb_integration_points,
-            tabulation_grid_shape=self.tabulation_grid_shape_index, nr=nr if nr > 1 and nz > 1 else 0,
+            tabulation_grid_shape=self._grid_shape_flags(table), nr=nr if nr > 1 and nz > 1 else 0,
             nz=nz if nr > 1 and nz > 1 else 0,
             r_range_dev=r.data_ptr() if r is not None else 0, z_range_dev=z.data_ptr() if z is not None else 0,
             table_dev=table.data_ptr() if table is not None else 0,
@@ -569,7 +574,7 @@ class Delhommeau:
             areas_dev=dm2.areas.data_ptr(), radii_dev=dm2.radii.data_ptr(), nb_quad_points=dm2.nb_quad_points,
             quad_points_dev=dm2.quad_points.data_ptr(), quad_weights_dev=dm2.quad_weights.data_ptr(),
             tabulation_nb_integration_points=self.tabulation_nb_integration_points,
-            tabulation_grid_shape=self.tabulation_grid_shape_index, nr=nr if nr > 1 and nz > 1 else 0,
+            tabulation_grid_shape=self._grid_shape_flags(table), nr=nr if nr > 1 and nz > 1 else 0,
             nz=nz if nr > 1 and nz > 1 else 0,
             r_range_dev=r.data_ptr() if r is not None else 0, z_range_dev=z.data_ptr() if z is not None else 0,
             table_dev=table.data_ptr() if table is not None else 0,

@@ -37,6 +37,8 @@ extern "C" {
 /* ---- enums (values of libDelhommeau constants.f90:40-52) ------------------ */
 #define BEM_GRID_LEGACY 0
 #define BEM_GRID_SCALED_NEMOH3 1
+/* or-ed to bem_assembly_args' tabulation_grid_shape: packed_table_dev is set */
+#define BEM_GRID_PACKED_TABLE 256
 #define BEM_GF_HIGH_FREQ 0
 #define BEM_GF_LOW_FREQ 1
 #define BEM_GF_LOW_FREQ_WITH_RANKINE_PART 2
@@ -146,8 +148,10 @@ typedef struct {
    * (3 per node, bem_tabulation_inverse_denominators); NULL: divided each time */
   const double* r_inv_den_dev;     /* (nr, 3)                                                  */
   const double* z_inv_den_dev;     /* (nz, 3)                                                  */
-  /* optional: the table packed by bem_pack_table from the same grids and table
-   * (32-byte aligned); NULL: the wave term reads the plain table              */
+  /* optional, read with BEM_GRID_PACKED_TABLE only (so that a struct without this
+   * member may be passed): the table packed by bem_pack_table from the same grids
+   * and table (32-byte aligned); NULL or no flag: the wave term reads the plain
+   * table                                                                     */
   const double* packed_table_dev;
 } bem_assembly_args;
 
