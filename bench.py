@@ -473,14 +473,14 @@ def run_profile_case(case):
         return K, wv, piv
 
     if case == "gemm":
-        m, kp, batch = 4480, 512, 2
-        Aop = torch.randn((batch, m, kp), device="cuda", dtype=torch.float32)
-        Bop = torch.randn((batch, 2 * m, kp), device="cuda", dtype=torch.float32)
+        m, k, batch = 4480, 256, 2
+        Aop = torch.randn((batch, m, 2 * k), device="cuda", dtype=torch.float32)
+        Bop = torch.randn((batch, 2 * m, k), device="cuda", dtype=torch.float32)
         Cr = torch.randn((batch, m, m), device="cuda", dtype=torch.float32)
         Ci = torch.randn((batch, m, m), device="cuda", dtype=torch.float32)
         for _ in range(3):
-            _lib.check(lib.bem_cgemm_tf32_update(vp(Aop), m, 0, vp(Bop), 2 * m, 0, kp, vp(Cr), vp(Ci), m, m * m,
-                                                 0, 0, m, m, batch, vp(err), s))
+            _lib.check(lib.bem_cgemm_tf32_parts(vp(Aop), m, 0, vp(Bop), 2 * m, 0, k, vp(Cr), vp(Ci), m, m * m,
+                                                0, 0, m, m, batch, vp(err), s))
     elif case == "gj":
         for _ in range(2):
             factor(1024, 2)
@@ -624,19 +624,19 @@ def isolated_update_rate(n, batch):
     from capytaine_b200 import _lib
     lib = _lib.load()
     npad = -(-n // 128) * 128
-    m, kp = npad - 256, 512
+    m, k = npad - 256, 256
     vp = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
     g = torch.Generator(device="cuda").manual_seed(3)
-    Aop = torch.randn((batch, m, kp), device="cuda", dtype=torch.float32, generator=g)
-    Bop = torch.randn((batch, 2 * m, kp), device="cuda", dtype=torch.float32, generator=g)
+    Aop = torch.randn((batch, m, 2 * k), device="cuda", dtype=torch.float32, generator=g)
+    Bop = torch.randn((batch, 2 * m, k), device="cuda", dtype=torch.float32, generator=g)
     Cr = torch.zeros((batch, m, m), device="cuda", dtype=torch.float32)
     Ci = torch.zeros((batch, m, m), device="cuda", dtype=torch.float32)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     s = _lib.stream_ptr()
 
     def launch():
-        _lib.check(lib.bem_cgemm_tf32_update(vp(Aop), m, 0, vp(Bop), 2 * m, 0, kp, vp(Cr), vp(Ci), m, m * m,
-                                             0, 0, m, m, batch, vp(err), s))
+        _lib.check(lib.bem_cgemm_tf32_parts(vp(Aop), m, 0, vp(Bop), 2 * m, 0, k, vp(Cr), vp(Ci), m, m * m,
+                                            0, 0, m, m, batch, vp(err), s))
     for _ in range(2):
         launch()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -649,7 +649,7 @@ def isolated_update_rate(n, batch):
     if int(err.item()) != 0:
         raise RuntimeError("isolated update: kernel error flag set")
     ms = e0.elapsed_time(e1) / 5
-    flops = 8.0 * m * m * 256 * batch
+    flops = 8.0 * m * m * k * batch
     del Aop, Bop, Cr, Ci
     return {"m": m, "depth": 256, "batch": batch, "ms_per_launch": ms, "achieved": flops / (ms * 1e-3) / 1e12,
             "unit": "TFLOP/s"}

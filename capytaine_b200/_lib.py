@@ -132,6 +132,8 @@ _SIGNATURES = {
     "bem_reciprocals": ([c_int, c_i64, c_void_p, c_void_p, c_void_p], c_int),
     "bem_cgemm_tf32_update": ([c_void_p, c_i64, c_int, c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p, c_i64,
                                c_i64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
+    "bem_cgemm_tf32_parts": ([c_void_p, c_i64, c_int, c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p, c_i64,
+                              c_i64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "bem_clu_workspace_bytes": ([c_int, c_int], c_i64),
     "bem_clu_factor": ([c_void_p, c_i64, c_i64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_void_p], c_int),

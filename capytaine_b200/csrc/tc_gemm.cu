@@ -9,8 +9,8 @@
 //   Bop[b][r][:]      per group of 128 complex output columns j0..j0+127, rows
 //                     2*j0 + t   (t < 128): Re B(:, j0+t)
 //                     2*j0 + 128 + t     : Im B(:, j0+t)
-// (the public entry point's B operand is the real embedding, whose rows begin with
-// these parts; see CgemmDepth).
+// (bem_cgemm_tf32_update takes the real embedding of B instead, as any real rows:
+// embedded in CgemmDepth).
 // A CTA owns 128 x 128 complex tiles of C (accumulator 128 lanes x 256 fp32
 // columns: real parts then imaginary parts).  Warp 0 streams operand slices with
 // TMA (128-byte swizzle) through a three-stage shared-memory ring, 32 values of
@@ -622,20 +622,47 @@ int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float*
 
 }  // namespace bem
 
+namespace bem {
+namespace {
+int check_update(const char* who, const float* Aop, int64_t a_rows, int a_row0, const float* Bop, int64_t b_rows,
+                 int b_row0, int k, const float* Cr, const float* Ci, int64_t ldc, int c_row0, int m, int n, int batch,
+                 const int* err) {
+  char msg[120];
+  const char* what = nullptr;
+  if (!Aop || !Bop || !Cr || !Ci || !err || batch <= 0 || ldc < c_row0 + m || k <= 0) what = "bad arguments";
+  else if ((int64_t)a_row0 + m > a_rows || (int64_t)b_row0 + 2 * (int64_t)n > b_rows) what = "operand rows out of range";
+  else if ((reinterpret_cast<uintptr_t>(Aop) | reinterpret_cast<uintptr_t>(Bop)) & 15)
+    what = "operands must be 16-byte aligned";
+  if (!what) return BEM_OK;
+  std::snprintf(msg, sizeof(msg), "%s: %s", who, what);
+  return set_error(BEM_ERR_INVALID_ARGUMENT, msg);
+}
+}  // namespace
+}  // namespace bem
+
+// The rows of B taken whole, whatever they hold (the real embedding for a complex
+// product): nothing of their structure is assumed.
 extern "C" int bem_cgemm_tf32_update(const float* Aop_dev, int64_t a_rows, int a_row0, const float* Bop_dev,
                                      int64_t b_rows, int b_row0, int kp, float* Cr_dev, float* Ci_dev, int64_t ldc,
                                      int64_t c_stride, int c_row0, int c_col0, int m, int n, int batch, int* err_dev,
                                      void* stream) {
-  if (!Aop_dev || !Bop_dev || !Cr_dev || !Ci_dev || !err_dev || batch <= 0 || ldc < c_row0 + m || kp <= 0)
-    return bem::set_error(BEM_ERR_INVALID_ARGUMENT, "bem_cgemm_tf32_update: bad arguments");
-  if ((int64_t)a_row0 + m > a_rows || (int64_t)b_row0 + 2 * (int64_t)n > b_rows)
-    return bem::set_error(BEM_ERR_INVALID_ARGUMENT, "bem_cgemm_tf32_update: operand rows out of range");
-  if ((reinterpret_cast<uintptr_t>(Aop_dev) | reinterpret_cast<uintptr_t>(Bop_dev)) & 15)
-    return bem::set_error(BEM_ERR_INVALID_ARGUMENT, "bem_cgemm_tf32_update: operands must be 16-byte aligned");
-  // K' = 2k: the rows of B begin with Re B and Im B; an odd number of 16-deep
-  // steps (K' not a multiple of 64) takes the embedding as it stands
-  const bem::CgemmDepth depth = kp % 64 == 0 ? bem::CgemmDepth{kp / 2, kp, kp, 1, kp / 2, 0, {0, 0, 0}, false}
-                                             : bem::CgemmDepth{kp, kp, kp, 1, 0, 0, {0, 0, 0}, true};
+  const int st = bem::check_update("bem_cgemm_tf32_update", Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, kp, Cr_dev,
+                                   Ci_dev, ldc, c_row0, m, n, batch, err_dev);
+  if (st) return st;
+  const bem::CgemmDepth depth{kp, kp, kp, 1, 0, 0, {0, 0, 0}, true};
+  return bem::cgemm_tf32_update(Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, depth, Cr_dev, Ci_dev, ldc, c_stride,
+                                c_row0, c_col0, m, n, batch, err_dev, (cudaStream_t)stream, 0, nullptr, nullptr, 0, 0,
+                                nullptr, nullptr, bem::kPackNone, 0, bem::kTilesAll, 0);
+}
+
+extern "C" int bem_cgemm_tf32_parts(const float* Aop_dev, int64_t a_rows, int a_row0, const float* Bop_dev,
+                                    int64_t b_rows, int b_row0, int k, float* Cr_dev, float* Ci_dev, int64_t ldc,
+                                    int64_t c_stride, int c_row0, int c_col0, int m, int n, int batch, int* err_dev,
+                                    void* stream) {
+  const int st = bem::check_update("bem_cgemm_tf32_parts", Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, k, Cr_dev,
+                                   Ci_dev, ldc, c_row0, m, n, batch, err_dev);
+  if (st) return st;
+  const bem::CgemmDepth depth{k, 2 * k, k, 1, k, 0, {0, 0, 0}, false};
   return bem::cgemm_tf32_update(Aop_dev, a_rows, a_row0, Bop_dev, b_rows, b_row0, depth, Cr_dev, Ci_dev, ldc, c_stride,
                                 c_row0, c_col0, m, n, batch, err_dev, (cudaStream_t)stream, 0, nullptr, nullptr, 0, 0,
                                 nullptr, nullptr, bem::kPackNone, 0, bem::kTilesAll, 0);

@@ -333,12 +333,22 @@ int bem_froude_krylov(int n, int batch, int ndof, int nhead, const double* waven
  *   Aop[b][a_row0 + i][:] = [Re A(i, :), Im A(i, :)]
  *   Bop[b][b_row0 + 2*j0 + t][:]       = [Re B(:, j0+t); -Im B(:, j0+t)]
  *   Bop[b][b_row0 + 2*j0 + 128 + t][:] = [Im B(:, j0+t);  Re B(:, j0+t)]
- * for each group of 128 columns j0 and t < 128.  err_dev is set to 1 when a
- * bounded wait inside the kernel gave up.  This is the trailing update of the
- * mixed-precision LU that replaces zgetrf's (tools/block_circulant_matrices.py:378). */
+ * for each group of 128 columns j0 and t < 128 (other real rows are taken as they
+ * are: Cr and Ci lose the products of Aop with the group's first and last 128).
+ * err_dev is set to 1 when a bounded wait inside the kernel gave up. */
 int bem_cgemm_tf32_update(const float* Aop_dev, int64_t a_rows, int a_row0, const float* Bop_dev, int64_t b_rows,
                           int b_row0, int kp, float* Cr_dev, float* Ci_dev, int64_t ldc, int64_t c_stride,
                           int c_row0, int c_col0, int m, int n, int batch, int* err_dev, void* stream);
+
+/* The same product from B's parts, each stored once (k a multiple of 32):
+ *   Aop[b][a_row0 + i][:] = [Re A(i, :), Im A(i, :)]  (2k values)
+ *   Bop[b][b_row0 + 2*j0 + t][:]       = Re B(:, j0+t)  (k values)
+ *   Bop[b][b_row0 + 2*j0 + 128 + t][:] = Im B(:, j0+t)
+ * This is the trailing update of the mixed-precision LU that replaces zgetrf's
+ * (tools/block_circulant_matrices.py:378). */
+int bem_cgemm_tf32_parts(const float* Aop_dev, int64_t a_rows, int a_row0, const float* Bop_dev, int64_t b_rows,
+                         int b_row0, int k, float* Cr_dev, float* Ci_dev, int64_t ldc, int64_t c_stride,
+                         int c_row0, int c_col0, int m, int n, int batch, int* err_dev, void* stream);
 
 /* ---- mixed-precision solve ------------------------------------------------- */
 /* Workspace of bem_clu_factor / bem_clu_solve (float32 planes of K, packed

@@ -64,3 +64,42 @@ def test_cgemm_tf32_update(m, n, k, batch):
         assert np.max(np.abs(got - ref) / (scale + 1e-30)) < 2e-3
         # entries outside the block are untouched
         assert float(Cr[b, :c0].abs().max()) == 0.0 and float(Cr[b, c0:, :r0].abs().max()) == 0.0
+
+
+def _operands(torch, m, n, ka, kb, batch):
+    rng = np.random.default_rng(m + n + ka)
+    host = [rng.standard_normal(s).astype(np.float32)
+            for s in ((batch, m, ka), (batch, 2 * n, kb), (batch, n, m), (batch, n, m))]
+    return host, [torch.as_tensor(a, device="cuda") for a in host], torch.zeros(1, dtype=torch.int32, device="cuda")
+
+
+# K' of an odd and of an even number of 32-deep stages
+@pytest.mark.parametrize("m,n,kp", [(128, 128, 32), (256, 128, 64), (128, 256, 256)])
+def test_cgemm_tf32_update_takes_any_real_rows(m, n, kp):
+    import torch
+    (A, B, Cr, Ci), (Ad, Bd, Crd, Cid), err = _operands(torch, m, n, kp, kp, 2)
+    _lib.check(_lib.load().bem_cgemm_tf32_update(_vp(Ad), m, 0, _vp(Bd), 2 * n, 0, kp, _vp(Crd), _vp(Cid), m, n * m, 0,
+                                                 0, m, n, 2, _vp(err), _lib.stream_ptr()))
+    assert int(err.item()) == 0
+    for b in range(2):
+        rows = B[b].reshape(n // 128, 2, 128, kp).astype(float)
+        for got, C, part in ((Crd, Cr, 0), (Cid, Ci, 1)):
+            right = rows[:, part].reshape(n, kp)
+            scale = np.abs(right) @ np.abs(A[b].T.astype(float))
+            assert np.max(np.abs(got[b].cpu().numpy() - (C[b] - right @ A[b].T.astype(float))) / scale) < 2e-3
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(128, 128, 32, 1), (256, 384, 64, 2), (2048, 2048, 96, 2)])
+def test_cgemm_tf32_parts(m, n, k, batch):
+    import torch
+    (A, B, Cr, Ci), (Ad, Bd, Crd, Cid), err = _operands(torch, m, n, 2 * k, k, batch)
+    _lib.check(_lib.load().bem_cgemm_tf32_parts(_vp(Ad), m, 0, _vp(Bd), 2 * n, 0, k, _vp(Crd), _vp(Cid), m, n * m, 0, 0,
+                                                m, n, batch, _vp(err), _lib.stream_ptr()))
+    assert int(err.item()) == 0
+    for b in range(batch):
+        rows = B[b].reshape(n // 128, 2, 128, k).astype(float)
+        left = A[b][:, :k].astype(float) + 1j * A[b][:, k:]
+        right = (rows[:, 0] + 1j * rows[:, 1]).reshape(n, k)
+        want = (Cr[b] + 1j * Ci[b]) - right @ left.T
+        got = Crd[b].cpu().numpy() + 1j * Cid[b].cpu().numpy()
+        assert np.max(np.abs(got - want) / (np.abs(right) @ np.abs(left.T))) < 2e-3
