@@ -73,3 +73,41 @@ def test_factors_at_every_scale(scale):
     X = Bt.cpu().numpy().T * scale  # X of the unscaled matrix
     want = np.linalg.solve(A / scale, B)
     assert np.abs(X - want).max() < 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("nrhs", [1, 4, 5, 8, 9, 15, 16, 17])
+def test_solves_at_the_edges_of_the_column_groups(nrhs):
+    # 13 block rows: long chains in both sweeps; the last block row is mostly padding
+    import torch
+    lib = _lib.load()
+    rng = np.random.default_rng(nrhs)
+    n, npad, batch = 773, 832, 3
+    mats = [rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3 * np.sqrt(n) * np.eye(n)
+            for _ in range(batch)]
+    B = rng.standard_normal((batch, n, nrhs)) + 1j * rng.standard_normal((batch, n, nrhs))
+    A = torch.zeros((batch, npad, npad), dtype=torch.complex128, device="cuda")
+    A[:, :n, :n] = torch.as_tensor(np.array([m.T for m in mats]))
+    s = _lib.stream_ptr()
+    _lib.check(lib.bem_zpad_identity(_vp(A), npad, npad * npad, batch, n, npad, s))
+    piv = torch.empty((batch, npad), dtype=torch.int32, device="cuda")
+    info = torch.zeros(batch, dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(lib.bem_zlu_workspace_bytes(npad, batch)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.bem_zlu_factor(_vp(A), npad, npad, npad * npad, batch, _vp(piv), _vp(info), _vp(work), s))
+
+    def solve(columns):
+        nc = columns.shape[2]
+        X = torch.zeros((batch, nc, npad), dtype=torch.complex128, device="cuda")
+        X[:, :, :n] = torch.as_tensor(np.ascontiguousarray(columns.transpose(0, 2, 1)))
+        _lib.check(lib.bem_zlu_solve(_vp(A), npad, npad, npad * npad, batch, _vp(piv), _vp(work), _vp(X), npad,
+                                     npad * nc, nc, _vp(err), s))
+        assert int(err.item()) == 0 and float(X[:, :, n:].abs().sum()) == 0.0
+        return X[:, :, :n].cpu().numpy().transpose(0, 2, 1)
+    X = solve(B)
+    assert info.cpu().numpy().tolist() == [0] * batch
+    for b in range(batch):
+        want = np.linalg.solve(mats[b], B[b])
+        # backward error below 1e-12 (see above), condition below 10
+        assert np.abs(X[b] - want).max() < 1e-11 * np.abs(want).max()
+    one = solve(B[:, :, -1:])
+    assert np.abs(X[:, :, -1:] - one).max() < 1e-13 * np.abs(one).max()
