@@ -111,3 +111,29 @@ def test_solves_at_the_edges_of_the_column_groups(nrhs):
         assert np.abs(X[b] - want).max() < 1e-11 * np.abs(want).max()
     one = solve(B[:, :, -1:])
     assert np.abs(X[:, :, -1:] - one).max() < 1e-13 * np.abs(one).max()
+
+
+@pytest.mark.parametrize("weak", [1.0, 1e-2, 1e-4, 1e-6])
+@pytest.mark.parametrize("n", [128, 320])
+def test_factors_of_blocks_with_ill_conditioned_triangles(n, weak):
+    # a first block close to rank one: its triangles are ill-conditioned.  The entries
+    # of L U of an elimination are off by at most n u (|L| |U|) (Higham, Accuracy and
+    # Stability of Numerical Algorithms, theorem 9.3), and by sqrt(n) of that in place
+    # of n as the roundings' signs are random; products of the panels with the
+    # triangles' whole inverses add up to ten times as much.
+    import torch
+    lib = _lib.load()
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[:64, :64] = weak * A[:64, :64] + np.outer(rng.standard_normal(64), rng.standard_normal(64))
+    At = torch.as_tensor(np.ascontiguousarray(A.T), device="cuda")
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(lib.bem_zlu_workspace_bytes(n, 1)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.bem_zlu_factor(_vp(At), n, n, n * n, 1, _vp(piv), _vp(info), _vp(work), _lib.stream_ptr()))
+    lu, p = At.cpu().numpy().T, piv.cpu().numpy()
+    rows = np.concatenate([k + p[k:k + 64] for k in range(0, n, 64)])
+    L, U = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+    error = np.abs((L.astype(np.clongdouble) @ U - A[rows]).astype(complex))
+    ratio = (error / (np.abs(L) @ np.abs(U))).max() / (n * 2.0 ** -53)
+    assert ratio <= 1 / np.sqrt(n)
