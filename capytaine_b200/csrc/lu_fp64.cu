@@ -210,31 +210,30 @@ __device__ __forceinline__ void invert_upper16(double2* T, int base, int lane) {
 // rows j0 .. j0 + 7 of those columns, rows from first_row on only (a multiple of 8).
 __device__ __forceinline__ void panel_update_tile(double2* T, int j0, int m0, int n0, int first_row, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  double re[4], im[4];
+  double2 c[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const double2 c = T[(n0 + 2 * t + (e & 1)) * kLdD + m0 + g + 8 * (e >> 1)];
-    re[e] = c.x;
-    im[e] = c.y;
-  }
-  double ai[4], nr[4], ni[4];
+  for (int e = 0; e < 4; ++e) c[e] = T[(n0 + 2 * t + (e & 1)) * kLdD + m0 + g + 8 * (e >> 1)];
+  double ar[4], ai[4], ni[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const double2 v = T[(j0 + t + 4 * (e >> 1)) * kLdD + m0 + g + 8 * (e & 1)];
+    ar[e] = v.x;
     ai[e] = v.y;
-    nr[e] = -v.x;
     ni[e] = -v.y;
   }
   const double2 b0 = T[(n0 + g) * kLdD + j0 + t], b1 = T[(n0 + g) * kLdD + j0 + t + 4];
   const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
-  dmma(re, nr, br);
-  dmma(im, nr, bi);
-  dmma(re, ai, bi);
-  dmma(im, ni, br);
+  // the product on its own first: one rounding of the tile's size per entry
+  double re[4] = {}, im[4] = {};
+  dmma(re, ar, br);
+  dmma(im, ar, bi);
+  dmma(re, ni, bi);
+  dmma(im, ai, br);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int r = m0 + g + 8 * (e >> 1);
-    if (r >= first_row) T[(n0 + 2 * t + (e & 1)) * kLdD + r] = make_double2(re[e], im[e]);
+    if (r >= first_row)
+      T[(n0 + 2 * t + (e & 1)) * kLdD + r] = make_double2(c[e].x - re[e], c[e].y - im[e]);
   }
 }
 
@@ -574,29 +573,21 @@ __global__ void __launch_bounds__(256, 2)
   issue(0);
   issue(1);
   if (FACTOR) {
-    // C - A B as -(-C + A B): the accumulators start from the tile, so that
-    // its loads overlap the operands' (read one by one in the epilogue, behind
-    // stores that might alias, they took longer than the products)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const double2 c = C[(size_t)(m0 + wm + g + 8 * (e >> 1)) + (size_t)(n0 + wn + 8 * j + 2 * tt + (e & 1)) * ldc];
-        re[j][e] = -c.x;
-        im[j][e] = -c.y;
-      }
-    // meanwhile the tile of the CTA that follows in this place comes into L2: its loads
-    // are the only ones that otherwise wait for DRAM (2688 x 4: 9.66 -> 9.28 ms)
-    const int next = (int)blockIdx.x + kResident;
-    if (next >= batch && next < tiles * batch) {  // the first `batch` CTAs take the first tiles
-      const int tn = 1 + (next - batch) % (tiles - 1), bn = (next - batch) / (tiles - 1);
-      const double2* Cn = C + (int64_t)(bn - b) * strideC + (tn % tiles_m) * kTile +
-                          (int64_t)(tn / tiles_m) * kTile * ldc;
+    // this tile of C (the first CTAs') and the tile of the CTA that follows in this
+    // place come into L2 meanwhile: their loads are the only ones that otherwise wait
+    // for DRAM (2688 x 4: 9.66 -> 9.28 ms)
+    auto prefetch = [&](const double2* tile) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int line = tid + 256 * i;  // 8 lines of 128 bytes per column
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(Cn + 8 * (line & 7) + (int64_t)(line >> 3) * ldc));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + 8 * (line & 7) + (int64_t)(line >> 3) * ldc));
       }
+    };
+    if ((int)blockIdx.x < kResident) prefetch(C + m0 + (int64_t)n0 * ldc);
+    const int next = (int)blockIdx.x + kResident;
+    if (next >= batch && next < tiles * batch) {  // the first `batch` CTAs take the first tiles
+      const int tn = 1 + (next - batch) % (tiles - 1), bn = (next - batch) / (tiles - 1);
+      prefetch(C + (int64_t)(bn - b) * strideC + (tn % tiles_m) * kTile + (int64_t)(tn / tiles_m) * kTile * ldc);
     }
   }
 #pragma unroll 1
@@ -613,15 +604,28 @@ __global__ void __launch_bounds__(256, 2)
       cp_async_wait<0>();
       __syncthreads();  // the ring becomes the block
     }
+    // C - (the whole product): one rounding of C's size per entry (accumulators that
+    // start from C round to its size with every product).  The loads run a
+    // step ahead of the stores, which might alias them.
+    auto at = [&](int j, int e) {
+      return C + (size_t)(m0 + wm + g + 8 * (e >> 1)) + (size_t)(n0 + wn + 8 * j + 2 * tt + (e & 1)) * ldc;
+    };
+    double2 c[2][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int e = 0; e < 4; ++e) c[0][e] = *at(0, e);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j + 1 < 4) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[(j + 1) & 1][e] = *at(j + 1, e);
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int m = wm + g + 8 * (e >> 1), n = wn + 8 * j + 2 * tt + (e & 1);
-        const double2 c = make_double2(-re[j][e], -im[j][e]);
-        if (diagonal) sm[n * kLdD + m] = c;
-        else C[(size_t)(m0 + m) + (size_t)(n0 + n) * ldc] = c;
+        const double2 v = make_double2(c[j & 1][e].x - re[j][e], c[j & 1][e].y - im[j][e]);
+        if (diagonal) sm[(wn + 8 * j + 2 * tt + (e & 1)) * kLdD + wm + g + 8 * (e >> 1)] = v;
+        else *at(j, e) = v;
       }
+    }
     if (!diagonal) return;
     __syncthreads();
     factor_diagonal(sm, sm + kNB * kLdD, sh, C - kk - (int64_t)kk * ldc, ldc, kk, piv + (size_t)b * piv_stride,

@@ -137,3 +137,25 @@ def test_factors_of_blocks_with_ill_conditioned_triangles(n, weak):
     error = np.abs((L.astype(np.clongdouble) @ U - A[rows]).astype(complex))
     ratio = (error / (np.abs(L) @ np.abs(U))).max() / (n * 2.0 ** -53)
     assert ratio <= 1 / np.sqrt(n)
+
+
+@pytest.mark.parametrize("n", [64, 192, 448])
+def test_updates_round_to_a_dominant_matrix_once(n):
+    # products far smaller than the diagonal: what is left of the error is the
+    # rounding of each update of a diagonal entry, one per eight columns in its own
+    # block and one per block before it, half a unit of 2^-53 each
+    import torch
+    lib = _lib.load()
+    rng = np.random.default_rng(n)
+    A = 0.02 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n) + np.eye(n) * (0.6 + 0.7j)
+    At = torch.as_tensor(np.ascontiguousarray(A.T), device="cuda")
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(lib.bem_zlu_workspace_bytes(n, 1)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.bem_zlu_factor(_vp(At), n, n, n * n, 1, _vp(piv), _vp(info), _vp(work), _lib.stream_ptr()))
+    lu, p = At.cpu().numpy().T, piv.cpu().numpy()
+    assert np.array_equal(p, np.tile(np.arange(64), n // 64))
+    L, U = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+    diagonal = np.diag(L.astype(np.clongdouble) @ U - A)
+    error = np.maximum(np.abs(diagonal.real), np.abs(diagonal.imag)).max()
+    assert error <= (8 + n // 64) * 2.0 ** -54
