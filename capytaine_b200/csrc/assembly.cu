@@ -903,6 +903,18 @@ __device__ __forceinline__ void packed_integrals(double r, double z, const Packe
 struct WavePair {
   double g_re, g_im, h_re, h_im, v_re, v_im;
 };
+// Green_wave.f90:128-158, a panel of the free surface with itself: its value takes
+// the panel's area in place of the quadrature weight and its derivative along z has
+// a term in 4 sqrt(pi area).
+__device__ __forceinline__ WavePair own_pair(double area, double k) {
+  WavePair w;
+  w.g_re = (1 - log(k * k * area / kPI)) + 2 * (kEulerGamma - kLog2);
+  w.g_im = -2 * kPI;
+  w.h_re = w.h_im = 0.0;
+  w.v_re = w.g_re + 4 * sqrt(kPI * area) / (k * area);
+  w.v_im = w.g_im;
+  return w;
+}
 template <bool HIGH>
 __device__ __forceinline__ WavePair wave_pair(double r, double z, double k, double inv_k, double inv_R,
                                               const PackedTab& P) {
@@ -1048,18 +1060,12 @@ __global__ void __launch_bounds__(kPairRows, 3)
       const double hB = adjoint ? hJ : hI, vB = adjoint ? f.dn[2] : nI[2];
       double cJ = kMinusOneOverFourPi * k * f.w, cB = cI;
       WavePair w;
-      if (rr < kLit1em10 && fabs(zz) < kLit1em10) {
-        // Green_wave.f90:128-158, panel on the free surface with itself; its
-        // value takes the panel's area in place of the quadrature weight and
-        // its derivative along z has a term in 4 sqrt(pi area)
+      const bool own = rr < kLit1em10 && fabs(zz) < kLit1em10;
+      if (own) {
         const double c = kMinusOneOverFourPi * k;
         cJ = c * f.area;
         cB = c * areaI;
-        w.g_re = (1 - log(k * k * f.area / kPI)) + 2 * (kEulerGamma - kLog2);
-        w.g_im = -2 * kPI;
-        w.h_re = w.h_im = 0.0;
-        w.v_re = w.g_re + 4 * sqrt(kPI * f.area) / (k * f.area);
-        w.v_im = w.g_im;
+        w = own_pair(f.area, k);
       } else {
         w = wave_pair<HIGH>(rr, zz, k, inv_k, inv_R, P);
       }
@@ -1068,6 +1074,7 @@ __global__ void __launch_bounds__(kPairRows, 3)
       double kre = fma(ckJ, hA * w.h_re + vA * w.v_re, kMinusOneOverFourPi * rk.y);
       const double kim = ckJ * (hA * w.h_im + vA * w.v_im);
       if (mirrored) {
+        if (own) w = own_pair(areaI, k);  // coincident panels: each entry has its own panel's area
         const double ckI = cB * k;
         mS[u * kMirLd + lane] = make_double2(cB * w.g_re, cB * w.g_im);
         mK[u * kMirLd + lane] =
