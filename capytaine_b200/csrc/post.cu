@@ -12,6 +12,7 @@
 //   F_d = sum_i p_i (-dof_d . n_i) area_i (bodies/bodies.py:238-250) of the
 //   radiated/diffracted pressure i*omega*rho*phi and of the incident-wave
 //   pressure (airy_waves.py:19-53, 98-102).
+#include <algorithm>
 #include <cmath>
 
 #include "dmma.cuh"
@@ -277,19 +278,22 @@ extern "C" int bem_build_rhs(int n, int batch, const double* omega_dev, const do
 // 256 columns: shorter ones spend their time filling the ring (3741 in shares of
 // 47 columns 66 us, of 187 58 us), and every split writes and reads M x nrhs
 // partial sums.
+constexpr int kTsFill = 4 * 148, kTsFillCols = 32;
+constexpr int kTsEven = 32 * 148, kTsEvenCols = 256;
 static int ts_nsplit(int M, int K, int batch) {
   const long long rows = (long long)ceil_div(M, kTsRows) * batch;
-  const int fill = std::min(ceil_div(4 * 148, rows), K / 32), even = std::min(ceil_div(32 * 148, rows), K / 256);
-  return std::max(1, std::max(fill, even));
+  return std::max(1, std::max(std::min(ceil_div(kTsFill, rows), K / kTsFillCols),
+                              std::min(ceil_div(kTsEven, rows), K / kTsEvenCols)));
 }
 
+// For these sizes and all smaller ones (which may take more splits): rows blocks
+// of 128 rows have at most `kTsFill / rows + 1` splits by the first rule,
+// `kTsEven / rows + 1` by the second.
 extern "C" int64_t bem_zgemm_ts_workspace_bytes(int M, int K, int nrhs, int batch) {
-  // enough for calls with fewer matrices too, which may take more splits
-  int64_t most = 0;
-  for (int b = 1; b <= std::max(1, batch); ++b) {
-    most = std::max(most, (int64_t)b * ts_nsplit(M, K, b));
-  }
-  return most * (int64_t)M * nrhs * (int64_t)sizeof(double2);
+  const int64_t rows = (int64_t)ceil_div(std::max(M, 1), kTsRows) * std::max(batch, 1);
+  const int64_t blocks = std::max({rows, std::min(rows + kTsFill, rows * (K / kTsFillCols)),
+                                   std::min(rows + kTsEven, rows * (K / kTsEvenCols))});
+  return blocks * kTsRows * nrhs * (int64_t)sizeof(double2);
 }
 
 namespace bem {
