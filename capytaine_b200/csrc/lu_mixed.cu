@@ -1236,7 +1236,10 @@ int clu_factor_impl(const void* K_dev, int64_t ldk, int64_t strideK, int n, int 
   // in all matrices together (8 x 3072: 4.13 -> 3.70 ms with 200, 3.88 with 100;
   // 15 x 6144 the same with 100, 200 and 400), and up to 24 matrices, whose
   // next blocks still fit the GPU at once (24 x 1024 1.18 -> 1.13 ms, but
-  // 32 x 1536 2.41 -> 2.46, 60 x 1536 3.81 -> 3.95)
+  // 32 x 1536 2.41 -> 2.46, 60 x 1536 3.81 -> 3.95).  The two ways round
+  // differently, so that the factors of a matrix follow its batch; one way for
+  // every batch costs 29% without (3840: 2.96 -> 3.82 ms) or 20% with it (60 x 1536:
+  // 3.82 -> 4.58 ms)
   auto direct = [&](int kk) {
     return batch <= 24 && (long long)batch * (npad - kk - 2 * kB) < 200ll * kB;
   };

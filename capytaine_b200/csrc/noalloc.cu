@@ -190,7 +190,7 @@ extern "C" int bem_zgemm_ts_static(int M, int K, int nrhs, double alpha_re, doub
   double2* scratch = nullptr;
   int st = static_scratch_address(&scratch);
   if (st) return st;
-  // As many K-splits as bem_zgemm_ts would use, reduced to fit the array.
+  // One K-split per 96 columns, at most 64, reduced to fit the array.
   int nsplit = std::max(1, std::min(64, K / 96));
   nsplit = (int)std::min<long long>(nsplit, kStaticScratch / per_split);
   nsplit = std::max(nsplit, 1);

@@ -29,7 +29,10 @@ Scheduling
   tabulation are resident in the Green function's caches.
 
 Results do not depend on what else runs: every kernel is deterministic and
-requests share no mutable device memory.
+requests share no mutable device memory.  With ``batch_max`` above 1 a request may
+be factored in one batch with others; the block steps of the LU and the splits of
+sums follow the batch's size, so its results then agree with those of the request
+alone to the solve's relative residual (1e-10), not bit for bit.
 """
 from __future__ import annotations
 

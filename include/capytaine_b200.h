@@ -305,7 +305,9 @@ int bem_build_rhs(int n, int batch, const double* omega_dev, const double* waven
                   int64_t ldb, int64_t strideB, void* stream);
 
 /* Y = alpha A X + beta Y, A (M x K) complex128, X (K x nrhs), nrhs <= 16:
- * the potential S @ sigma (bem/solver.py:197-198) and residuals. */
+ * the potential S @ sigma (bem/solver.py:197-198) and residuals.  The workspace of
+ * these sizes serves every smaller call too.  The depth is summed in parts whose
+ * number follows M, K and batch: a matrix alone and in a batch agree to rounding. */
 int64_t bem_zgemm_ts_workspace_bytes(int M, int K, int nrhs, int batch);
 int bem_zgemm_ts(int M, int K, int nrhs, double alpha_re, double alpha_im, const void* A_dev, int64_t lda,
                  int64_t strideA, const void* X_dev, int64_t ldx, int64_t strideX, double beta_re, double beta_im,
@@ -363,7 +365,10 @@ int64_t bem_clu_workspace_bytes(int npad, int batch);
  * its rows, trailing updates run on the tcgen05 tensor cores (TF32 inputs,
  * FP32 accumulation).  piv_dev (batch x npad ints) is reserved: no row
  * permutation leaves the diagonal blocks.  info_dev: batch ints, 0 or the
- * 1-based column of the first zero pivot; err_dev: bounded-wait timeout flag.
+ * 1-based column of the first pivot that is zero or has no finite reciprocal;
+ * err_dev: bounded-wait timeout flag.  The order of the block steps follows the
+ * batch's size: the factors of a matrix alone and in a batch agree to float32
+ * rounding, not bit for bit.
  * Replaces the LU of tools/block_circulant_matrices.py:361-378 in the
  * mixed-precision engine. */
 int bem_clu_factor(const void* K_dev, int64_t ldk, int64_t strideK, int n, int npad, int batch, int* piv_dev,
