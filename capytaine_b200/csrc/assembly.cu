@@ -8,10 +8,13 @@
 // self-panel term) and Delhommeau_integrals.f90:157-402 (tabulation lookup,
 // asymptotic branch).
 //
-// Work decomposition: a CTA owns 128 consecutive collocation points (rows I) and
-// a tile of kTileJ source panels (columns J) staged in shared memory.  Each
-// thread walks its row across the tile, so each column store of a warp is 32
-// consecutive complex entries of the column-major output.
+// Work decomposition: a CTA owns 128 consecutive collocation points (rows I), a
+// warp 32 of them, and a run of source panels (columns J) staged in shared memory.
+// Each lane walks its row across them, so each column store of a warp is 32
+// consecutive complex entries of the column-major output.  A mesh with itself from a
+// cached Rankine part: wave_pairs_kernel (each unordered pair once); any points, any
+// depth: assemble_entries_kernel; without a packed table or with the float32 wave
+// term: wave_symmetric_kernel and assemble_kernel.
 //
 // Precision: BEM_PREC_FP64 evaluates every term in float64.  BEM_PREC_MIXED
 // evaluates the tabulated wave term (table values, Lagrange interpolation,
@@ -77,7 +80,7 @@ __device__ __forceinline__ double norm2_2(double a, double b) {
 }
 
 // Green_Rankine.f90:68-157
-__device__ void exact_rankine(const double M[3], const FaceRec& f, bool deriv_first, double& G, double dG[3]) {
+__device__ void exact_rankine(const double M[3], const FaceRec& f, double& G, double dG[3]) {
   const double* c = f.c;
   const double* n = f.n;
   const double GZ = (M[0] - c[0]) * n[0] + (M[1] - c[1]) * n[1] + (M[2] - c[2]) * n[2];
@@ -133,11 +136,6 @@ __device__ void exact_rankine(const double M[3], const FaceRec& f, bool deriv_fi
       dG[1] = dG[1] + ALDEN * GYX1 - cA * n[1] + c1 * ANLX1 - cB * (two_dk * GYX1 * DNT - DNTX1 * ANT);
       dG[2] = dG[2] + ALDEN * GYX2 - cA * n[2] + c1 * ANLX2 - cB * (two_dk * GYX2 * DNT - DNTX2 * ANT);
     }
-  }
-  if (!deriv_first) {
-    dG[0] = -dG[0];
-    dG[1] = -dG[1];
-    dG[2] = -dG[2];
   }
 }
 
@@ -472,7 +470,7 @@ __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_a
         dGr[1] = dg[1];
         dGr[2] = dg[2];
       } else {
-        exact_rankine(M, f, true, Gr, dGr);
+        exact_rankine(M, f, Gr, dGr);
       }
     }
     double Gre = Gr;
@@ -493,7 +491,7 @@ __global__ void __launch_bounds__(kRows, 4) assemble_kernel(const bem_assembly_a
           dGf[1] = dg[1];
           dGf[2] = dg[2];
         } else {
-          exact_rankine(Mr, f, true, Gf, dGf);
+          exact_rankine(Mr, f, Gf, dGf);
         }
         dGf[2] = -dGf[2];  // reflection coefficient c0 = -1
       }
@@ -905,15 +903,11 @@ struct WavePair {
 };
 // Green_wave.f90:128-158, a panel of the free surface with itself: its value takes
 // the panel's area in place of the quadrature weight and its derivative along z has
-// a term in 4 sqrt(pi area).
-__device__ __forceinline__ WavePair own_pair(double area, double k) {
-  WavePair w;
-  w.g_re = (1 - log(k * k * area / kPI)) + 2 * (kEulerGamma - kLog2);
-  w.g_im = -2 * kPI;
-  w.h_re = w.h_im = 0.0;
-  w.v_re = w.g_re + 4 * sqrt(kPI * area) / (k * area);
-  w.v_im = w.g_im;
-  return w;
+// a term in 4 sqrt(pi area).  The real parts of g and v (the imaginary ones are
+// -2 pi).  Out of line: two calls cost the pair kernel 1.3%, in line 2.4%.
+__device__ __noinline__ double2 own_pair(double area, double k) {
+  const double g = (1 - log(k * k * area / kPI)) + 2 * (kEulerGamma - kLog2);
+  return make_double2(g, g + 4 * sqrt(kPI * area) / (k * area));
 }
 template <bool HIGH>
 __device__ __forceinline__ WavePair wave_pair(double r, double z, double k, double inv_k, double inv_R,
@@ -959,7 +953,7 @@ struct PairFace {
 // tiles the wave term is evaluated once per unordered pair and the mirrored
 // entries go through the warp's own shared memory, 8 columns at a time, so
 // that both stores are coalesced and no warp waits for another.
-// Bound: the load pipe of L1 (68% busy, float64 pipe 18%): the nine quads of a
+// Bound: the load pipe of L1 (62% busy, hit rate 56%): the nine quads of a
 // lookup are 288 bytes per lane from its own place in the table.  The 15
 // wavenumbers of the 6084-panel barge take 8.9 ms (0.60 ms each, 42 float64
 // operations fewer per pair and 11 loads in place of 57), from 15.4 ms with the
@@ -1065,7 +1059,8 @@ __global__ void __launch_bounds__(kPairRows, 3)
         const double c = kMinusOneOverFourPi * k;
         cJ = c * f.area;
         cB = c * areaI;
-        w = own_pair(f.area, k);
+        const double2 g = own_pair(f.area, k);
+        w = WavePair{g.x, -2 * kPI, 0.0, 0.0, g.y, -2 * kPI};
       } else {
         w = wave_pair<HIGH>(rr, zz, k, inv_k, inv_R, P);
       }
@@ -1074,7 +1069,11 @@ __global__ void __launch_bounds__(kPairRows, 3)
       double kre = fma(ckJ, hA * w.h_re + vA * w.v_re, kMinusOneOverFourPi * rk.y);
       const double kim = ckJ * (hA * w.h_im + vA * w.v_im);
       if (mirrored) {
-        if (own) w = own_pair(areaI, k);  // coincident panels: each entry has its own panel's area
+        if (own) {  // coincident panels: each entry has its own panel's area
+          const double2 g = own_pair(areaI, k);
+          w.g_re = g.x;
+          w.v_re = g.y;
+        }
         const double ckI = cB * k;
         mS[u * kMirLd + lane] = make_double2(cB * w.g_re, cB * w.g_im);
         mK[u * kMirLd + lane] =
