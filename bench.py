@@ -602,9 +602,9 @@ def fp64_tensor_peak_tflops():
 
 # DRAM bytes per algorithmic flop of the trailing-update GEMM, from one ncu
 # capture of a full trailing update of two block steps (m = 4480, depth 256, 2
-# matrices: 640.0 MB read + written for 82.2 GFLOP); the traffic of the
+# matrices: 619.8 MB read + written for 82.2 GFLOP); the traffic of the
 # average launch is scaled from it by its flops.
-CGEMM_DRAM_BYTES_PER_FLOP = 640.0e6 / (8 * 4480 ** 2 * 256 * 2)
+CGEMM_DRAM_BYTES_PER_FLOP = 619.8e6 / (8 * 4480 ** 2 * 256 * 2)
 
 
 def lu_update_flops(npad, block):
@@ -691,7 +691,8 @@ def kernel_roofline(kernels, n, frequencies, engine, peaks, peak_src, frequencie
         return base | {"bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                        "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (float64 has no entry in "
                                       "MEASURED_PEAKS.json)",
-                       "algorithmic": "8 m^2 64 real flops per complex update of m x m by depth 64"}
+                       "algorithmic": "8 m^2 64 real flops per complex update of m x m by depth 64; the time includes "
+                               "the factorisation of the next diagonal block inside each update"}
     if name == "ctrsm_persistent_kernel":
         npad = -(-n // 128) * 128
         # one forward and one backward sweep read the float32 planes once (8 bytes per entry)

@@ -26,7 +26,7 @@ TimerState& timers() {
 std::atomic<int> g_timing{0};
 const char* const kClassNames[kKClassCount] = {
     "assemble_kernel",   "zgemm_dmma_kernel",  "cgemm_tf32_update_kernel", "clu_gj_kernel",
-    "clu_panel_kernel",  "ctrsm_persistent_kernel", "zlu_diag_kernel",  "zlu_panel_kernel",
+    "clu_panel_kernel",  "ctrsm_persistent_kernel", "zlu_first_kernel",  "zlu_panel_kernel",
     "ztrsm_persistent_kernel", "zgemm_ts_partial_kernel+reduce"};
 void clear_timers_locked(TimerState& t) {
   for (auto& v : t.pairs) {

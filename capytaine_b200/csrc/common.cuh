@@ -68,7 +68,7 @@ enum KernelClass {
   kKCluGj,
   kKCluPanel,
   kKCtrsm,
-  kKZluDiag,
+  kKZluFirst,  // the first diagonal block; the others are factored inside zgemm_dmma_kernel's updates
   kKZluPanel,
   kKZtrsm,
   kKZgemmTs,
@@ -83,8 +83,8 @@ struct TimedLaunch {
 };
 
 // Default iteration limit of the flag waits in the persistent block
-// substitutions (polls of ~64 ns sleeps: a wait gives up after about a
-// quarter of a second and reports BEM_ERR_TIMEOUT).
+// substitutions (polls of 0.22 us, an acquire load and a sleep of 20 ns: a wait gives
+// up after about 0.9 s and reports BEM_ERR_TIMEOUT).
 constexpr long long kDefaultSpinLimit = 4000000;
 
 // Stream-ordered pieces shared between the solver files.
@@ -123,17 +123,16 @@ struct CgemmDepth {
   bool embedded;
 };
 
-// Tiles of a block that a product covers: all, all but the first, or the first
-// row and column of a square block without their common tile.
+// Tiles of a block that a product covers: all of them; L: the first row and the first
+// column of a square block, without their common tile; or all but the first tile.
 enum TileRegion { kTilesAll = 0, kTilesL = 1, kTilesNoCorner = 2 };
 
 // C (m x n complex in two float32 planes) -= A' B' (store = 0) or = A' B'
 // (store = 1) on the tensor cores from packed operands; an optional second
 // operand pair adds a second segment in the same pass over C; limit_host: per-matrix
 // active sizes (grouped launches); pack: a packed copy of the result; region:
-// which tiles of the block;
-// reserve_sms: SMs that a kernel beside this one holds (left out of the
-// launch's width).
+// which tiles of the block; reserve_sms: SMs that a kernel beside this one holds
+// (left out of the launch's width).
 int cgemm_tf32_update(const float* Aop, int64_t a_rows, int a_row0, const float* Bop, int64_t b_rows, int b_row0,
                       const CgemmDepth& depth, float* Cr, float* Ci, int64_t ldc, int64_t c_stride, int c_row0, int c_col0, int m,
                       int n, int batch, int* err, cudaStream_t stream, int store = 0, const float* Aop1 = nullptr,

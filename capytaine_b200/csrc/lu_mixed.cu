@@ -298,8 +298,9 @@ __device__ __forceinline__ void gj_factor(GjColumns& a, int q, int kk, int b, in
 // Bound: the chain of panels on one SM, 8000 cycles each: the factorisation 4400
 // (540 a column: shuffles of the pivot row, reciprocal, multipliers, the key and
 // its reduction), the next warp's rank-8 update 2050, the exchange 1300; the
-// other warps' updates (5000 a scheduler) run beside it.  79 us per block (80
-// with a pass of its own for the scaling and a serial loop of the stores).  One
+// other warps' updates (5000 a scheduler) run beside it.  79 us per block (77
+// without the range check of the pivots' squares, 80 with a pass of its own for the
+// scaling and a serial loop of the stores besides).  One
 // step per exchange took 1800 cycles a column (121 us per block with the packed
 // copies written by the same CTA): a pivot search, two trips through shared
 // memory and a barrier each.  Row pairs and duplicated pivot entries feed the
@@ -468,8 +469,8 @@ __global__ void __launch_bounds__(256) clu_inverse_pack_kernel(const float2* __r
   dst[kB / 4] = make_float4(tf32_rn(v[0].y), tf32_rn(v[1].y), tf32_rn(v[2].y), tf32_rn(v[3].y));
 }
 
-// Operand packing of block step kk of the block LU (A_kk^{-1} comes packed
-// from the Gauss-Jordan kernel, L21 from the epilogue of the panel product).
+// Operand packing of block step kk of the block LU (A_kk^{-1} is packed by
+// clu_inverse_pack_kernel, L21 by the epilogue of the panel product).
 // Blocks [0, nrest): the block row to the right of the diagonal, 64 columns
 // each, packed as the B operand (U12 = A12).  Blocks [nrest, nrest +
 // nrows/32): 32 rows of the block column [col0, col0 + 128) from row row0 on,
@@ -970,8 +971,10 @@ int sm_count(int* out) {
   return BEM_OK;
 }
 
-// Workspace layout (bytes): [planes 2*npad^2 floats][Aop npad*2kB floats][Bop 2*npad*2kB floats]
-// [diagonal inverses nblk*kB*kB float2][flags batch*nblk + 1 ints], each per matrix except flags.
+// Workspace layout, each part for the whole batch: planes 2 npad^2 floats per matrix,
+// three A operands of npad x 2 kB floats, three B operands of 2 npad x kB floats,
+// diagonal inverses nblk x kB x kB float2, the packed operands of the current block
+// (see the members), then batch nblk + 2 + batch ints (flags, ticket, refinement).
 struct MixedWork {
   float* W;
   float* Aop;

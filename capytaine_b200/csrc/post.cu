@@ -88,8 +88,8 @@ constexpr int kTsMaxRhs = 16;
 // plain multiply-adds (27 TF/s, one row per thread, X from shared memory) 8
 // columns already cost as much as the reads and 16 twice as much.  A CTA owns 128
 // rows, 16 per warp; A and X stream through a five-stage cp.async ring of depth 8.
-// 15 x 6084^2, 7 columns: 1.91 -> 1.42 ms (6.25 TB/s, 0.96 of the measured copy
-// rate); 20493^2, 16 columns: 3.31 -> 1.83 ms (1.5 of MMAs).
+// 15 x 6084^2, 7 columns: 1.91 -> 1.31 ms (6.8 TB/s, a little above the measured copy
+// rate: reads only); 20493^2, 16 columns: 3.31 -> 1.83 ms (1.5 of MMAs).
 constexpr int kTsRows = 128, kTsDepth = 8, kTsStages = 5;
 constexpr int kTsLdA = kTsRows + 2, kTsLdX = kTsDepth + 4;
 constexpr int kTsStage = kTsDepth * kTsLdA + kTsMaxRhs * kTsLdX;

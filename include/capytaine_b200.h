@@ -405,7 +405,7 @@ int bem_reciprocals(int kind, int64_t n, const double* in_dev, double* out_dev, 
 
 /* No counterpart in the reference: a test of the bounded waits.  bem_clu_solve
  * with the iteration limit of the flag waits of its block substitutions given
- * (spin_limit > 0 polls of ~64 ns; bem_clu_solve uses 4e6) and, when
+ * (spin_limit > 0 polls of about 0.22 us; bem_clu_solve uses 4e6) and, when
  * withheld_block >= 0, that block row's completion flag never published, so
  * that every wait on it runs out: each waiting block then sets *err_dev = 1
  * and finishes (its result is invalid, every access stays in bounds), and the
