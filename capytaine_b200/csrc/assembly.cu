@@ -1254,6 +1254,11 @@ struct EntryParams {
 constexpr int kImageUnroll = 2;  // 4: 3% faster in finite depth, 8% slower with two images
 constexpr int kEntryCols = 32;   // most columns per CTA
 constexpr int kEntryQueue = 64;  // near pairs of a warp waiting
+// Squares of distances whose reciprocal square root rsqrt_pos gives (2^-997 to 2^997,
+// told by the exponent); outside, norms that do not overflow take its place.
+__device__ __forceinline__ bool plain_square(double x) {
+  return (unsigned)(__double2hiint(x) - 0x01a00000) < 0x7ca00000u;
+}
 
 // S and K (dot product taken or the three gradient planes) entry by entry:
 // matrices.f90:28-325 in infinite or finite depth (Delhommeau's method).  RANK:
@@ -1358,10 +1363,12 @@ __global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_as
     const double h2 = dx * dx + dy * dy;
     const double far_hi = f.far2 * (1.0 + 1e-12);
     if (!near_pass) {
-      // near: an image may be within 7 radii (every image is as far as h2 at least)
+      // near: an image may be within 7 radii (every image is as far as h2 at least),
+      // or squares of distances are near the end of the range
       const double z0 = Mz - cz, z1 = Mz + cz;
-      const bool near = active && !(h2 > far_hi) &&
-                        (finite_depth || !(h2 + z0 * z0 > far_hi) || (nimg > 1 && !(h2 + z1 * z1 > far_hi)));
+      const double d0 = h2 + z0 * z0;
+      const bool clear = finite_depth ? h2 > far_hi : d0 > far_hi && (nimg == 1 || h2 + z1 * z1 > far_hi);
+      const bool near = active && !(clear && plain_square(d0 + z1 * z1));
       const unsigned m = __ballot_sync(0xffffffffu, near);
       if (near) queue[warp][waiting + __popc(m & ((1u << lane) - 1))] = (unsigned short)(c << 5 | r);
       __syncwarp();
@@ -1400,7 +1407,8 @@ __global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_as
           far = (t == 0 ? norm2_3(dx, dy, Mz - cz) : hypot(norm2_2(dx, dy), zi - cz)) > 7 * f.radius;
         double g, gz;
         if (far) {
-          const double inv = ro2 > kLit1em7 * kLit1em7 ? rsqrt_pos(ro2) : 0.0;
+          double inv = ro2 > kLit1em7 * kLit1em7 ? rsqrt_pos(ro2) : 0.0;
+          if (ro2 > 1.0 && !plain_square(ro2)) inv = 1.0 / norm2_3(dx, dy, vz);
           g = f.area * inv;
           const double s = g * (inv * inv);
           H -= m.weight * s;
@@ -1436,8 +1444,12 @@ __global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_as
         }
         const double wx = Mx - qx, wy = My - qy;
         const double w2 = wx * wx + wy * wy;
-        const double ih = w2 > 1e-300 ? rsqrt_pos(w2) : 0.0;
-        const double rr = k * (w2 * ih);
+        double ih = rsqrt_pos(w2), w = w2 * ih;
+        if (!plain_square(w2)) {
+          w = norm2_2(wx, wy);
+          ih = w > 1e-150 ? 1.0 / w : 0.0;
+        }
+        const double rr = k * w;
         // no horizontal derivative at r = 0 (Green_wave.f90:186)
         const double unit = rr > 16 * kEpsilon ? ih : 0.0;
         // the panel's own term is at its centre (Green_wave.f90:75-80)
@@ -1488,7 +1500,7 @@ __global__ void __launch_bounds__(kRows, 3) assemble_entries_kernel(const bem_as
           }
           // infinite where the point meets a quadrature point of the free surface
           const double r2 = rr * rr + zz * zz;
-          const double inv_r1 = r2 > 1e-300 ? rsqrt_pos(r2) : 1.0 / hypot(rr, zz);
+          const double inv_r1 = plain_square(r2) ? rsqrt_pos(r2) : 1.0 / hypot(rr, zz);
           double hr = I[2], vr = I[0];
           if (high) {
             const double s3 = 2 * inv_r1 * inv_r1 * inv_r1;

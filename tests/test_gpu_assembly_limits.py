@@ -39,3 +39,22 @@ def test_point_that_is_no_number_is_reported(gf, axis, free_surface, wavenumber)
     with pytest.raises(_lib.GreenFunctionEvaluationError):
         gf.evaluate(points, _hull(), free_surface=free_surface, wavenumber=wavenumber)
 
+
+
+@pytest.mark.parametrize("depth", [np.inf, 9.0])
+@pytest.mark.parametrize("free_surface,wavenumber", [(np.inf, 1.0), (0.0, 0.0), (0.0, np.inf), (0.0, 0.5)])
+@pytest.mark.parametrize("points", [[[1e160, 0, -1], [0, -1e170, -2]], [[1e160, 0, -1], [3.0, 0, -2]]])
+def test_points_beyond_the_range_of_squares(gf, points, free_surface, wavenumber, depth):
+    if depth != np.inf and (free_surface == np.inf or wavenumber == 0.0):
+        pytest.skip("refused: a finite depth without a free surface or with k h below 0.1")
+    hull = _hull()
+    kw = dict(free_surface=free_surface, water_depth=depth, wavenumber=wavenumber, diagonal_term_in_double_layer=False)
+    S, K = gf.evaluate(np.array(points, dtype=float), hull, early_dot_product=False, **kw)
+    # 1 / r, and the wave term's 1 / sqrt(r), are all that is left
+    far = np.max(np.abs(points), axis=1) > 1e150
+    assert np.all(np.abs(S[far]) < 1e-60) and np.all(np.abs(K[:, far]) < 1e-60)
+    # a point beside them keeps its entries (other sums of a pair's terms: 1e-12 of the largest)
+    if not np.all(far):
+        s, k = gf.evaluate(np.array(points, dtype=float)[~far], hull, early_dot_product=False, **kw)
+        assert np.abs(S[~far] - s).max() <= 1e-12 * np.abs(s).max()
+        assert np.abs(K[:, ~far] - k).max() <= 1e-12 * np.abs(k).max()
